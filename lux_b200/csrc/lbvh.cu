@@ -1029,124 +1029,151 @@ int lbvh_refit(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
 
 namespace {
 
-struct WideSlots {
-    box3 box[4];
-    int ch[4];
-    int count;
-    LUX_D void add(int handle, const box3& b) {
-        if (count >= 4) return;
-        box[count] = b;
-        ch[count] = handle;
-        ++count;
-    }
-};
-
-// Biased exponent of an axis grid: from 2^e >= extent / 255, raised until the top grid
-// point decodes at or above hi.
-// Grid of one axis of a wide node whose children span [origin, hi] (the node's box):
-// the smallest exponent e (biased into *biased) for which the grid's points k * 2^e,
-// k = floor(origin / 2^e) with |k| <= 2^22, reach hi within 255 steps; *c = (k - 2^23) * 2^e
-// (exact).  False when no exponent up to 103 does (the node is then left unbounded).
-LUX_D bool wide_axis(float origin, float hi, unsigned* biased, float* c) {
-    const float extent = sub(hi, origin);
-    int e = -126;
+// Grid of one axis of a wide node whose children span [lo, hi]: the smallest exponent e
+// whose grid, starting at k * 2^e with k * 2^e <= lo - kWideMargin * 2^e, holds hi and the
+// margin within 255 steps.  False when no exponent within the range does.
+LUX_D bool wide_axis(float lo, float hi, float* scale, float* inv_scale, float* origin,
+                     float* c) {
+    const float extent = sub(hi, lo);
+    int e = -kWideMaxExp;
     if (extent > 0.0f) {
         int ex;
         frexpf(extent / 255.0f, &ex);
-        e = max(ex, -126);
+        e = max(ex, -kWideMaxExp);
     }
-    for (; e <= 103; ++e) {
-        const unsigned b = static_cast<unsigned>(e + 127);
-        const float scale = wide_scale(b);
-        const float inv = wide_scale(254u - b);  // 2^-e, exact for the exponents used
-        const float k = floorf(mul(origin, inv));
-        if (!(fabsf(k) <= 4194304.0f)) continue;            // 2^22
-        const float cc = mul(sub(k, 8388608.0f), scale);    // (k - 2^23) * 2^e, exact
-        if (wide_decode(cc, 255u, scale) < hi) continue;
-        *biased = b;
-        *c = cc;
+    for (; e <= kWideMaxExp; ++e) {
+        const float s = wide_scale(e);
+        const float inv = wide_scale(-e);
+        const float x = mul(lo, inv);           // exact: a power of two
+        float k = floorf(x);
+        if (!(fabsf(k) < 4194304.0f)) continue;  // 2^22
+        if (sub(x, k) < kWideMargin) k = sub(k, 1.0f);
+        const float o = mul(k, s);              // exact
+        if (!(add(mul(sub(hi, o), inv), kWideMargin) <= 255.0f)) continue;
+        *scale = s;
+        *inv_scale = inv;
+        *origin = o;
+        *c = mul(sub(k, 32768.0f), s);          // exact
         return true;
     }
     return false;
 }
 
-// Outward-rounded grid coordinates of [lo, hi]: the largest q_lo whose decode is <= lo
-// and the smallest q_hi whose decode is >= hi (grid offset c, see wide_axis).
-LUX_D void wide_quantize(float c, unsigned biased, float lo, float hi, unsigned& qlo,
+// Grid coordinates of [lo, hi], at least kWideMargin (less the rounding of the difference,
+// 2^-16 of a step) outside it.
+LUX_D void wide_quantize(float origin, float inv, float lo, float hi, unsigned& qlo,
                          unsigned& qhi) {
-    const float scale = wide_scale(biased);
-    const float inv = wide_scale(254u - biased);  // 2^-e, exact for the exponents used
-    const float origin = wide_decode(c, 0u, scale);
-    const float fa = floorf(mul(sub(lo, origin), inv));
-    int a = fa >= 255.0f ? 255 : (fa > 0.0f ? static_cast<int>(fa) : 0);
-    while (a > 0 && wide_decode(c, static_cast<unsigned>(a), scale) > lo) --a;
-    const float fb = ceilf(mul(sub(hi, origin), inv));
-    int b = fb >= 255.0f ? 255 : (fb > 0.0f ? static_cast<int>(fb) : 0);
-    while (b < 255 && wide_decode(c, static_cast<unsigned>(b), scale) < hi) ++b;
-    qlo = static_cast<unsigned>(a);
-    qhi = static_cast<unsigned>(b);
+    const float a = floorf(sub(mul(sub(lo, origin), inv), kWideMargin));
+    const float b = ceilf(add(mul(sub(hi, origin), inv), kWideMargin));
+    qlo = static_cast<unsigned>(fminf(fmaxf(a, 0.0f), 255.0f));
+    qhi = static_cast<unsigned>(fminf(fmaxf(b, 0.0f), 255.0f));
 }
 
-// Wide node i from binary node i and its internal children (see WideNode).
+LUX_D float half_area(const box3& b) {
+    const f3 d = b.hi - b.lo;
+    return add(add(mul(d.x, d.y), mul(d.y, d.z)), mul(d.z, d.x));
+}
+
+// Wide node i from binary node i and the nodes below it (see WideNode).
 __global__ void __launch_bounds__(kThreads) k_widen(const BvhNode* nodes, int n,
                                                     WideNode* wide, int* error) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
-    WideSlots s;
-    s.count = 0;
-    BvhNode nd = load_node(nodes, i);
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        int h = side ? nd.ch.y : nd.ch.x;
-        if (h >= n - 1) {  // cannot happen for a consistent hierarchy
-            atomicOr(error, kErrLoopBound);
-            continue;
+    const BvhNode nd = load_node(nodes, i);
+    if (nd.ch.x >= n - 1 || nd.ch.y >= n - 1) {  // cannot happen for a consistent hierarchy
+        atomicOr(error, kErrLoopBound);
+        return;
+    }
+    box3 box[4];
+    int ch[4];
+    int count;
+    if (nd.ch.x >= 0 && nd.ch.y >= 0) {
+        const BvhNode l = load_node(nodes, nd.ch.x), r = load_node(nodes, nd.ch.y);
+        box[0] = node_left_box(l); ch[0] = l.ch.x;
+        box[1] = node_right_box(l); ch[1] = l.ch.y;
+        box[2] = node_left_box(r); ch[2] = r.ch.x;
+        box[3] = node_right_box(r); ch[3] = r.ch.y;
+        count = 4;
+    } else if (nd.ch.x < 0 && nd.ch.y < 0) {
+        box[0] = node_left_box(nd); ch[0] = nd.ch.x;
+        box[1] = node_right_box(nd); ch[1] = nd.ch.y;
+        count = 2;
+    } else {
+        // One leaf and one internal child: the leaf, the child's children, and one of
+        // those opened (the larger box first).
+        const bool leaf_first = nd.ch.x < 0;
+        const BvhNode m = load_node(nodes, leaf_first ? nd.ch.y : nd.ch.x);
+        const box3 lb = leaf_first ? node_left_box(nd) : node_right_box(nd);
+        const int lh = leaf_first ? nd.ch.x : nd.ch.y;
+        box3 b3[3] = {node_left_box(m), node_right_box(m), box3{}};
+        int c3[3] = {m.ch.x, m.ch.y, kNoNode};
+        int c3n = 2;
+        int open = -1;
+        if (m.ch.x >= 0 && (m.ch.y < 0 || half_area(b3[0]) >= half_area(b3[1]))) open = 0;
+        else if (m.ch.y >= 0) open = 1;
+        if (open >= 0 && c3[open] < n - 1) {
+            const BvhNode g = load_node(nodes, open ? m.ch.y : m.ch.x);
+            if (open == 0) {
+                b3[2] = b3[1]; c3[2] = c3[1];
+                b3[0] = node_left_box(g); c3[0] = g.ch.x;
+                b3[1] = node_right_box(g); c3[1] = g.ch.y;
+            } else {
+                b3[1] = node_left_box(g); c3[1] = g.ch.x;
+                b3[2] = node_right_box(g); c3[2] = g.ch.y;
+            }
+            c3n = 3;
         }
-        if (h >= 0) {
-            BvhNode cn = load_node(nodes, h);
-            s.add(cn.ch.x, node_left_box(cn));
-            s.add(cn.ch.y, node_right_box(cn));
+        count = c3n + 1;
+        if (leaf_first) {
+            box[0] = lb; ch[0] = lh;
+            box[1] = b3[0]; ch[1] = c3[0];
+            box[2] = b3[1]; ch[2] = c3[1];
+            box[3] = b3[2]; ch[3] = c3[2];
         } else {
-            s.add(h, side ? node_right_box(nd) : node_left_box(nd));
+            box[0] = b3[0]; ch[0] = c3[0];
+            box[1] = b3[1]; ch[1] = c3[1];
+            box[2] = c3n == 3 ? b3[2] : lb; ch[2] = c3n == 3 ? c3[2] : lh;
+            box[3] = lb; ch[3] = lh;
         }
     }
-    box3 u = box_union(node_left_box(nd), node_right_box(nd));
-    float o[3] = {u.lo.x, u.lo.y, u.lo.z};
-    float top[3] = {u.hi.x, u.hi.y, u.hi.z};
-    bool finite = true;
-    for (int a = 0; a < 3; ++a) finite = finite && isfinite(o[a]) && isfinite(top[a]);
-    unsigned ebits[3] = {127u, 127u, 127u};
-    float cgrid[3] = {0.0f, 0.0f, 0.0f};
+    const box3 u = box_union(node_left_box(nd), node_right_box(nd));
+    const float o[3] = {u.lo.x, u.lo.y, u.lo.z};
+    const float top[3] = {u.hi.x, u.hi.y, u.hi.z};
+    bool fits = true;
+    float scale[3] = {1.0f, 1.0f, 1.0f}, inv[3], origin[3], cgrid[3];
+    for (int a = 0; a < 3 && fits; ++a)
+        fits = isfinite(o[a]) && isfinite(top[a]) &&
+               wide_axis(o[a], top[a], &scale[a], &inv[a], &origin[a], &cgrid[a]);
     unsigned lo_w[3] = {0, 0, 0}, hi_w[3] = {0, 0, 0};
-    for (int a = 0; a < 3 && finite; ++a) finite = wide_axis(o[a], top[a], &ebits[a], &cgrid[a]);
-    if (finite) {
-        for (int c = 0; c < s.count; ++c) {
-            float lo[3] = {s.box[c].lo.x, s.box[c].lo.y, s.box[c].lo.z};
-            float hi[3] = {s.box[c].hi.x, s.box[c].hi.y, s.box[c].hi.z};
+    if (fits) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c >= count) break;
+            const float lo[3] = {box[c].lo.x, box[c].lo.y, box[c].lo.z};
+            const float hi[3] = {box[c].hi.x, box[c].hi.y, box[c].hi.z};
+#pragma unroll
             for (int a = 0; a < 3; ++a) {
                 unsigned ql, qh;
-                wide_quantize(cgrid[a], ebits[a], lo[a], hi[a], ql, qh);
+                wide_quantize(origin[a], inv[a], lo[a], hi[a], ql, qh);
                 lo_w[a] |= ql << (8 * c);
                 hi_w[a] |= qh << (8 * c);
             }
         }
     } else {
         for (int a = 0; a < 3; ++a) {
-            ebits[a] = 127u;
-            cgrid[a] = 0.0f;
+            cgrid[a] = __int_as_float(0x7fffffff);
+            scale[a] = 1.0f;
         }
     }
-    unsigned meta = ebits[0] | (ebits[1] << 8) | (ebits[2] << 16) |
-                    (static_cast<unsigned>(s.count) << 24) | (finite ? 0u : kWideUnbounded);
-    int ch[4] = {0, 0, 0, 0};
-    for (int c = 0; c < s.count; ++c) ch[c] = s.ch[c];
+    if (count < 4) ch[3] = kNoNode;
+    if (count < 3) ch[2] = kNoNode;
     WideNode w;
-    w.q0 = make_float4(cgrid[0], cgrid[1], cgrid[2], __uint_as_float(meta));
+    w.q0 = make_float4(cgrid[0], cgrid[1], cgrid[2], scale[2]);
     w.q1 = make_float4(__uint_as_float(lo_w[0]), __uint_as_float(lo_w[1]),
                        __uint_as_float(lo_w[2]), __uint_as_float(hi_w[0]));
     w.q2 = make_float4(__uint_as_float(hi_w[1]), __uint_as_float(hi_w[2]), __int_as_float(ch[0]),
                        __int_as_float(ch[1]));
-    w.q3 = make_float4(__int_as_float(ch[2]), __int_as_float(ch[3]), 0.0f, 0.0f);
+    w.q3 = make_float4(__int_as_float(ch[2]), __int_as_float(ch[3]), scale[0], scale[1]);
     wide[i] = w;
 }
 

@@ -11,10 +11,24 @@
 
 namespace lux {
 
+// 32 bytes from a 32-byte aligned address through the read-only path, and 32 bytes to one,
+// in one instruction each: half the requests of 16-byte accesses to records that every
+// lane has at another place.
+LUX_D void ldg8(const void* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+LUX_D void stg8(void* p, const float4& a, const float4& b) {
+    asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                 ::"f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w),
+                 "l"(p) : "memory");
+}
+
 // Child handle: >= 0 internal node index; < 0 leaf, sorted leaf index k = ~handle.
 LUX_HD bool is_leaf_handle(int h) { return h < 0; }
 
-struct alignas(16) BvhNode {
+struct alignas(32) BvhNode {
     float4 a;  // left.lo.x  left.lo.y  left.lo.z  left.hi.x
     float4 b;  // left.hi.y  left.hi.z  right.lo.x right.lo.y
     float4 c;  // right.lo.z right.hi.x right.hi.y right.hi.z
@@ -39,38 +53,42 @@ LUX_HD box3 node_right_box(const BvhNode& n) {
     return box3{make_f3(n.b.z, n.b.w, n.c.x), make_f3(n.c.y, n.c.z, n.c.w)};
 }
 
-// 4-wide node of binary internal node i: its grandchildren in left-first order, a leaf
-// child standing for itself, so 2 to 4 children.  One is built for every internal node;
-// a walk from the root enters only those at even binary depth.  Child boxes are stored
-// quantised to 8 bits per plane on a per-axis power-of-two grid s = 2^e whose points are
-// integer multiples of s (the grid starts at k * s, the node's lower corner rounded down
-// to the grid), rounded outward, so each decoded box contains the exact one; the node is
-// 64 bytes.  Plane q decodes to (k + q) * s, which is a float exactly (|k| <= 2^22), as
-// one fused multiply-add fma(2^23 + q, s, c) with c = (k - 2^23) * s: the 2^23 + q is the
-// plane byte placed in the mantissa of 2^23 by one byte permute.  Decoded boxes only
-// steer the walk: a leaf is accepted by the exact test of its own box when the walk
-// reaches it.
-//   q0 = c.xyz, meta (bits 0-23: biased exponents x, y, z; 24-26: child count;
-//        27: unbounded, every child passes)
+// 4-wide node of binary internal node i in left-first order: its grandchildren; where one
+// child is a leaf, that leaf and the other child's children, one of them opened once more.
+// So 2 to 4 children, and a walk goes down at least two binary levels per node.  One is
+// built for every internal node; a walk from the root enters some of them.  Child boxes
+// are stored quantised to 8 bits per plane on a per-axis power-of-two grid s = 2^e whose
+// points are integer multiples k * s (|k| <= 2^22), rounded outward by at least 1/32 of a
+// grid step, so that a decoded box contains the exact one with room for the rounding of
+// the walk's slab test (wide_test).  Plane q is (k + q) * s = fma(2^15 + q, s, c) exactly,
+// with c = (k - 2^15) * s; 2^15 + q is the plane byte placed in the mantissa of 2^15 by
+// one byte permute.  Decoded boxes only steer the walk: a leaf is accepted by the exact
+// test of its own box when the walk reaches it.  A node that no grid fits (not finite, or
+// outside the exponents' range) has c = NaN: every child passes every test.
+//   q0 = c.xyz, scale s.z
 //   q1 = lo.x, lo.y, lo.z, hi.x bytes of children 0..3 (byte c of each word: child c)
 //   q2 = hi.y, hi.z bytes, child handles 0, 1
-//   q3 = child handles 2, 3, 0, 0
-struct alignas(16) WideNode {
+//   q3 = child handles 2, 3 (kNoNode: no such child), scales s.x, s.y
+struct alignas(32) WideNode {
     float4 q0, q1, q2, q3;
 };
 static_assert(sizeof(WideNode) == 64, "one wide node is one 64-byte record");
 
-constexpr unsigned kWideUnbounded = 1u << 27;
+constexpr int kNoNode = static_cast<int>(0x80000000u);   // neither a node nor a leaf handle
+constexpr int kWideMaxExp = 60;    // grid exponents are within [-60, 60]
+constexpr float kWideMargin = 1.0f / 32.0f;   // of a grid step, outside every exact plane
 
-LUX_D float wide_scale(unsigned biased) { return __int_as_float(static_cast<int>(biased) << 23); }
+LUX_D float wide_scale(int e) { return __int_as_float((e + 127) << 23); }
 
-// Plane byte q as the float 2^23 + q (exact for q < 2^23).
-LUX_D float wide_biased(unsigned q) { return __uint_as_float(0x4B000000u | q); }
+// Plane byte c of a packed word as the float 2^15 + byte.
+LUX_D float wide_biased(unsigned word, int c) {
+    return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7504u + 0x10u * c));
+}
 
-// Decoded plane (k + q) * 2^e of grid offset c = (k - 2^23) * 2^e: the fused
+// Decoded plane (k + q) * 2^e of grid offset c = (k - 2^15) * 2^e: the fused
 // multiply-add's exact result is a float, so it is returned unrounded.
-LUX_D float wide_decode(float c, unsigned q, float scale) {
-    return __fmaf_rn(wide_biased(q), scale, c);
+LUX_D float wide_decode(float c, unsigned word, int child, float scale) {
+    return __fmaf_rn(wide_biased(word, child), scale, c);
 }
 
 // Non-owning view passed by value into kernels.
@@ -93,11 +111,11 @@ LUX_D box3 load_root(const float* root) {
 
 LUX_D BvhNode load_node(const BvhNode* nodes, int i) {
     BvhNode n;
-    const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    n.a = __ldg(p + 0);
-    n.b = __ldg(p + 1);
-    n.c = __ldg(p + 2);
-    n.ch = __ldg(reinterpret_cast<const int4*>(p + 3));
+    float4 d;
+    ldg8(nodes + i, n.a, n.b);
+    ldg8(reinterpret_cast<const float4*>(nodes + i) + 2, n.c, d);
+    n.ch = make_int4(__float_as_int(d.x), __float_as_int(d.y), __float_as_int(d.z),
+                     __float_as_int(d.w));
     return n;
 }
 

@@ -298,11 +298,12 @@ struct TwoLevelWalk {
     bool in_blas;
     const WideNode* b_wide;
     const TriRecord* b_tris;
-    int b_n, b_cur, b_sp, b_ignored, b_first;
+    int b_n, b_cur, b_ignored, b_first;
+    WideTop b_top;
     unsigned b_steps;
     f3 lo, ld;
     slab_ray lsr;
-    unsigned lneg;                // octant of the object-space ray (octant_ray::neg)
+    unsigned lneg;                // octant of the object-space ray (wide_octant)
     bool done;
     bool any_hit;                 // end at the first accepted triangle (occlusion only)
 
@@ -378,15 +379,8 @@ struct TwoLevelWalk {
         return false;
     }
     LUX_D bool pop_blas(const WalkStacks& k) {
-        while (b_sp > 0) {
-            --b_sp;
-            const int2 e = k.b[b_sp];
-            if (!(__int_as_float(e.y) > hit.t)) {
-                b_cur = e.x;
-                return true;
-            }
-        }
-        return false;
+        b_cur = b_top.pop(k.b, hit.t);
+        return b_cur != kNoNode;
     }
 
     // One step; returns true when the walk is complete (hit holds the result).
@@ -399,26 +393,19 @@ struct TwoLevelWalk {
                 fail(error, kErrLoopBound, INFINITY);
                 return true;
             }
-            const octant_ray lorr{lsr.o, lsr.inv, lsr.tmin, lneg};
             bool pop = true;
             if (b_cur >= 0) {
                 const WideNode w = load_wide(b_wide, b_cur);
                 float tt[4];
-                const unsigned m = wide_test(w, lsr, lorr, hit.t, tt);
-                if (m) {
-                    const int f = __ffs(m) - 1;
-                    if (b_sp + __popc(m) - 1 > kWideBlasStack) {
-                        fail(error, kErrStackOverflow, INFINITY);
-                        return true;
-                    }
-#pragma unroll
-                    for (int c = 3; c >= 1; --c) {
-                        if (c > f && ((m >> c) & 1u)) {
-                            k.b[b_sp] = make_int2(wide_ref(w, c), __float_as_int(tt[c]));
-                            ++b_sp;
-                        }
-                    }
-                    b_cur = wide_ref(w, f);
+                bool pp[4];
+                wide_test(w, lsr, lneg, hit.t, tt, pp);
+                if (b_top.full(kWideBlasStack)) {
+                    fail(error, kErrStackOverflow, INFINITY);
+                    return true;
+                }
+                const int next = wide_descend(w, tt, pp, k.b, b_top);
+                if (next != kNoNode) {
+                    b_cur = next;
                     pop = false;
                 }
             } else {
@@ -429,6 +416,7 @@ struct TwoLevelWalk {
                     const float4 p1 = __ldg(tp + 1);
                     const float4 p2 = __ldg(tp + 2);
                     float tn, t, u, v;
+                    const octant_ray lorr = make_octant_ray(lsr);
                     // The leaf's exact box (the triangle's box) under the current best t,
                     // then the triangle.
                     if (child_hit(triangle_box(xyz(p0), xyz(p1), xyz(p2)), lsr, lorr, hit.t, tn)
@@ -497,12 +485,12 @@ struct TwoLevelWalk {
         float tn;
         if (!slab_hit(lsr, load_root(b.root), hit.t, tn)) return false;
         in_blas = true;
-        lneg = make_octant_ray(lsr).neg;
+        lneg = wide_octant(lsr);
         b_wide = b.wide;
         b_tris = b.tris;
         b_n = b.n;
         b_cur = b.n == 1 ? ~0 : 0;
-        b_sp = 0;
+        b_top.clear();
         b_steps = 0;
         b_ignored = inst_id == ign_instance ? ign_local : -1;
         b_first = inst.first_primitive;

@@ -25,9 +25,10 @@ namespace {
 
 constexpr int kTraceThreads = 128;
 #ifndef LUX_TRACE_BLOCKS
-#define LUX_TRACE_BLOCKS 10
+#define LUX_TRACE_BLOCKS 9
 #endif
 constexpr int kTraceBlocks = LUX_TRACE_BLOCKS;   // resident blocks per SM of the wide walk
+constexpr int kSpreadWarps = 16;                 // warps per SM over which few rays are spread
 constexpr int kStack = 96;  // > max Karras depth: 64 (30-bit keys) or 95 (63-bit + index)
 
 struct RayHit {
@@ -319,132 +320,139 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_persistent(
     }
 }
 
-// Persistent warps with refill (as k_trace_persistent) over the 4-wide nodes: a step is
-// one wide-node fetch (four child boxes) or one triangle test, followed by the pops it
-// enables.  Decisions are those of wide_walk, step for step.
-// 10 resident blocks per SM (at most 48 registers): occupancy hides the node-load
-// latency that bounds this kernel.  The cap spills 44 bytes per thread, and the extra
-// warps still win: 468 against 439 Mrays/s at 64 registers and 425 at 40 (1,048,576
-// triangles, 4,194,304 rays, B200).  The deferred-child stack lives in local memory and
-// its reads mostly miss L1; keeping an entry's node and entry distance in one 8-byte
-// record (one access per push or pop rather than two) gives 479 against 467 Mrays/s.
+// Persistent warps with refill over the 4-wide nodes: the hits of wide_walk, leaf by leaf.
+//
+// A lane's walk is at a node (cur >= 0) or waits at a leaf (leaf, and perhaps a second one
+// in cur).  The warp tests nodes until no more than kNodeShare of its rays are at one (or
+// `budget` times), then the waiting leaves; a lane that meets a leaf goes on with the nodes
+// behind it meanwhile.  That keeps every verdict: a node test only has to keep each leaf
+// that the reference reaches, which it does under any bound not below the current one, and
+// the leaves are tested in order, each under the bound of its turn.
+//
+// Bound by the latency of the node loads (about 93 dependent nodes per ray of the
+// microbenchmark, 1.04 passing children each) and by L1 requests.  Measured there
+// (1,048,576 triangles, 4,194,304 uniform rays): one step of whatever kind per lane and
+// round, 16-byte node loads 6.85 ms; leaves apart and planes' t by one fused multiply-add
+// 5.93 ms; nodes by two 32-byte loads 5.04 ms; two planes per packed multiply-add and 9
+// blocks per SM 4.99 ms.  Blocks per SM (56 registers at 9): 8 5.14 ms, 10 5.16 ms, 12
+// 6.2 ms.  Shares: 1/3 6.40 ms, 1/2 6.05 ms, 2/3 5.93 ms, 5/6 5.89 ms with 16-byte loads,
+// but a coherent view of a terrain takes 5 % longer at 5/6 than at 2/3.
+//
+// Few rays are spread over the SMs, `lanes` of a warp taking one each (launch_trace): 2,048
+// rays take 192 us there, and took 335 us in 64 full warps.
+constexpr int kNodeShareNum = 2, kNodeShareDen = 3;
+
 template <bool AnyHit>
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocks) k_trace_wide_persistent(
         BvhView bvh, const float4* rays, int nrays, int* hit_id, float* hit_t,
-        unsigned* ray_counter, int budget, int* error) {
+        unsigned* ray_counter, int budget, int lanes, int* error) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt_u();
-    const box3 root = load_root(bvh.root);
     const unsigned bound = 2u * static_cast<unsigned>(bvh.n) + 64u;  // n <= 2^30
+    // The first rays go by the lane's place, the others through the counter.
+    const unsigned placed = gridDim.x * (kTraceThreads / 32) * static_cast<unsigned>(lanes);
+    unsigned next = (blockIdx.x * (kTraceThreads / 32) + (threadIdx.x >> 5)) *
+                    static_cast<unsigned>(lanes) + lane;
+    bool first = true;
 
-    int ray_idx = -1;   // >= 0 active ray, -1 needs a ray, -2 no rays left
-    ray3 ray;
-    slab_ray sr;
-    octant_ray orr;
+    // >= 0 active ray, -1 needs a ray, -2 no rays left
+    int ray_idx = lane < static_cast<unsigned>(lanes) ? -1 : -2;
+    f3 d = make_f3(0, 0, 0);
+    slab_ray sr{};
+    unsigned oct = 0;
     float best_t = 0.0f;
     int best_k = -1;
-    int cur = 0;
-    int sp = 0;
+    int cur = kNoNode, leaf = kNoNode;
     unsigned steps = 0;
-    bool root_missed = false;
+    WideTop top;
+    top.clear();
     int2 stack[kWideStack];  // (node ref, entry t bits): one 8-byte access per entry
 
     for (;;) {
-        bool need = ray_idx == -1;
-        unsigned need_mask = __ballot_sync(0xffffffffu, need);
+        const bool need = ray_idx == -1;
+        const unsigned need_mask = __ballot_sync(0xffffffffu, need);
         if (need_mask) {
-            int leader = __ffs(need_mask) - 1;
-            unsigned base = 0;
-            if (lane == leader) base = atomicAdd(ray_counter, __popc(need_mask));
-            base = __shfl_sync(0xffffffffu, base, leader);
+            if (!first) {
+                next = static_cast<unsigned>(nrays);
+                if (placed < static_cast<unsigned>(nrays)) {
+                    const int leader = __ffs(need_mask) - 1;
+                    unsigned base = 0;
+                    if (lane == leader) base = atomicAdd(ray_counter, __popc(need_mask));
+                    base = __shfl_sync(0xffffffffu, base, leader);
+                    next = placed + base + __popc(need_mask & lt);
+                }
+            }
+            first = false;
             if (need) {
-                unsigned idx = base + __popc(need_mask & lt);
-                if (idx >= static_cast<unsigned>(nrays)) {
+                if (next >= static_cast<unsigned>(nrays)) {
                     ray_idx = -2;
                 } else {
-                    ray_idx = static_cast<int>(idx);
-                    ray = load_ray(rays, ray_idx);
+                    ray_idx = static_cast<int>(next);
+                    const ray3 ray = load_ray(rays, ray_idx);
+                    d = ray.d;
                     sr = make_slab_ray(ray);
-                    orr = make_octant_ray(sr);
+                    oct = wide_octant(sr);
                     best_t = ray.tmax;
                     best_k = -1;
-                    sp = 0;
                     steps = 0;
+                    cur = leaf = kNoNode;
+                    top.clear();
                     float tn;
-                    root_missed = bvh.n <= 0 || !slab_hit(sr, root, best_t, tn);
-                    cur = bvh.n == 1 ? ~0 : 0;
+                    if (bvh.n > 0 && slab_hit(sr, load_root(bvh.root), best_t, tn)) {
+                        if (bvh.n == 1) leaf = ~0;
+                        else cur = 0;
+                    }
                 }
             }
         }
-        if (__all_sync(0xffffffffu, ray_idx == -2)) break;
-
-        bool done = false;
-        if (ray_idx >= 0) {
-            if (root_missed) done = true;
-            for (int s = 0; s < budget && !done; ++s) {
-                if (++steps > bound || cur >= bvh.n - 1 || ~cur >= bvh.n) {
-                    atomicOr(error, kErrLoopBound);
-                    best_k = -1;
-                    best_t = ray.tmax;
-                    done = true;
-                    break;
-                }
-                bool pop = true;
-                if (cur >= 0) {
-                    const WideNode w = load_wide(bvh.wide, cur);
-                    float t[4];
-                    unsigned m = wide_test(w, sr, orr, best_t, t);
-                    if (m) {
-                        const int f = __ffs(m) - 1;
-                        if (sp + __popc(m) - 1 > kWideStack) {
-                            atomicOr(error, kErrStackOverflow);
-                            best_k = -1;
-                            best_t = ray.tmax;
-                            done = true;
-                            break;
-                        }
-#pragma unroll
-                        for (int c = 3; c >= 1; --c) {
-                            if (c > f && ((m >> c) & 1u)) {
-                                stack[sp] = make_int2(wide_ref(w, c), __float_as_int(t[c]));
-                                ++sp;
-                            }
-                        }
-                        cur = wide_ref(w, f);
-                        pop = false;
-                    }
-                } else if (float4 p0, p1, p2;
-                           leaf_record_hit(bvh, ~cur, sr, orr, best_t, p0, p1, p2)) {
-                    int k = ~cur;
-                    float t, u, v;
-                    if (moller_trumbore(ray.o, ray.d, make_f3(p0.x, p0.y, p0.z),
-                                        make_f3(p1.x, p1.y, p1.z), make_f3(p2.x, p2.y, p2.z),
-                                        t, u, v)
-                        && t > ray.tmin && t < best_t) {
-                        best_k = k;
-                        best_t = t;
-                        if (AnyHit) {
-                            done = true;
-                            break;
-                        }
+        const int live = __popc(__ballot_sync(0xffffffffu, ray_idx >= 0));
+        if (live == 0) break;
+        for (int round = 0; round < budget; ++round) {
+            const int on = __popc(__ballot_sync(0xffffffffu, cur >= 0));
+            if (on * kNodeShareDen <= live * kNodeShareNum) break;
+            if (cur < 0) continue;
+            if (++steps > bound || cur >= bvh.n - 1 || top.full(kWideStack)) {
+                atomicOr(error, top.full(kWideStack) ? kErrStackOverflow : kErrLoopBound);
+                best_k = -1;
+                cur = leaf = kNoNode;
+                top.clear();
+                continue;
+            }
+            const WideNode w = load_wide(bvh.wide, cur);
+            float t[4];
+            bool p[4];
+            wide_test(w, sr, oct, best_t, t, p);
+            cur = wide_descend(w, t, p, stack, top);
+            wide_move_on(cur, leaf, stack, top, best_t);
+        }
+        if (leaf != kNoNode) {
+            const int k = ~leaf;
+            leaf = kNoNode;
+            if (k >= bvh.n) {
+                atomicOr(error, kErrLoopBound);
+                best_k = -1;
+                cur = kNoNode;
+                top.clear();
+            } else {
+                const octant_ray orr = make_octant_ray(sr);
+                float4 p0, p1, p2;
+                float t, u, v;
+                if (leaf_record_hit(bvh, k, sr, orr, best_t, p0, p1, p2) &&
+                    moller_trumbore(sr.o, d, make_f3(p0.x, p0.y, p0.z),
+                                    make_f3(p1.x, p1.y, p1.z), make_f3(p2.x, p2.y, p2.z), t, u,
+                                    v) &&
+                    t > sr.tmin && t < best_t) {
+                    best_k = k;
+                    best_t = t;
+                    if (AnyHit) {
+                        cur = kNoNode;
+                        top.clear();
                     }
                 }
-                if (pop) {
-                    bool resumed = false;
-                    while (sp > 0) {
-                        --sp;
-                        const int2 e = stack[sp];
-                        if (!(__int_as_float(e.y) > best_t)) {
-                            cur = e.x;
-                            resumed = true;
-                            break;
-                        }
-                    }
-                    if (!resumed) done = true;
-                }
+                wide_move_on(cur, leaf, stack, top, best_t);
             }
         }
-        if (done) {
+        if (ray_idx >= 0 && cur == kNoNode && leaf == kNoNode) {
             int id = -1;
             if (best_k >= 0)
                 id = __float_as_int(__ldg(reinterpret_cast<const float*>(bvh.tris + best_k) + 3));
@@ -565,11 +573,20 @@ int launch_trace(lux_ctx* ctx, const lux_bvh* bvh, const float* rays, int nrays,
         if (int st = lbvh_ensure_wide(ctx, const_cast<lux_bvh*>(bvh))) return st;
         const int bps = occupancy_blocks(ctx, AnyHit ? kOccWideAny : kOccWideClosest,
                                          k_trace_wide_persistent<AnyHit>, kTraceThreads);
-        int grid = std::min(ctx->sm_count * bps, (nrays + kTraceThreads - 1) / kTraceThreads);
-        cudaError_t err = cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream);
-        if (err != cudaSuccess) return cuda_fail(err, "ray counter reset");
+        // Up to kSpreadWarps warps per SM a warp takes only as many rays as give each SM its
+        // share: rays that do not wait for others' steps end sooner.  With more warps than
+        // that (four per scheduler) full ones are better: 65,536 rays take 376 us at 16,
+        // 393 us at 24, 419 us at 32.
+        const int spread = ctx->sm_count * kSpreadWarps;
+        const int lanes = std::max(1, std::min(32, nrays / spread + (nrays % spread != 0)));
+        const int per_block = lanes * (kTraceThreads / 32);
+        const int grid = std::min(ctx->sm_count * bps, nrays / per_block + (nrays % per_block != 0));
+        if (static_cast<long long>(grid) * per_block < nrays) {
+            cudaError_t err = cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream);
+            if (err != cudaSuccess) return cuda_fail(err, "ray counter reset");
+        }
         k_trace_wide_persistent<AnyHit><<<grid, kTraceThreads, 0, ctx->stream>>>(
-            bvh->view(), r4, nrays, hit_id, hit_t, ctx->d_counter, ctx->trace_budget,
+            bvh->view(), r4, nrays, hit_id, hit_t, ctx->d_counter, ctx->trace_budget, lanes,
             ctx->d_error);
         ctx->launches += 1;
         return cuda_fail(cudaGetLastError(), "k_trace_wide_persistent");

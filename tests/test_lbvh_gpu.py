@@ -415,3 +415,47 @@ def test_autotune_trace_keeps_results_and_picks_a_candidate(ctx):
     finally:
         ctx.set_option(lux_b200.OPT_TRACE_VARIANT, variant0)
         ctx.set_option(lux_b200.OPT_TRACE_BUDGET, budget0)
+
+
+# Few rays are spread over 16 warps of each of the 148 SMs, by the lanes of a warp: one
+# ray short of, at and past a second lane, full warps, and rays past the resident lanes.
+@pytest.mark.parametrize("count", [1, 2, 3, 31, 33, 2367, 2368, 2369, 4737, 75775, 75777,
+                                   170497])
+def test_few_rays_match_oracle(ctx, oracle, count):
+    tris = W.soup_triangles(3000, seed=41, median_len=0.03)
+    rays = W.uniform_rays(count, seed=42 + count)
+    want_id, want_t = oracle.trace(tris, oracle.build(oracle.triangle_bounds(tris)), rays)
+    bvh = ctx.build_lbvh(tris)
+    got_id, got_t = bvh.trace_closest(rays)
+    assert np.array_equal(got_id, want_id) and np.array_equal(got_t, want_t)
+    assert np.array_equal(bvh.trace_any(rays) >= 0, want_id >= 0)
+
+
+# Triangles at distances that halve towards a corner: a hierarchy of leaf-and-node pairs,
+# whose wide nodes open the node side twice, over many scales in one scene; at scales where
+# a node's grid fits, just fits and does not fit, and for directions whose reciprocals are
+# far from one.
+@pytest.mark.parametrize("scale", [1e-30, 1e-18, 1e-6, 1.0, 1e6, 1e17, 1e22])
+@pytest.mark.parametrize("speed", [1.0, 1e-9, 1e19])
+def test_wide_walk_exact_on_leaf_chains_at_any_scale(ctx, oracle, scale, speed):
+    rng = np.random.default_rng(5)
+    k = np.arange(1500)
+    centre = np.exp2(-(k % 30) * 0.5)[:, None] * (0.2 + rng.random((1500, 3)))
+    verts = centre[:, None, :] * (1 + 0.4 * rng.standard_normal((1500, 3, 3)))
+    tris = (verts.reshape(-1, 9) * scale).astype(np.float32)
+    rays = np.zeros((4000, 8), np.float32)
+    origin = rng.random((4000, 3)) * 1.2
+    target = verts[rng.integers(0, 1500, 4000)].mean(1)
+    d = target - origin
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays[:, 0:3] = origin * scale
+    rays[:, 4:7] = d * speed
+    rays[:10, 4] = 0                              # a parallel axis
+    rays[:, 7] = np.inf
+    rays[2000:, 3] = -0.1 * scale / speed         # hits behind the origin count too
+    with np.errstate(all="ignore"):
+        tree = oracle.build(oracle.triangle_bounds(tris))
+        want_id, want_t = oracle.trace(tris, tree, rays)
+    bvh = ctx.build_lbvh(tris)
+    got_id, got_t = bvh.trace_closest(rays)
+    assert np.array_equal(got_id, want_id) and np.array_equal(got_t, want_t)
