@@ -301,6 +301,15 @@ constexpr int kLookbackBatch = LUX_LOOKBACK_BATCH;   // earlier tiles' words loa
 // prefix, and publishes its own inclusive prefix.  A tile waits only on tiles that were
 // handed out before it (and so are running or done); each wait is bounded and a wait
 // that runs out reports through `error`.
+//
+// The scatter goes through shared memory: the tile's keys and values are first placed in
+// digit order there, so that consecutive threads store runs of a digit at consecutive
+// addresses (stored straight from the ranking order, a warp's 32 stores met 32 sectors).
+template <typename Key>
+constexpr int onesweep_smem() {
+    return kSortTile * static_cast<int>(sizeof(Key) + sizeof(int));
+}
+
 template <typename Key, bool First>
 __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
                                                            const int* vals_in, Key* keys_out,
@@ -311,8 +320,11 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
     static_assert(kSortThreads >= kRadix, "one thread per digit in the look-back");
     constexpr int kWarps = kSortThreads / 32;
     constexpr int kWarpSpan = kSortTile / kWarps;
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    Key* skeys = reinterpret_cast<Key*>(sort_smem);
+    int* svals = reinterpret_cast<int*>(skeys + kSortTile);
     __shared__ unsigned wcount[kWarps][kRadix];
-    __shared__ unsigned gbase[kRadix];
+    __shared__ unsigned loff[kRadix], gbase[kRadix], warp_sums[kRadix / 32];
     __shared__ int tile_s;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -348,21 +360,44 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
         rank[j] = valid ? before + __popc(peers & lt) : 0xffffffffu;
     }
     __syncthreads();
+    unsigned total = 0, incl = 0;
+    unsigned* mine = lookback + static_cast<size_t>(tile) * kRadix + threadIdx.x;
     if (threadIdx.x < kRadix) {
         const int d = threadIdx.x;
-        unsigned total = 0;
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) {
             unsigned c = wcount[w][d];
             wcount[w][d] = total;
             total += c;
         }
-        unsigned* mine = lookback + static_cast<size_t>(tile) * kRadix + d;
+        st_relaxed(mine, tile == 0 ? kTilePrefix | total : kTileAggregate | total);
+        incl = total;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += o;
+        }
+        if (lane == 31) warp_sums[warp] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x < kRadix) {
+        unsigned before = 0;
+        for (int w = 0; w < warp; ++w) before += warp_sums[w];
+        loff[threadIdx.x] = before + incl - total;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) {
+        if (rank[j] == 0xffffffffu) continue;
+        const unsigned d = digit_of(k[j], shift);
+        const unsigned at = loff[d] + wcount[warp][d] + rank[j];   // < kSortTile
+        skeys[at] = k[j];
+        svals[at] = v[j];
+    }
+    if (threadIdx.x < kRadix) {
+        const int d = threadIdx.x;
         unsigned prefix = 0;
-        if (tile == 0) {
-            st_relaxed(mine, kTilePrefix | total);
-        } else {
-            st_relaxed(mine, kTileAggregate | total);
+        if (tile > 0) {
             // Walk back kLookbackBatch tiles at a time (their words are loaded together,
             // so a run of aggregates costs one load latency per batch): take every
             // published word up to the nearest inclusive prefix, and re-read from the
@@ -397,20 +432,162 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
             }
             st_relaxed(mine, kTilePrefix | (prefix + total));
         }
-        gbase[d] = bases[d] + prefix;
+        gbase[d] = bases[d] + prefix - loff[d];
     }
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
-        if (rank[j] == 0xffffffffu) continue;
-        unsigned d = digit_of(k[j], shift);
-        unsigned pos = gbase[d] + wcount[warp][d] + rank[j];
+    const int count = min(kSortTile, n - tile * kSortTile);
+    for (int j = threadIdx.x; j < count; j += kSortThreads) {
+        const Key key = skeys[j];
+        const unsigned pos = gbase[digit_of(key, shift)] + j;
         if (pos >= static_cast<unsigned>(n)) {  // cannot happen for consistent counts
             atomicOr(error, kErrLoopBound);
             continue;
         }
-        keys_out[pos] = k[j];
-        vals_out[pos] = v[j];
+        keys_out[pos] = key;
+        vals_out[pos] = svals[j];
+    }
+}
+
+// Root box, Morton codes and their stable sort by one block, for up to kSmallSort
+// primitives: the keys and (16-bit) input indices stay in shared memory over all passes.
+// A chain of kernels over so few keys is launch and look-back latency and nothing else.
+constexpr int kSmallSort = 8192;
+constexpr int kSmallThreads = 1024;
+
+template <typename Key>
+constexpr int small_sort_smem() {
+    return 2 * kSmallSort * static_cast<int>(sizeof(Key) + sizeof(unsigned short)) +
+           (kSmallThreads / 32) * kRadix * static_cast<int>(sizeof(unsigned));
+}
+
+template <int Kind, typename Key>
+__global__ void __launch_bounds__(kSmallThreads) k_sort_small(const float* prims, int n,
+                                                              Key* codes, int* sorted_ids) {
+    constexpr int kWarps = kSmallThreads / 32;
+    constexpr int kPasses = sizeof(Key) == 4 ? 4 : 8;
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    Key* keys[2];
+    unsigned short* ids[2];
+    keys[0] = reinterpret_cast<Key*>(sort_smem);
+    keys[1] = keys[0] + kSmallSort;
+    unsigned (*wcount)[kRadix] = reinterpret_cast<unsigned (*)[kRadix]>(keys[1] + kSmallSort);
+    ids[0] = reinterpret_cast<unsigned short*>(wcount + kWarps);
+    ids[1] = ids[0] + kSmallSort;
+    __shared__ float part[kWarps][6];
+    __shared__ unsigned loff[kRadix], warp_sums[kRadix / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // The scene box (min and max are order-free).
+    float lo[3] = {INFINITY, INFINITY, INFINITY};
+    float hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        f3 v0, v1, v2;
+        box3 b;
+        load_prim<Kind>(prims, i, v0, v1, v2, b);
+        lo[0] = fminf(lo[0], b.lo.x); lo[1] = fminf(lo[1], b.lo.y); lo[2] = fminf(lo[2], b.lo.z);
+        hi[0] = fmaxf(hi[0], b.hi.x); hi[1] = fmaxf(hi[1], b.hi.y); hi[2] = fmaxf(hi[2], b.hi.z);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+        }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            part[warp][a] = lo[a];
+            part[warp][3 + a] = hi[a];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = part[lane][a];
+        hi[a] = part[lane][3 + a];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+        }
+    }
+    const box3 root{make_f3(lo[0], lo[1], lo[2]), make_f3(hi[0], hi[1], hi[2])};
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        f3 v0, v1, v2;
+        box3 b;
+        load_prim<Kind>(prims, i, v0, v1, v2, b);
+        keys[0][i] = sizeof(Key) == 4 ? static_cast<Key>(morton30(b, root))
+                                      : static_cast<Key>(morton63(b, root));
+        ids[0][i] = static_cast<unsigned short>(i);
+    }
+    // Each warp ranks a run of `rounds` * 32 consecutive keys, as k_onesweep's warps do.
+    const unsigned lt = lanemask_lt();
+    const int rounds = (n + kSmallThreads - 1) / kSmallThreads;
+    const int base = warp * rounds * 32;
+    int cur = 0;
+    for (int p = 0; p < kPasses; ++p) {
+        const int shift = 8 * p;
+        for (int i = threadIdx.x; i < kWarps * kRadix; i += kSmallThreads) (&wcount[0][0])[i] = 0;
+        __syncthreads();
+        unsigned rank[kSmallSort / kSmallThreads];
+#pragma unroll
+        for (int j = 0; j < kSmallSort / kSmallThreads; ++j) {
+            if (j >= rounds) break;
+            const int idx = base + j * 32 + lane;
+            const bool valid = idx < n;
+            const unsigned d = valid ? digit_of(keys[cur][idx], shift) : 0u;
+            const unsigned peers = digit_peers(d, valid);
+            const unsigned before = valid ? wcount[warp][d] : 0u;
+            __syncwarp();
+            if (valid && lane == __ffs(peers) - 1) wcount[warp][d] = before + __popc(peers);
+            __syncwarp();
+            rank[j] = before + __popc(peers & lt);
+        }
+        __syncthreads();
+        unsigned total = 0, incl = 0;
+        if (threadIdx.x < kRadix) {
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+                const unsigned c = wcount[w][threadIdx.x];
+                wcount[w][threadIdx.x] = total;
+                total += c;
+            }
+            incl = total;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off) incl += o;
+            }
+            if (lane == 31) warp_sums[warp] = incl;
+        }
+        __syncthreads();
+        if (threadIdx.x < kRadix) {
+            unsigned before = 0;
+            for (int w = 0; w < warp; ++w) before += warp_sums[w];
+            loff[threadIdx.x] = before + incl - total;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kSmallSort / kSmallThreads; ++j) {
+            if (j >= rounds) break;
+            const int idx = base + j * 32 + lane;
+            if (idx >= n) break;
+            const Key key = keys[cur][idx];
+            const unsigned d = digit_of(key, shift);
+            const unsigned at = loff[d] + wcount[warp][d] + rank[j];   // < n
+            keys[cur ^ 1][at] = key;
+            ids[cur ^ 1][at] = ids[cur][idx];
+        }
+        cur ^= 1;
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        codes[i] = keys[cur][i];
+        sorted_ids[i] = ids[cur][i];
     }
 }
 
@@ -854,8 +1031,8 @@ int morton_and_sort(lux_ctx* ctx, const float* prims, const unsigned* root_ord, 
     for (int p = 0; p < kPasses && err == cudaSuccess; ++p) {
         unsigned* words = lookback + static_cast<size_t>(p) * tiles * kRadix;
         err = chain_launch(ctx, p == 0 ? k_onesweep<Key, true> : k_onesweep<Key, false>, tiles,
-                           kSortThreads, 0, kin, vin, kout, vout, n, 8 * p, bases + p * kRadix,
-                           words, counters + p, ctx->d_error);
+                           kSortThreads, onesweep_smem<Key>(), kin, vin, kout, vout, n, 8 * p,
+                           bases + p * kRadix, words, counters + p, ctx->d_error);
         std::swap(kin, kout);
         std::swap(vin, vout);
     }
@@ -893,16 +1070,47 @@ int climb(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
                      "k_leaf_climb");
 }
 
+// More than 48 KB of dynamic shared memory has to be asked for, once per device and kernel
+// (asking again changes nothing, so calls from several threads are harmless).
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kernel, int bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+template <int Kind, typename Key>
+int hierarchy(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
+    const int n = bvh->n;
+    if (n > 1) {
+        cudaError_t err = chain_launch(ctx, k_karras<Key>, grid_for(n - 1), kThreads, 0,
+                                       static_cast<const Key*>(bvh->codes), n, bvh->nodes,
+                                       bvh->node_parent, bvh->leaf_parent, bvh->node_info);
+        if (err != cudaSuccess) return cuda_fail(err, "k_karras");
+    }
+    return climb<Kind>(ctx, bvh, prims);
+}
+
 template <int Kind, typename Key>
 int build_typed(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
     int n = bvh->n;
     Key* codes = static_cast<Key*>(bvh->codes);
-    unsigned* root_ord = reinterpret_cast<unsigned*>(bvh->root + 8);
-    // Every reset first, so that the kernels follow one another directly.
-    cudaError_t err = cudaMemsetAsync(root_ord, 0xff, 6 * sizeof(unsigned), ctx->stream);
-    if (err == cudaSuccess && n == 1)
+    cudaError_t err = cudaSuccess;
+    if (n == 1)
         // A lone leaf has no parent (the storage may hold a larger earlier tree).
         err = cudaMemsetAsync(bvh->leaf_parent, 0xff, sizeof(int), ctx->stream);
+    if (err != cudaSuccess) return cuda_fail(err, "memset leaf parent");
+    if (n <= kSmallSort) {
+        err = allow_smem(k_sort_small<Kind, Key>, small_sort_smem<Key>());
+        if (err == cudaSuccess)
+            err = chain_launch(ctx, k_sort_small<Kind, Key>, 1, kSmallThreads,
+                               small_sort_smem<Key>(), prims, n, codes, bvh->sorted_ids);
+        if (err != cudaSuccess) return cuda_fail(err, "k_sort_small");
+        return hierarchy<Kind, Key>(ctx, bvh, prims);
+    }
+    unsigned* root_ord = reinterpret_cast<unsigned*>(bvh->root + 8);
+    // Every reset first, so that the kernels follow one another directly.
+    err = cudaMemsetAsync(root_ord, 0xff, 6 * sizeof(unsigned), ctx->stream);
+    if (err == cudaSuccess) err = allow_smem(k_onesweep<Key, true>, onesweep_smem<Key>());
+    if (err == cudaSuccess) err = allow_smem(k_onesweep<Key, false>, onesweep_smem<Key>());
     if (err != cudaSuccess) return cuda_fail(err, "memset root");
     if (int st = reset_sort_scratch<Key>(ctx, n)) return st;
     err = chain_launch(ctx, k_root_reduce<Kind>, stride_grid(ctx, n), kThreads, 0, prims, n,
@@ -910,12 +1118,7 @@ int build_typed(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
     if (err != cudaSuccess) return cuda_fail(err, "k_root_reduce");
     int st = morton_and_sort<Kind, Key>(ctx, prims, root_ord, codes, bvh->sorted_ids, n);
     if (st) return st;
-    if (n > 1) {
-        err = chain_launch(ctx, k_karras<Key>, grid_for(n - 1), kThreads, 0, codes, n, bvh->nodes,
-                           bvh->node_parent, bvh->leaf_parent, bvh->node_info);
-        if (err != cudaSuccess) return cuda_fail(err, "k_karras");
-    }
-    return climb<Kind>(ctx, bvh, prims);
+    return hierarchy<Kind, Key>(ctx, bvh, prims);
 }
 
 }  // namespace
