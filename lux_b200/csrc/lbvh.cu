@@ -7,11 +7,13 @@
 //   3. radix sort      stable LSD sort of (code, input index), 8-bit digits: one
 //                      k_onesweep launch per digit (local ranking, then the tile's digit
 //                      offsets by a decoupled look-back over the earlier tiles)
-//   4. k_karras        Karras 2012 hierarchy over the sorted codes (+ each node's range)
-//   5. k_leaf_climb    leaf boxes + triangle records in sorted order, then one bottom-up
-//                      climb per leaf that writes every child box into its parent: in
-//                      shared memory while a node's leaves lie in the block's own leaves,
-//                      through global memory above that
+//      k_sort_small    1 to 3 in one block, for few primitives
+//   4. k_climb         leaf boxes + triangle records in sorted order, then one bottom-up
+//                      climb per leaf through the binary radix tree of the codes (Karras's
+//                      hierarchy and node numbers), each node written once with both its
+//                      child boxes: within a block's own leaves through shared memory
+//      k_climb_top     the levels above the blocks, through global memory
+// A refit (k_refit) climbs the known hierarchy with new geometry.
 //
 // Reference counterparts (src/): bvh/gpu_bvh.cu:135-149 (codes), 582-584 (sort),
 // 151-180 (hierarchy), 182-214 (bottom-up boxes), 535-613 (build/refit drivers);
@@ -33,11 +35,11 @@ namespace {
 
 // Launch shapes; the LUX_* macros exist so that other shapes can be built and timed
 // against these defaults (results do not depend on them).
-#ifndef LUX_SORT_ITEMS
-#define LUX_SORT_ITEMS 16
-#endif
 #ifndef LUX_CLIMB_THREADS
 #define LUX_CLIMB_THREADS 256
+#endif
+#ifndef LUX_CLIMB_BLOCKS
+#define LUX_CLIMB_BLOCKS 6
 #endif
 #ifndef LUX_LOOKBACK_BATCH
 #define LUX_LOOKBACK_BATCH 8
@@ -48,9 +50,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kRadix = 256;
-constexpr int kSortItems = LUX_SORT_ITEMS;
 constexpr int kSortThreads = LUX_SORT_THREADS;      // threads of a k_onesweep block
-constexpr int kSortTile = kSortThreads * kSortItems;  // keys per tile
 // The allocation-free sort's tiles (its scratch size is part of the ABI): fixed.
 constexpr int kStaticItems = 16;
 constexpr int kStaticTile = kThreads * kStaticItems;
@@ -58,7 +58,6 @@ constexpr int kScanThreads = 1024;
 constexpr int kClimbBound = 160;                 // > max tree depth (64 + 96 bits)
 constexpr int kMaxPasses = 8;                    // 8-bit digits of a 63-bit key
 constexpr int kClimbThreads = LUX_CLIMB_THREADS; // leaves per climb block
-constexpr int kClimbSmem = kClimbThreads * (6 * 8 + 4);   // k_leaf_climb's shared memory
 constexpr long long kLookbackSpins = 1ll << 22;  // bound of one look-back wait
 
 // Relaxed device-scope accesses of the look-back words (each word carries its own value,
@@ -182,16 +181,17 @@ __global__ void __launch_bounds__(kThreads) k_root_reduce(const float* prims, in
         const int a = threadIdx.x;
         float v = part[0][a];
         for (int w = 1; w < kThreads / 32; ++w) v = a < 3 ? fminf(v, part[w][a]) : fmaxf(v, part[w][a]);
-        if (a < 3) atomicMin(root_ord + a, float_to_ordered(v));
-        else atomicMin(root_ord + a, ~float_to_ordered(v));
+        // Maxima of ordered integers (of the complement for the lower corner): zero is their
+        // identity.
+        atomicMax(root_ord + a, a < 3 ? ~float_to_ordered(v) : float_to_ordered(v));
     }
 }
 
 LUX_D box3 decode_root(const unsigned* root_ord) {
-    return box3{make_f3(ordered_to_float(root_ord[0]), ordered_to_float(root_ord[1]),
-                        ordered_to_float(root_ord[2])),
-                make_f3(ordered_to_float(~root_ord[3]), ordered_to_float(~root_ord[4]),
-                        ordered_to_float(~root_ord[5]))};
+    return box3{make_f3(ordered_to_float(~root_ord[0]), ordered_to_float(~root_ord[1]),
+                        ordered_to_float(~root_ord[2])),
+                make_f3(ordered_to_float(root_ord[3]), ordered_to_float(root_ord[4]),
+                        ordered_to_float(root_ord[5]))};
 }
 
 // ---------------------------------------------------------------- 2. Morton codes
@@ -252,25 +252,6 @@ __global__ void __launch_bounds__(kThreads) k_morton_hist(const float* prims, in
     }
 }
 
-// Exclusive prefix of each pass's digit counts: bases[p * kRadix + d] = the number of
-// keys whose pass-p digit is below d.  One block of kRadix threads per pass.
-__global__ void __launch_bounds__(kRadix) k_digit_bases(const unsigned* hist, unsigned* bases) {
-    __shared__ unsigned warp_sums[kRadix / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned v = hist[blockIdx.x * kRadix + threadIdx.x];
-    unsigned incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += o;
-    }
-    if (lane == 31) warp_sums[warp] = incl;
-    __syncthreads();
-    unsigned before = 0;
-    for (int w = 0; w < warp; ++w) before += warp_sums[w];
-    bases[blockIdx.x * kRadix + threadIdx.x] = before + incl - v;
-}
-
 // Lanes of the warp whose digit (and validity) equal this lane's: a validity ballot and
 // one ballot per digit bit, ANDed (cheaper than a general match on sm_100a).
 LUX_D unsigned digit_peers(unsigned d, bool valid) {
@@ -286,7 +267,7 @@ LUX_D unsigned digit_peers(unsigned d, bool valid) {
 }
 
 // Look-back words, 32 bits: 0 while not yet published; kTileAggregate | this tile's own
-// count (at most kSortTile); kTilePrefix | the count over tiles 0..t (at most 2^30, the
+// count (at most the tile's keys); kTilePrefix | the count over tiles 0..t (at most 2^30, the
 // primitive limit, so it fits below the flag bit).
 constexpr unsigned kTileAggregate = 1u << 30;
 constexpr unsigned kTilePrefix = 1u << 31;
@@ -295,7 +276,7 @@ constexpr int kLookbackBatch = LUX_LOOKBACK_BATCH;   // earlier tiles' words loa
 // One stable LSD pass over all keys.  Tiles of kSortTile keys are taken in launch order
 // (an atomic counter), ranked inside the tile as k_sort_downsweep ranks them (per-warp
 // digit counts in input order, so equal digits keep input order), and placed at
-// bases[d] + (digit d's count in earlier tiles) + the rank in the tile.  The count in
+// (keys of smaller digits) + (digit d's count in earlier tiles) + the rank in the tile.  The count in
 // earlier tiles comes from a decoupled look-back: each tile publishes its per-digit
 // count, then walks back over the earlier tiles' words until one holds an inclusive
 // prefix, and publishes its own inclusive prefix.  A tile waits only on tiles that were
@@ -305,30 +286,33 @@ constexpr int kLookbackBatch = LUX_LOOKBACK_BATCH;   // earlier tiles' words loa
 // The scatter goes through shared memory: the tile's keys and values are first placed in
 // digit order there, so that consecutive threads store runs of a digit at consecutive
 // addresses (stored straight from the ranking order, a warp's 32 stores met 32 sectors).
-template <typename Key>
+template <typename Key, int Items>
 constexpr int onesweep_smem() {
-    return kSortTile * static_cast<int>(sizeof(Key) + sizeof(int));
+    return kSortThreads * Items * static_cast<int>(sizeof(Key) + sizeof(int));
 }
 
-template <typename Key, bool First>
+template <typename Key, bool First, int kSortItems>
 __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
                                                            const int* vals_in, Key* keys_out,
                                                            int* vals_out, int n, int shift,
-                                                           const unsigned* bases,
+                                                           const unsigned* hist,
                                                            unsigned* lookback,
                                                            unsigned* tile_counter, int* error) {
     static_assert(kSortThreads >= kRadix, "one thread per digit in the look-back");
+    constexpr int kSortTile = kSortThreads * kSortItems;
     constexpr int kWarps = kSortThreads / 32;
     constexpr int kWarpSpan = kSortTile / kWarps;
     extern __shared__ __align__(16) unsigned char sort_smem[];
     Key* skeys = reinterpret_cast<Key*>(sort_smem);
     int* svals = reinterpret_cast<int*>(skeys + kSortTile);
     __shared__ unsigned wcount[kWarps][kRadix];
-    __shared__ unsigned loff[kRadix], gbase[kRadix], warp_sums[kRadix / 32];
+    __shared__ unsigned loff[kRadix], gbase[kRadix];
+    __shared__ uint2 warp_sums[kRadix / 32];
     __shared__ int tile_s;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) tile_s = static_cast<int>(atomicAdd(tile_counter, 1u));
+    const unsigned all = threadIdx.x < kRadix ? hist[threadIdx.x] : 0u;
     for (int i = threadIdx.x; i < kWarps * kRadix; i += kSortThreads) (&wcount[0][0])[i] = 0;
     __syncthreads();
     const int tile = tile_s;
@@ -360,7 +344,10 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
         rank[j] = valid ? before + __popc(peers & lt) : 0xffffffffu;
     }
     __syncthreads();
-    unsigned total = 0, incl = 0;
+    // Exclusive sums over the digits: of the tile's counts (the keys' places in it) and of
+    // all keys' counts (the digits' places in the output).
+    unsigned total = 0;
+    uint2 incl = make_uint2(0, 0);
     unsigned* mine = lookback + static_cast<size_t>(tile) * kRadix + threadIdx.x;
     if (threadIdx.x < kRadix) {
         const int d = threadIdx.x;
@@ -371,26 +358,34 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
             total += c;
         }
         st_relaxed(mine, tile == 0 ? kTilePrefix | total : kTileAggregate | total);
-        incl = total;
+        incl = make_uint2(total, all);
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += o;
+            const unsigned x = __shfl_up_sync(0xffffffffu, incl.x, off);
+            const unsigned y = __shfl_up_sync(0xffffffffu, incl.y, off);
+            if (lane >= off) {
+                incl.x += x;
+                incl.y += y;
+            }
         }
         if (lane == 31) warp_sums[warp] = incl;
     }
     __syncthreads();
     if (threadIdx.x < kRadix) {
-        unsigned before = 0;
-        for (int w = 0; w < warp; ++w) before += warp_sums[w];
-        loff[threadIdx.x] = before + incl - total;
+        uint2 before = make_uint2(0, 0);
+        for (int w = 0; w < warp; ++w) {
+            before.x += warp_sums[w].x;
+            before.y += warp_sums[w].y;
+        }
+        loff[threadIdx.x] = before.x + incl.x - total;
+        gbase[threadIdx.x] = before.y + incl.y - all;
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kSortItems; ++j) {
         if (rank[j] == 0xffffffffu) continue;
         const unsigned d = digit_of(k[j], shift);
-        const unsigned at = loff[d] + wcount[warp][d] + rank[j];   // < kSortTile
+        const unsigned at = loff[d] + wcount[warp][d] + rank[j];   // < the tile's keys
         skeys[at] = k[j];
         svals[at] = v[j];
     }
@@ -432,7 +427,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
             }
             st_relaxed(mine, kTilePrefix | (prefix + total));
         }
-        gbase[d] = bases[d] + prefix - loff[d];
+        gbase[d] += prefix - loff[d];
     }
     __syncthreads();
     const int count = min(kSortTile, n - tile * kSortTile);
@@ -450,8 +445,10 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
 
 // Root box, Morton codes and their stable sort by one block, for up to kSmallSort
 // primitives: the keys and (16-bit) input indices stay in shared memory over all passes.
-// A chain of kernels over so few keys is launch and look-back latency and nothing else.
-constexpr int kSmallSort = 8192;
+// A chain of kernels over so few keys is launch and look-back latency and nothing else: it
+// takes about 40 us whatever their number, this kernel 15 us for 1,000, 29 us for 5,000 and
+// 44 us for 8,192 (hence the line at 6,144).
+constexpr int kSmallSort = 6144;
 constexpr int kSmallThreads = 1024;
 
 template <typename Key>
@@ -746,72 +743,255 @@ LUX_D int delta(const Key* codes, int i, int j) {
     }
 }
 
-// node_info[i]: (first leaf, last leaf, parent code, unused) of internal node i; the
-// range is written by node i's thread, the parent code by its parent's.
-template <typename Key>
-__global__ void __launch_bounds__(kThreads) k_karras(const Key* codes, int n, BvhNode* nodes,
-                                                     int* node_parent, int* leaf_parent,
-                                                     int4* node_info) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
+// One subtree on its way up: its box, its sorted leaves [first, last], and the common
+// prefix lengths with the neighbours outside it (-1 at the ends of the array).
+struct Subtree {
+    box3 b;
     int first, last;
-    if (i == 0) {
-        first = 0;
-        last = n - 1;
-        node_parent[0] = -1;
-        reinterpret_cast<int*>(node_info)[2] = -1;
-    } else {
-        // determine_range (bvh/gpu_bvh.cu:76-105).
-        int dl = delta(codes, i, i - 1);
-        int dr = delta(codes, i, i + 1);
-        int dir = dr > dl ? 1 : -1;
-        int dmin = min(dl, dr);
-        int lmax = 2;
-        for (;;) {
-            int c = i + dir * lmax;
-            if (c < 0 || c >= n) break;
-            if (delta(codes, i, c) <= dmin) break;
-            lmax <<= 1;
-        }
-        int len = 0;
-        for (int step = lmax >> 1; step > 0; step >>= 1) {
-            int c = i + (len + step) * dir;
-            if (c < 0 || c >= n) continue;
-            if (delta(codes, i, c) > dmin) len += step;
-        }
-        int other = i + len * dir;
-        first = dir < 0 ? other : i;
-        last = dir < 0 ? i : other;
-    }
-    // find_split (bvh/gpu_bvh.cu:107-121).
-    int node_delta = delta(codes, first, last);
-    int split = first;
-    int stride = last - first;
-    do {
-        stride = (stride + 1) >> 1;
-        int mid = split + stride;
-        if (mid < last && delta(codes, first, mid) > node_delta) split = mid;
-    } while (stride > 1);
+    int dl, dr;
+    // The parent splits its range after this leaf: the subtree joins the neighbour it shares
+    // more bits with (the two lengths never agree: the keys with their indices are distinct).
+    LUX_D bool is_left() const { return dr > dl; }
+    LUX_D bool is_root() const { return dl < 0 && dr < 0; }
+    // Karras node number: a left child is numbered by its last leaf, a right child by its
+    // first, the root 0 (bvh/gpu_bvh.cu:151-180 numbers its nodes so).
+    LUX_D int id() const { return is_root() ? 0 : is_left() ? last : first; }
+};
 
-    int left = first == split ? ~split : split;
-    int right = last == split + 1 ? ~(split + 1) : split + 1;
-    reinterpret_cast<int2*>(&nodes[i].ch)[0] = make_int2(left, right);
-    reinterpret_cast<int2*>(node_info + i)[0] = make_int2(first, last);
-    if (left < 0) {
-        leaf_parent[split] = i << 1;
-    } else {
-        node_parent[split] = i << 1;
-        reinterpret_cast<int*>(node_info + split)[2] = i << 1;
-    }
-    if (right < 0) {
-        leaf_parent[split + 1] = (i << 1) | 1;
-    } else {
-        node_parent[split + 1] = (i << 1) | 1;
-        reinterpret_cast<int*>(node_info + split + 1)[2] = (i << 1) | 1;
-    }
+// Joins left = [.., s] and right = [s + 1, ..] and writes the new node's record, parent
+// links included.  ch.z, ch.w of the record: the other end of its leaves and the prefix
+// length beyond it, which the sibling that meets this node in global memory reads.
+LUX_D Subtree join(const Subtree& left, const Subtree& right, BvhNode* nodes, int* leaf_parent,
+                   int* node_parent) {
+    Subtree t;
+    t.b = box_union(left.b, right.b);
+    t.first = left.first;
+    t.last = right.last;
+    t.dl = left.dl;
+    t.dr = right.dr;
+    const int id = t.id(), s = left.last;
+    const bool ll = left.first == left.last, rl = right.first == right.last;
+    const box3 &l = left.b, &r = right.b;
+    const bool side = t.is_left();
+    float4* o = reinterpret_cast<float4*>(nodes + id);
+    stg8(o, make_float4(l.lo.x, l.lo.y, l.lo.z, l.hi.x),
+         make_float4(l.hi.y, l.hi.z, r.lo.x, r.lo.y));
+    stg8(o + 2, make_float4(r.lo.z, r.hi.x, r.hi.y, r.hi.z),
+         make_float4(__int_as_float(ll ? ~s : s), __int_as_float(rl ? ~(s + 1) : s + 1),
+                     __int_as_float(side ? t.first : t.last),
+                     __int_as_float(side ? t.dl : t.dr)));
+    (ll ? leaf_parent : node_parent)[s] = id << 1;
+    (rl ? leaf_parent : node_parent)[s + 1] = (id << 1) | 1;
+    if (t.is_root()) node_parent[0] = -1;
+    return t;
 }
 
-// ---------------------------------------------------------------- 5. boxes bottom-up
+LUX_D void store_root(float* root, const box3& b) {
+    root[0] = b.lo.x; root[1] = b.lo.y; root[2] = b.lo.z;
+    root[3] = b.hi.x; root[4] = b.hi.y; root[5] = b.hi.z;
+}
+
+// Hierarchy and boxes in one bottom-up pass over the sorted codes, in two kernels.  The tree
+// is Karras's (the binary radix tree of the codes), node numbers included, without his
+// searches: the codes are read once.
+//
+// k_climb: one thread per sorted leaf.  The leaf's box (and, for triangles, its sorted
+// record) is formed; then the thread climbs: from the prefix lengths at the two ends of its
+// subtree it knows the leaf after which the parent splits, where the two children meet at a
+// counter in shared memory, and the second to arrive joins them, writes the node and goes
+// on.  A subtree whose sibling reaches beyond the block waits there for nobody: when the
+// block has come to rest, every subtree that is left is listed for k_climb_top.
+//
+// Bound by latency: the gather of the primitives (one random record per leaf), then a chain
+// of some tens of shared-memory steps.
+template <int Kind, typename Key>
+__global__ void __launch_bounds__(kClimbThreads, LUX_CLIMB_BLOCKS) k_climb(
+        const float* prims, int n, const Key* codes, const int* sorted_ids, TriRecord* tris,
+        BvhNode* nodes, int* leaf_parent, int* node_parent, int2* open, int* open_count,
+        float* root, int* error) {
+    constexpr int T = kClimbThreads;
+    // By the subtree's number within the block (a left child: its last leaf, a right child:
+    // its first): box and other end.  The number is free again once the sibling has read it.
+    __shared__ float sbox[6][T];
+    __shared__ int send[T];
+    __shared__ unsigned sflag[T];     // per split: 1 the left child arrived, 2 the right one
+    __shared__ int sdelta[T + 1];     // prefix length of leaves lo + j - 1 and lo + j
+    __shared__ int left_over;
+    const int tid = threadIdx.x;
+    const int lo = blockIdx.x * T;
+    const int k = lo + tid;
+    sflag[tid] = 0;
+    if (tid == 0) {
+        left_over = 0;
+        sdelta[T] = lo + T < n ? delta(codes, lo + T - 1, lo + T) : -1;
+    }
+    sdelta[tid] = k > 0 && k < n ? delta(codes, k - 1, k) : -1;
+    Subtree t{};
+    bool climbing = k < n;
+    if (climbing) {
+        const int pid = sorted_ids[k];
+        if (pid < 0 || pid >= n) {  // cannot happen for a consistent sort
+            atomicOr(error, kErrLoopBound);
+            climbing = false;
+        } else {
+            f3 v0, v1, v2;
+            load_prim_vec<Kind>(prims, n, pid, aligned16(prims), v0, v1, v2, t.b);
+            if (Kind == LUX_PRIM_TRIANGLES) {
+                TriRecord r;
+                r.p0 = make_float4(v0.x, v0.y, v0.z, __int_as_float(pid));
+                r.p1 = make_float4(v1.x, v1.y, v1.z, 0.0f);
+                r.p2 = make_float4(v2.x, v2.y, v2.z, 0.0f);
+                tris[k] = r;
+            }
+            t.first = t.last = k;
+        }
+    }
+    __syncthreads();
+    auto leave = [&](int first, int last) {
+        // Fewer than T: the subtrees are disjoint runs of the block's leaves.
+        open[lo + atomicAdd(&left_over, 1)] = make_int2(first, last);
+    };
+    if (climbing) {
+        t.dl = sdelta[tid];
+        t.dr = sdelta[tid + 1];
+    }
+    while (climbing) {   // at most T - 1 joins in the block
+        if (t.is_root()) {
+            store_root(root, t.b);
+            break;
+        }
+        const bool left = t.is_left();
+        const int s = (left ? t.last : t.first - 1) - lo;   // split, within the block
+        if (s < 0 || s >= T - 1) {
+            leave(t.first, t.last);
+            break;
+        }
+        const int own = left ? s : s + 1, sib = left ? s + 1 : s;
+        sbox[0][own] = t.b.lo.x; sbox[1][own] = t.b.lo.y; sbox[2][own] = t.b.lo.z;
+        sbox[3][own] = t.b.hi.x; sbox[4][own] = t.b.hi.y; sbox[5][own] = t.b.hi.z;
+        send[own] = left ? t.first : t.last;
+        // The block fences order these stores before the counter's add, and the add before
+        // the sibling's values are read (they are also compiler barriers).
+        __threadfence_block();
+        if (atomicAdd(&sflag[s], left ? 1u : 2u) == 0) break;   // the sibling joins them
+        __threadfence_block();
+        Subtree o;
+        o.b = box3{make_f3(sbox[0][sib], sbox[1][sib], sbox[2][sib]),
+                   make_f3(sbox[3][sib], sbox[4][sib], sbox[5][sib])};
+        if (left) {
+            o.first = lo + s + 1;
+            o.last = send[sib];
+            o.dl = t.dr;
+            o.dr = sdelta[o.last + 1 - lo];
+            t = join(t, o, nodes, leaf_parent, node_parent);
+        } else {
+            o.first = send[sib];
+            o.last = lo + s;
+            o.dl = sdelta[o.first - lo];
+            o.dr = t.dl;
+            t = join(o, t, nodes, leaf_parent, node_parent);
+        }
+    }
+    __syncthreads();
+    const unsigned arrived = sflag[tid];   // split lo + tid: one child came, the other is outside
+    if (arrived == 1u) leave(send[tid], lo + tid);
+    else if (arrived == 2u) leave(lo + tid + 1, send[tid + 1]);
+    __syncthreads();
+    if (tid == 0) open_count[blockIdx.x] = left_over;
+}
+
+// Box of a finished subtree from what it wrote: its node's record, or its leaf.
+template <int Kind>
+LUX_D box3 finished_box(bool leaf, int at, const float* prims, int n, const int* sorted_ids,
+                        const TriRecord* tris, const BvhNode* nodes, int4& ch) {
+    box3 b;
+    if (!leaf) {
+        const float4* p = reinterpret_cast<const float4*>(nodes + at);
+        const float4 x = __ldcg(p), y = __ldcg(p + 1), z = __ldcg(p + 2);
+        ch = __ldcg(reinterpret_cast<const int4*>(p + 3));
+        b = box_union(box3{make_f3(x.x, x.y, x.z), make_f3(x.w, y.x, y.y)},
+                      box3{make_f3(y.z, y.w, z.x), make_f3(z.y, z.z, z.w)});
+    } else if (Kind == LUX_PRIM_TRIANGLES) {
+        const float4* p = reinterpret_cast<const float4*>(tris + at);
+        const float4 x = __ldcg(p), y = __ldcg(p + 1), z = __ldcg(p + 2);
+        b = triangle_box(make_f3(x.x, x.y, x.z), make_f3(y.x, y.y, y.z), make_f3(z.x, z.y, z.z));
+    } else {
+        f3 v0, v1, v2;
+        load_prim<Kind>(prims, min(max(sorted_ids[at], 0), n - 1), v0, v1, v2, b);
+    }
+    return b;
+}
+
+// The climb above k_climb's blocks: one warp per block of leaves takes the subtrees that it
+// listed.  The children of a split meet at a counter in global memory (acquire-release,
+// zeroed again by the second arrival), which publishes the first one's record; the second
+// reads it for the box, the other end and the prefix length there.  Some fifteen levels,
+// each one atomic and one dependent load.
+constexpr int kTopThreads = 256;
+template <int Kind, typename Key>
+__global__ void __launch_bounds__(kTopThreads) k_climb_top(
+        const float* prims, int n, const Key* codes, const int* sorted_ids,
+        const TriRecord* tris, BvhNode* nodes, int* leaf_parent, int* node_parent,
+        const int2* open, const int* open_count, int blocks, unsigned* flags, float* root,
+        int* error) {
+    const int block = (blockIdx.x * kTopThreads + threadIdx.x) >> 5;
+    if (block >= blocks) return;
+    const int count = min(open_count[block], kClimbThreads);
+    for (int e = threadIdx.x & 31; e < count; e += 32) {
+        const int2 range = open[block * kClimbThreads + e];
+        Subtree t;
+        t.first = range.x;
+        t.last = range.y;
+        if (t.first < 0 || t.last >= n || t.first > t.last) {  // cannot happen
+            atomicOr(error, kErrLoopBound);
+            return;
+        }
+        t.dl = t.first > 0 ? delta(codes, t.first - 1, t.first) : -1;
+        t.dr = t.last + 1 < n ? delta(codes, t.last, t.last + 1) : -1;
+        int4 ch;
+        t.b = finished_box<Kind>(t.first == t.last, t.first == t.last ? t.first : t.id(), prims,
+                                 n, sorted_ids, tris, nodes, ch);
+        bool climbing = true;
+        for (int level = 0; climbing; ++level) {
+            const bool left = t.is_left();
+            const int s = left ? t.last : t.first - 1;
+            if (level >= kClimbBound || s < 0 || s >= n - 1) {   // cannot happen for sorted codes
+                atomicOr(error, kErrClimbBound);
+                return;
+            }
+            // 1: arrived, 2: and is a leaf.
+            const unsigned prior = atomic_add_acq_rel(flags + s, t.first == t.last ? 3u : 1u);
+            if (prior == 0) break;            // the sibling joins them
+            flags[s] = 0;
+            const int sib = left ? s + 1 : s;
+            Subtree o;
+            const bool leaf = (prior & 2u) != 0;
+            o.b = finished_box<Kind>(leaf, sib, prims, n, sorted_ids, tris, nodes, ch);
+            const int end = leaf ? sib : ch.z;
+            if (end < 0 || end >= n) {        // cannot happen for a consistent record
+                atomicOr(error, kErrClimbBound);
+                return;
+            }
+            if (left) {
+                o.first = sib;
+                o.last = end;
+                o.dl = t.dr;
+                o.dr = !leaf ? ch.w : sib + 1 < n ? delta(codes, sib, sib + 1) : -1;
+                t = join(t, o, nodes, leaf_parent, node_parent);
+            } else {
+                o.first = end;
+                o.last = sib;
+                o.dl = !leaf ? ch.w : sib > 0 ? delta(codes, sib - 1, sib) : -1;
+                o.dr = t.dl;
+                t = join(o, t, nodes, leaf_parent, node_parent);
+            }
+            if (t.is_root()) {
+                store_root(root, t.b);
+                climbing = false;
+            }
+        }
+    }
+}
 
 LUX_D void store_slot(BvhNode* node, int slot, const box3& b) {
     float* f = reinterpret_cast<float*>(node);
@@ -836,7 +1016,20 @@ LUX_D box3 load_slot_cg(const BvhNode* node, int slot) {
     return box3{make_f3(a.x, a.y, b.x), make_f3(b.y, b.z, b.w)};
 }
 
-// One thread per sorted leaf.  The leaf box (and, for triangles, the sorted triangle
+// What a refit's climb reads of a node in one load: its first and last sorted leaf and its
+// parent's code (the node is numbered by one end of its leaves, ch.z is the other).  Made on
+// the first refit of a hierarchy: stored while the nodes are joined, the word more per node
+// takes a build 3 % longer.
+__global__ void __launch_bounds__(kThreads) k_node_info(const BvhNode* nodes,
+                                                        const int* node_parent, int n,
+                                                        int4* node_info) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n - 1) return;
+    const int end = nodes[i].ch.z;
+    node_info[i] = make_int4(min(i, end), max(i, end), node_parent[i], 0);
+}
+
+// Refit: one thread per sorted leaf.  The leaf box (and, for triangles, the sorted triangle
 // record) is written; then the thread climbs: it hands its box to the parent, and the
 // second of the two children to arrive (a counter) unions both and continues upward, so
 // every node box is the union of its children's boxes (merge_bounds_kernel,
@@ -845,20 +1038,20 @@ LUX_D box3 load_slot_cg(const BvhNode* node, int slot) {
 // that range too (a Karras node is numbered by one end of its range), so the hand-over
 // goes through shared memory; above that through the node's slot in global memory with
 // an acquire-release counter, which the second arrival resets to zero.  One 16-byte load
-// of node_info per level gives the node's range and its parent link.
+// of node_info per level gives the node's range and its parent link.  The topology being
+// known, this is one kernel (117 us for 1,048,576 triangles, 22 us for 5,000), where a
+// build's climb and its top take 122 and 27 us.
 template <int Kind>
-__global__ void __launch_bounds__(kClimbThreads) k_leaf_climb(const float* prims, int n,
+__global__ void __launch_bounds__(kClimbThreads) k_refit(const float* prims, int n,
                                                               const int* sorted_ids,
                                                               TriRecord* tris, BvhNode* nodes,
                                                               const int* leaf_parent,
                                                               const int4* node_info,
                                                               unsigned* flags, float* root,
                                                               int* error) {
-    // Per node of the block: each child's box (three float2) and an arrival counter, in
-    // dynamic shared memory (kClimbSmem bytes).
-    extern __shared__ float2 climb_smem[];
-    float2 (*sbox)[2][3] = reinterpret_cast<float2 (*)[2][3]>(climb_smem);
-    unsigned* sflag = reinterpret_cast<unsigned*>(climb_smem + 6 * kClimbThreads);
+    // Per node of the block: each child's box (three float2) and an arrival counter.
+    __shared__ float2 sbox[kClimbThreads][2][3];
+    __shared__ unsigned sflag[kClimbThreads];
     const int lo = blockIdx.x * kClimbThreads;
     sflag[threadIdx.x] = 0;
     __syncthreads();
@@ -981,112 +1174,146 @@ int stride_grid(const lux_ctx* ctx, int count) {
     return std::max(1, std::min(grid_for(count), ctx->sm_count * 8));
 }
 
-// Device scratch of a build: the sort's alternate keys and values, the digit counts and
-// bases of every pass, the tile counters and the look-back words.
+// More than 48 KB of dynamic shared memory has to be asked for, once per device and kernel
+// (asking again changes nothing, so calls from several threads are harmless).
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kernel, int bytes) {
+    if (bytes <= 24 * 1024) return cudaSuccess;   // with the static part within 48 KB
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+// Device scratch of a build: the sort's alternate keys and values; then the words that start
+// at zero (the scene box's ordered words, every pass's digit counts, the tile counters and
+// the look-back words).
 struct SortScratch {
-    size_t key_bytes, val_bytes, counts_bytes, lookback_bytes;
-    size_t total() const { return key_bytes + val_bytes + counts_bytes + lookback_bytes; }
+    size_t key_bytes, val_bytes, zero_bytes, lookback_bytes;
+    size_t total() const { return key_bytes + val_bytes + zero_bytes + lookback_bytes; }
+    // Word offsets within the zeroed part.
+    static constexpr int kRoot = 0, kCounters = 8, kHist = 64;
+    static constexpr int kLookback = kHist + kMaxPasses * kRadix;
 };
 
+// Keys per thread of a k_onesweep block: the more the fewer tiles look back, but the longer
+// each tile's chain of ranking rounds.
+constexpr int kFewKeys = 1 << 20, kFewestKeys = 1 << 19;
+int sort_items(int n) {
+#ifdef LUX_SORT_ITEMS
+    return LUX_SORT_ITEMS;
+#endif
+    return n > kFewKeys ? 16 : n > kFewestKeys ? 8 : 4;
+}
+
 SortScratch sort_scratch(int n, size_t key_size, int passes) {
-    const size_t tiles = static_cast<size_t>((n + kSortTile - 1) / kSortTile);
+    // Tiles of any count up to n (a smaller one may take smaller tiles), so that a rebuild of
+    // fewer primitives never needs more room.
+    size_t tiles = 0;
+    for (int m : {n, std::min(n, kFewKeys), std::min(n, kFewestKeys)}) {
+        const int tile = kSortThreads * sort_items(m);
+        tiles = std::max(tiles, static_cast<size_t>((m + tile - 1) / tile));
+    }
     SortScratch s;
     s.key_bytes = (static_cast<size_t>(n) * key_size + 255) & ~size_t(255);
     s.val_bytes = (static_cast<size_t>(n) * sizeof(int) + 255) & ~size_t(255);
-    // hist[kMaxPasses * kRadix], tile counters[kMaxPasses] (padded), bases[...]
-    s.counts_bytes = 2 * sizeof(unsigned) * kMaxPasses * kRadix + 256;
+    s.zero_bytes = sizeof(unsigned) * SortScratch::kLookback;
     s.lookback_bytes = sizeof(unsigned) * kRadix * tiles * passes;
     return s;
 }
 
 // Morton codes of the primitives into `codes` and their stable sort with the input
-// indices into (codes, vals): k_morton_hist, k_digit_bases, then one k_onesweep per
+// indices into (codes, vals): k_morton_hist, then one k_onesweep per
 // 8-bit digit (an even count, so the result lands back in the caller's arrays).
 template <int Kind, typename Key>
-int morton_and_sort(lux_ctx* ctx, const float* prims, const unsigned* root_ord, Key* codes,
-                    int* vals, int n) {
+int morton_and_sort(lux_ctx* ctx, const float* prims, Key* codes, int* vals, int n) {
     constexpr int kPasses = sizeof(Key) == 4 ? 4 : 8;   // 30 bits: 4 digits; 63 bits: 8
-    const int tiles = grid_for(n, kSortTile);
+    const int items = sort_items(n);
+    const int tiles = grid_for(n, kSortThreads * items);
     const SortScratch layout = sort_scratch(n, sizeof(Key), kPasses);
     int st = ensure_scratch(ctx, layout.total());
     if (st) return st;
     char* s = static_cast<char*>(ctx->scratch);
     Key* keys_alt = reinterpret_cast<Key*>(s);
     int* vals_alt = reinterpret_cast<int*>(s + layout.key_bytes);
-    unsigned* hist = reinterpret_cast<unsigned*>(s + layout.key_bytes + layout.val_bytes);
-    unsigned* bases = hist + kMaxPasses * kRadix;
-    unsigned* counters = bases + kMaxPasses * kRadix;
-    auto* lookback = reinterpret_cast<unsigned*>(
-        s + layout.key_bytes + layout.val_bytes + layout.counts_bytes);
+    unsigned* zeroed = reinterpret_cast<unsigned*>(s + layout.key_bytes + layout.val_bytes);
+    const unsigned* root_ord = zeroed + SortScratch::kRoot;
+    unsigned* hist = zeroed + SortScratch::kHist;
+    unsigned* counters = zeroed + SortScratch::kCounters;
+    unsigned* lookback = zeroed + SortScratch::kLookback;
     // Counts, tile counters and look-back words start at zero (reset by the caller
     // before the chain's first kernel, reset_sort_scratch).
     const int hist_grid = std::max(1, std::min(grid_for(n), ctx->sm_count * 2));
     cudaError_t err = chain_launch(ctx, k_morton_hist<Kind, Key, kPasses>, hist_grid, kThreads,
                                    0, prims, n, root_ord, codes, hist);
-    if (err == cudaSuccess) err = chain_launch(ctx, k_digit_bases, kPasses, kRadix, 0, hist, bases);
     Key* kin = codes;
     int* vin = vals;
     Key* kout = keys_alt;
     int* vout = vals_alt;
     for (int p = 0; p < kPasses && err == cudaSuccess; ++p) {
         unsigned* words = lookback + static_cast<size_t>(p) * tiles * kRadix;
-        err = chain_launch(ctx, p == 0 ? k_onesweep<Key, true> : k_onesweep<Key, false>, tiles,
-                           kSortThreads, onesweep_smem<Key>(), kin, vin, kout, vout, n, 8 * p,
-                           bases + p * kRadix, words, counters + p, ctx->d_error);
+        auto pass = [&](auto first, auto rest, int smem) {
+            err = allow_smem(p == 0 ? first : rest, smem);
+            if (err == cudaSuccess)
+                err = chain_launch(ctx, p == 0 ? first : rest, tiles, kSortThreads, smem, kin,
+                                   vin, kout, vout, n, 8 * p, hist + p * kRadix, words,
+                                   counters + p, ctx->d_error);
+        };
+        if (items == 16)
+            pass(k_onesweep<Key, true, 16>, k_onesweep<Key, false, 16>, onesweep_smem<Key, 16>());
+        else if (items == 8)
+            pass(k_onesweep<Key, true, 8>, k_onesweep<Key, false, 8>, onesweep_smem<Key, 8>());
+        else
+            pass(k_onesweep<Key, true, 4>, k_onesweep<Key, false, 4>, onesweep_smem<Key, 4>());
         std::swap(kin, kout);
         std::swap(vin, vout);
     }
     return cuda_fail(err, "radix sort");
 }
 
-// Zeroes the sort's counts, tile counters and look-back words in ctx's scratch (laid out
-// as morton_and_sort lays it out); grows the scratch first.
+// Zeroes the words of ctx's scratch that start at zero (laid out as morton_and_sort lays it
+// out); grows the scratch first.  *root_ord: the scene box's words.
 template <typename Key>
-int reset_sort_scratch(lux_ctx* ctx, int n) {
+int reset_sort_scratch(lux_ctx* ctx, int n, unsigned** root_ord) {
     constexpr int kPasses = sizeof(Key) == 4 ? 4 : 8;
     const SortScratch layout = sort_scratch(n, sizeof(Key), kPasses);
     if (int st = ensure_scratch(ctx, layout.total())) return st;
-    char* s = static_cast<char*>(ctx->scratch);
-    unsigned* hist = reinterpret_cast<unsigned*>(s + layout.key_bytes + layout.val_bytes);
-    unsigned* counters = hist + 2 * kMaxPasses * kRadix;
-    cudaError_t err = cudaMemsetAsync(hist, 0, sizeof(unsigned) * kMaxPasses * kRadix,
-                                      ctx->stream);
-    if (err == cudaSuccess)
-        err = cudaMemsetAsync(counters, 0, 256 + layout.lookback_bytes, ctx->stream);
-    return err == cudaSuccess ? LUX_OK : cuda_fail(err, "sort scratch reset");
-}
-
-template <int Kind>
-int climb(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
-    if (kClimbSmem > 48 * 1024) {
-        cudaError_t err = cudaFuncSetAttribute(
-            k_leaf_climb<Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClimbSmem);
-        if (err != cudaSuccess) return cuda_fail(err, "k_leaf_climb shared memory");
-    }
-    return cuda_fail(chain_launch(ctx, k_leaf_climb<Kind>, grid_for(bvh->n, kClimbThreads),
-                                  kClimbThreads, kClimbSmem, prims, bvh->n, bvh->sorted_ids,
-                                  bvh->tris, bvh->nodes, bvh->leaf_parent, bvh->node_info,
-                                  bvh->flags, bvh->root, ctx->d_error),
-                     "k_leaf_climb");
-}
-
-// More than 48 KB of dynamic shared memory has to be asked for, once per device and kernel
-// (asking again changes nothing, so calls from several threads are harmless).
-template <typename Kernel>
-cudaError_t allow_smem(Kernel kernel, int bytes) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    unsigned* zeroed = reinterpret_cast<unsigned*>(static_cast<char*>(ctx->scratch) +
+                                                   layout.key_bytes + layout.val_bytes);
+    *root_ord = zeroed + SortScratch::kRoot;
+    const size_t tiles = static_cast<size_t>(grid_for(n, kSortThreads * sort_items(n)));
+    return cuda_fail(cudaMemsetAsync(zeroed, 0,
+                                     layout.zero_bytes + sizeof(unsigned) * kRadix * kPasses * tiles,
+                                     ctx->stream),
+                     "sort scratch reset");
 }
 
 template <int Kind, typename Key>
-int hierarchy(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
-    const int n = bvh->n;
-    if (n > 1) {
-        cudaError_t err = chain_launch(ctx, k_karras<Key>, grid_for(n - 1), kThreads, 0,
-                                       static_cast<const Key*>(bvh->codes), n, bvh->nodes,
-                                       bvh->node_parent, bvh->leaf_parent, bvh->node_info);
-        if (err != cudaSuccess) return cuda_fail(err, "k_karras");
-    }
-    return climb<Kind>(ctx, bvh, prims);
+int climb(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
+    const int blocks = grid_for(bvh->n, kClimbThreads);
+    const Key* codes = static_cast<const Key*>(bvh->codes);
+    cudaError_t err = chain_launch(ctx, k_climb<Kind, Key>, blocks, kClimbThreads, 0, prims,
+                                   bvh->n, codes, bvh->sorted_ids, bvh->tris, bvh->nodes,
+                                   bvh->leaf_parent, bvh->node_parent, bvh->open,
+                                   bvh->open_count, bvh->root, ctx->d_error);
+    if (err == cudaSuccess && blocks > 1)
+        err = chain_launch(ctx, k_climb_top<Kind, Key>, grid_for(blocks, kTopThreads / 32),
+                           kTopThreads, 0, prims, bvh->n, codes, bvh->sorted_ids, bvh->tris,
+                           bvh->nodes, bvh->leaf_parent, bvh->node_parent, bvh->open,
+                           bvh->open_count, blocks, bvh->flags, bvh->root, ctx->d_error);
+    return cuda_fail(err, "climb");
+}
+
+template <int Kind>
+int refit(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
+    cudaError_t err = cudaSuccess;
+    if (!bvh->info_current && bvh->n > 1)
+        err = chain_launch(ctx, k_node_info, grid_for(bvh->n - 1), kThreads, 0, bvh->nodes,
+                           bvh->node_parent, bvh->n, bvh->node_info);
+    if (err == cudaSuccess)
+        err = chain_launch(ctx, k_refit<Kind>, grid_for(bvh->n, kClimbThreads), kClimbThreads, 0,
+                           prims, bvh->n, bvh->sorted_ids, bvh->tris, bvh->nodes,
+                           bvh->leaf_parent, bvh->node_info, bvh->flags, bvh->root,
+                           ctx->d_error);
+    if (err == cudaSuccess) bvh->info_current = true;
+    return cuda_fail(err, "refit");
 }
 
 template <int Kind, typename Key>
@@ -1104,21 +1331,16 @@ int build_typed(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
             err = chain_launch(ctx, k_sort_small<Kind, Key>, 1, kSmallThreads,
                                small_sort_smem<Key>(), prims, n, codes, bvh->sorted_ids);
         if (err != cudaSuccess) return cuda_fail(err, "k_sort_small");
-        return hierarchy<Kind, Key>(ctx, bvh, prims);
+        return climb<Kind, Key>(ctx, bvh, prims);
     }
-    unsigned* root_ord = reinterpret_cast<unsigned*>(bvh->root + 8);
-    // Every reset first, so that the kernels follow one another directly.
-    err = cudaMemsetAsync(root_ord, 0xff, 6 * sizeof(unsigned), ctx->stream);
-    if (err == cudaSuccess) err = allow_smem(k_onesweep<Key, true>, onesweep_smem<Key>());
-    if (err == cudaSuccess) err = allow_smem(k_onesweep<Key, false>, onesweep_smem<Key>());
-    if (err != cudaSuccess) return cuda_fail(err, "memset root");
-    if (int st = reset_sort_scratch<Key>(ctx, n)) return st;
+    unsigned* root_ord = nullptr;
+    if (int st = reset_sort_scratch<Key>(ctx, n, &root_ord)) return st;
     err = chain_launch(ctx, k_root_reduce<Kind>, stride_grid(ctx, n), kThreads, 0, prims, n,
                        root_ord);
     if (err != cudaSuccess) return cuda_fail(err, "k_root_reduce");
-    int st = morton_and_sort<Kind, Key>(ctx, prims, root_ord, codes, bvh->sorted_ids, n);
+    int st = morton_and_sort<Kind, Key>(ctx, prims, codes, bvh->sorted_ids, n);
     if (st) return st;
-    return hierarchy<Kind, Key>(ctx, bvh, prims);
+    return climb<Kind, Key>(ctx, bvh, prims);
 }
 
 }  // namespace
@@ -1130,44 +1352,56 @@ size_t lbvh_scratch_bytes(int n, int morton_bits) {
 int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
     (void)ctx;
     bvh->capacity = std::max(bvh->capacity, std::max(bvh->n, 1));
-    int n = bvh->capacity;
-    size_t key = bvh->morton_bits == 63 ? 8 : 4;
+    const size_t n = static_cast<size_t>(bvh->capacity);
+    const size_t inner = std::max<size_t>(n - 1, 1);
+    const size_t key = bvh->morton_bits == 63 ? 8 : 4;
+    // One allocation for every array (each cudaMalloc of a build is time on the host).
     struct Req {
         void** ptr;
         size_t bytes;
     } reqs[] = {
-        {reinterpret_cast<void**>(&bvh->nodes), sizeof(BvhNode) * std::max(n - 1, 1)},
+        {reinterpret_cast<void**>(&bvh->nodes), sizeof(BvhNode) * inner},
         {reinterpret_cast<void**>(&bvh->tris), sizeof(TriRecord) * n},
         {reinterpret_cast<void**>(&bvh->sorted_ids), sizeof(int) * n},
         {reinterpret_cast<void**>(&bvh->leaf_parent), sizeof(int) * n},
-        {reinterpret_cast<void**>(&bvh->node_parent), sizeof(int) * std::max(n - 1, 1)},
-        {reinterpret_cast<void**>(&bvh->node_info), sizeof(int4) * std::max(n - 1, 1)},
-        {reinterpret_cast<void**>(&bvh->flags), sizeof(unsigned) * std::max(n - 1, 1)},
+        {reinterpret_cast<void**>(&bvh->node_parent), sizeof(int) * inner},
+        {reinterpret_cast<void**>(&bvh->node_info), sizeof(int4) * inner},
+        {reinterpret_cast<void**>(&bvh->flags), sizeof(unsigned) * inner},
+        {reinterpret_cast<void**>(&bvh->open_count),
+         sizeof(int) * static_cast<size_t>(grid_for(bvh->capacity, kClimbThreads))},
         {&bvh->codes, key * n},
         {reinterpret_cast<void**>(&bvh->root), sizeof(float) * 16},
     };
-    for (auto& r : reqs) {
-        cudaError_t err = cudaMalloc(r.ptr, r.bytes);
-        if (err != cudaSuccess) {
-            cudaGetLastError();
-            lbvh_free(bvh);
-            return fail(LUX_ERR_OUT_OF_MEMORY, "lbvh allocation failed");
-        }
+    size_t total = 0;
+    for (const auto& r : reqs) total += (r.bytes + 255) & ~size_t(255);
+    char* base = nullptr;
+    if (cudaMalloc(reinterpret_cast<void**>(&base), total) != cudaSuccess) {
+        cudaGetLastError();
+        lbvh_free(bvh);
+        return fail(LUX_ERR_OUT_OF_MEMORY, "lbvh allocation failed");
     }
-    cudaError_t err = cudaMemset(bvh->flags, 0, sizeof(unsigned) * std::max(n - 1, 1));
+    bvh->arena = base;
+    for (const auto& r : reqs) {
+        *r.ptr = base;
+        base += (r.bytes + 255) & ~size_t(255);
+    }
+    // A build's list of open subtrees ends with the build; the refits' node records are made
+    // after it.
+    static_assert(sizeof(int4) >= sizeof(int2), "open subtrees in the node records' place");
+    bvh->open = reinterpret_cast<int2*>(bvh->node_info);
+    cudaError_t err = cudaMemset(bvh->flags, 0, sizeof(unsigned) * inner);
     if (err == cudaSuccess) err = cudaMemset(bvh->leaf_parent, 0xff, sizeof(int) * n);
     return cuda_fail(err, "lbvh init");
 }
 
 void lbvh_free(lux_bvh* bvh) {
-    void* ptrs[] = {bvh->nodes, bvh->tris, bvh->sorted_ids, bvh->leaf_parent, bvh->node_parent,
-                    bvh->node_info, bvh->flags, bvh->codes, bvh->root, bvh->wide};
+    if (bvh->arena) cudaFree(bvh->arena);
+    if (bvh->wide) cudaFree(bvh->wide);
+    bvh->arena = nullptr;
     bvh->wide = nullptr;
     bvh->wide_capacity = 0;
     bvh->wide_current = false;
-    for (void* p : ptrs) {
-        if (p) cudaFree(p);
-    }
+    bvh->info_current = false;
     bvh->nodes = nullptr;
     bvh->tris = nullptr;
     bvh->sorted_ids = nullptr;
@@ -1175,12 +1409,15 @@ void lbvh_free(lux_bvh* bvh) {
     bvh->node_parent = nullptr;
     bvh->node_info = nullptr;
     bvh->flags = nullptr;
+    bvh->open = nullptr;
+    bvh->open_count = nullptr;
     bvh->codes = nullptr;
     bvh->root = nullptr;
 }
 
 int lbvh_build(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
     bvh->wide_current = false;
+    bvh->info_current = false;
     if (bvh->n <= 0) return LUX_OK;
     bool wide = bvh->morton_bits == 63;
     if (bvh->kind == LUX_PRIM_TRIANGLES) {
@@ -1226,8 +1463,8 @@ int lbvh_attach_triangles(lux_ctx* ctx, lux_bvh* bvh, const float* tris) {
 int lbvh_refit(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
     bvh->wide_current = false;
     if (bvh->n <= 0) return LUX_OK;
-    return bvh->kind == LUX_PRIM_TRIANGLES ? climb<LUX_PRIM_TRIANGLES>(ctx, bvh, prims)
-                                           : climb<LUX_PRIM_AABBS>(ctx, bvh, prims);
+    return bvh->kind == LUX_PRIM_TRIANGLES ? refit<LUX_PRIM_TRIANGLES>(ctx, bvh, prims)
+                                           : refit<LUX_PRIM_AABBS>(ctx, bvh, prims);
 }
 
 namespace {
@@ -1429,7 +1666,7 @@ int lbvh_export(lux_ctx* ctx, const lux_bvh* bvh, uint64_t* codes64, int* left, 
 // lux_lbvh_morton_sort_static keeps every temporary of the Morton sort in this array
 // instead of context scratch, so that a call allocates no device memory.  The module
 // holds it on every GPU it is loaded on until the process exits.  Layout in bytes:
-//   [0, 24)      six ordered-int root words (start at all ones: the identity of min)
+//   [0, 24)      six ordered-int root words (start at zero: the identity of max)
 //   [64, 68)     device error word (starts at zero)
 //   [256, ...)   digit histograms, kRadix x tiles words (fully rewritten every pass)
 //   then keys    LUX_STATIC_SORT_MAX_PRIMS x 8 bytes: 63-bit alternate keys, or both
@@ -1535,7 +1772,7 @@ int lbvh_morton_sort_static(lux_ctx* ctx, const float* prims, int n, int kind, i
     cudaStream_t stream = ctx->stream;
     // The array keeps the previous call's contents: reset the words that must start at a
     // fixed value.  Histograms, keys and values are fully written before they are read.
-    cudaError_t err = cudaMemsetAsync(root_ord, 0xff, 6 * sizeof(unsigned), stream);
+    cudaError_t err = cudaMemsetAsync(root_ord, 0, 6 * sizeof(unsigned), stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(error, 0, sizeof(int), stream);
     if (err != cudaSuccess) return cuda_fail(err, "static sort reset");
     int st;

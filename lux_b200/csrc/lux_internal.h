@@ -44,13 +44,18 @@ struct lux_bvh {
     int kind = 0;           // LUX_PRIM_TRIANGLES / LUX_PRIM_AABBS
     int morton_bits = 30;
     int device = 0;
+    void* arena = nullptr;              // the allocation behind the arrays below
     lux::BvhNode* nodes = nullptr;      // n - 1
     lux::TriRecord* tris = nullptr;     // n (triangle BVHs)
     int* sorted_ids = nullptr;          // n
     int* leaf_parent = nullptr;         // n
-    int* node_parent = nullptr;         // n - 1
+    int* node_parent = nullptr;         // n - 1: parent code
     int4* node_info = nullptr;          // n - 1: first and last sorted leaf, parent code
+    bool info_current = false;          // node_info matches the hierarchy (cleared by builds)
     unsigned* flags = nullptr;          // n - 1, zero between passes
+    int2* open = nullptr;               // n: leaf ranges of the subtrees a climb block leaves
+                                        // (in node_info's memory)
+    int* open_count = nullptr;          // their number, per climb block
     void* codes = nullptr;              // n sorted codes (uint32 or uint64)
     float* root = nullptr;              // 6
     lux::WideNode* wide = nullptr;      // capacity - 1, built on demand for ray queries

@@ -459,3 +459,31 @@ def test_wide_walk_exact_on_leaf_chains_at_any_scale(ctx, oracle, scale, speed):
     bvh = ctx.build_lbvh(tris)
     got_id, got_t = bvh.trace_closest(rays)
     assert np.array_equal(got_id, want_id) and np.array_equal(got_t, want_t)
+
+
+# The climb's 256-leaf blocks, one leaf more and one less, and a tree of a chain whose
+# subtrees leave their block one leaf at a time; then a refit of each.
+@pytest.mark.parametrize("n", [3, 255, 256, 257, 511, 769, 6144, 6145])
+@pytest.mark.parametrize("kind", [lux_b200.PRIM_TRIANGLES, lux_b200.PRIM_AABBS])
+@pytest.mark.parametrize("chain", [False, True])
+def test_climb_blocks_match_oracle(ctx, oracle, n, kind, chain):
+    tris = W.soup_triangles(n, seed=51)
+    if chain:
+        tris *= np.exp2(-(np.arange(n) % 9)).astype(np.float32)[:, None]
+    moved = W.jitter_triangles(tris, seed=52, sigma=1e-3)
+    boxes, moved_boxes = oracle.triangle_bounds(tris), oracle.triangle_bounds(moved)
+    prims, moved_prims = (tris, moved) if kind == lux_b200.PRIM_TRIANGLES else (boxes, moved_boxes)
+    bvh = ctx.build_lbvh(prims, kind=kind)
+    got = bvh.download()
+    _assert_tree_equal(got, oracle.build(boxes))
+    for _ in range(2):                            # the arrival counters are left at zero
+        bvh.refit(moved_prims)
+        after = bvh.download()
+        left, right, nb = after.node_left[:n - 1], after.node_right[:n - 1], after.node_bounds
+        assert np.array_equal(after.node_left, got.node_left)
+        assert np.array_equal(nb[n - 1:], moved_boxes[after.sorted_ids])
+        assert np.array_equal(nb[:n - 1], np.concatenate(
+            [np.minimum(nb[left, :3], nb[right, :3]), np.maximum(nb[left, 3:], nb[right, 3:])], 1))
+        assert bvh.validate()[0]
+    bvh.rebuild(moved_prims)
+    _assert_tree_equal(bvh.download(), oracle.build(moved_boxes))
