@@ -138,13 +138,9 @@ int check_ctx(lux_ctx* ctx) {
 
 // Waits for the stream, then reports (and clears) the device error word.
 int sync_and_check(lux_ctx* ctx) {
-    cudaError_t err = cudaStreamSynchronize(ctx->stream);
-    if (err != cudaSuccess) return lux::cuda_fail(err, "stream synchronize");
     int word = 0;
-    err = cudaMemcpy(&word, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) return lux::cuda_fail(err, "error word read");
+    if (int st = lux::wait_error_word(ctx, &word)) return st;
     if (word) {
-        cudaMemset(ctx->d_error, 0, sizeof(int));
         std::string what;
         if (word & lux::kErrClimbBound) what += " bottom-up level bound exceeded;";
         if (word & lux::kErrStackOverflow) what += " traversal stack overflow;";
@@ -279,6 +275,16 @@ int ensure_scratch(lux_ctx* ctx, size_t bytes) {
     return LUX_OK;
 }
 
+int wait_error_word(lux_ctx* ctx, int* word) {
+    cudaError_t err = cudaMemcpyAsync(ctx->h_words, ctx->d_error, sizeof(int),
+                                      cudaMemcpyDeviceToHost, ctx->stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
+    if (err != cudaSuccess) return cuda_fail(err, "stream synchronize");
+    *word = static_cast<int>(ctx->h_words[0] & 0xffffffffu);
+    if (*word) cudaMemset(ctx->d_error, 0, sizeof(int));
+    return LUX_OK;
+}
+
 }  // namespace lux
 
 extern "C" {
@@ -315,6 +321,9 @@ int lux_ctx_create(lux_ctx** out, int device, void* stream) {
     if (err == cudaSuccess) err = cudaMemset(ctx->d_error, 0, sizeof(int));
     if (err == cudaSuccess) err = cudaMalloc(&ctx->d_counter, 64);
     if (err == cudaSuccess) err = cudaMemset(ctx->d_counter, 0, 64);
+    if (err == cudaSuccess)
+        err = cudaMallocHost(reinterpret_cast<void**>(&ctx->h_words), 64);
+    if (err == cudaSuccess) std::memset(ctx->h_words, 0, 64);
     if (err != cudaSuccess) {
         if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
         delete ctx;
@@ -332,6 +341,7 @@ int lux_ctx_destroy(lux_ctx* ctx) {
     if (ctx->staging) cudaFree(ctx->staging);
     if (ctx->d_error) cudaFree(ctx->d_error);
     if (ctx->d_counter) cudaFree(ctx->d_counter);
+    if (ctx->h_words) cudaFreeHost(ctx->h_words);
     lux::render_runtime_free(ctx);
     if (ctx->copy_stream) {
         cudaStreamSynchronize(ctx->copy_stream);
@@ -756,7 +766,7 @@ static int render_common(lux_ctx* ctx, const lux_scene* scene, const lux_render_
     if (st) return st;
     st = lux::render(ctx, scene, *req, static_cast<float*>(d_out), per_sample);
     if (st) return st;
-    st = finish_call(ctx, staging);
+    st = staging.finish();
     if (st) return st;
     return sync_and_check(ctx);
 }
@@ -791,7 +801,7 @@ int lux_render_aovs(lux_ctx* ctx, const lux_scene* scene, const lux_render_reque
                      static_cast<float*>(d_shadow), static_cast<float*>(d_ng),
                      static_cast<float*>(d_ns));
     if (st) return st;
-    st = finish_call(ctx, staging);
+    st = staging.finish();
     if (st) return st;
     return sync_and_check(ctx);
 }
@@ -828,7 +838,7 @@ int lux_render_path_log(lux_ctx* ctx, const lux_scene* scene, const lux_render_r
                      nullptr, capacity > 0 ? static_cast<lux_path_log_record*>(d_records) : nullptr,
                      static_cast<unsigned long long*>(d_count), capacity);
     if (st) return st;
-    st = finish_call(ctx, staging);
+    st = staging.finish();
     if (st) return st;
     st = sync_and_check(ctx);
     if (st) return st;
@@ -873,7 +883,7 @@ int lux_scene_select_lights(lux_ctx* ctx, const lux_scene* scene, int32_t light_
                             static_cast<const float*>(d_u), n, static_cast<int32_t*>(d_index),
                             static_cast<float*>(d_pmf), static_cast<float*>(d_eval));
     if (st) return st;
-    st = finish_call(ctx, staging);
+    st = staging.finish();
     if (st) return st;
     return sync_and_check(ctx);
 }
@@ -903,7 +913,7 @@ int lux_render_traversal_stats(lux_ctx* ctx, const lux_scene* scene,
     st = lux::render(ctx, scene, *req, static_cast<float*>(d_film), false, nullptr, nullptr,
                      nullptr, nullptr, nullptr, 0, static_cast<unsigned long long*>(d_walk));
     if (st) return st;
-    st = finish_call(ctx, staging);
+    st = staging.finish();
     if (st) return st;
     st = sync_and_check(ctx);
     if (st) return st;

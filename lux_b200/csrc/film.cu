@@ -76,19 +76,18 @@ extern "C" int lux_film_encode(lux_ctx* ctx, const float* film_sum, int32_t widt
         return dev;
     };
     const bool in_dev = on_device(film_sum), out_dev = on_device(out);
-    void* d_in = const_cast<float*>(film_sum);  // replaced by staging when on the host
+    void* d_in = const_cast<float*>(film_sum);  // replaced by scratch when on the host
     void* d_out = out;
     cudaStream_t s = ctx->stream;
+    // The context's scratch, kept from call to call: allocations from the stream's default
+    // pool are mapped anew after every wait.
+    const size_t in_room = in_dev ? 0 : (in_bytes + 255) & ~size_t(255);
+    if (int st = lux::ensure_scratch(ctx, in_room + (out_dev ? 0 : out_bytes))) return st;
+    if (!in_dev) d_in = ctx->scratch;
+    if (!out_dev) d_out = static_cast<char*>(ctx->scratch) + in_room;
     cudaError_t err = cudaSuccess;
-    if (!in_dev) err = cudaMallocAsync(&d_in, in_bytes, s);
-    if (err == cudaSuccess && !out_dev) err = cudaMallocAsync(&d_out, out_bytes, s);
-    if (err == cudaSuccess && !in_dev)
-        err = cudaMemcpyAsync(d_in, film_sum, in_bytes, cudaMemcpyHostToDevice, s);
-    if (err != cudaSuccess) {
-        if (!in_dev && d_in != film_sum) cudaFreeAsync(d_in, s);
-        if (!out_dev && d_out != out) cudaFreeAsync(d_out, s);
-        return lux::cuda_fail(err, "film staging");
-    }
+    if (!in_dev) err = cudaMemcpyAsync(d_in, film_sum, in_bytes, cudaMemcpyHostToDevice, s);
+    if (err != cudaSuccess) return lux::cuda_fail(err, "film staging");
     const float inv_spp = spp > 0 ? 1.0f / static_cast<float>(spp) : 0.0f;
     const int grid = static_cast<int>(
         std::min<size_t>((pixels + lux::kEncodeThreads - 1) / lux::kEncodeThreads,
@@ -99,8 +98,6 @@ extern "C" int lux_film_encode(lux_ctx* ctx, const float* film_sum, int32_t widt
     err = cudaGetLastError();
     if (err == cudaSuccess && !out_dev)
         err = cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, s);
-    if (!in_dev) cudaFreeAsync(d_in, s);
-    if (!out_dev) cudaFreeAsync(d_out, s);
     if (err == cudaSuccess) err = cudaStreamSynchronize(s);
     return lux::cuda_fail(err, "film encode");
 }

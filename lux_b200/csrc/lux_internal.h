@@ -15,6 +15,9 @@ struct lux_ctx {
     int* d_error = nullptr;          // device error word (lux::kErr* bits)
     int64_t launches = 0;            // kernels launched through this context
     unsigned* d_counter = nullptr;   // device work counter (persistent kernels)
+    // Pinned words that results are read back through: [0] the error word, [1] and [2] the
+    // last render's rays and shadow segments (valid once the stream has been waited for).
+    unsigned long long* h_words = nullptr;
     // Tunables (lux_ctx_set_option).
     int trace_variant = 0;           // lux::kTrace* (auto: wide persistent)
     int trace_budget = 16;           // traversal steps per refill round (ray queries)
@@ -116,6 +119,8 @@ inline int occupancy_blocks(lux_ctx* ctx, int slot, Kernel kernel, int threads) 
 int fail(int status, const std::string& message);
 int cuda_fail(cudaError_t err, const char* what);
 int ensure_scratch(lux_ctx* ctx, size_t bytes);
+// Waits for the stream and reads (and clears) the device error word, in one wait.
+int wait_error_word(lux_ctx* ctx, int* word);
 
 // LBVH (lbvh.cu).  prims are device pointers.
 int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh);

@@ -105,6 +105,7 @@ int camera_perspective(const float* origin, const float* look_at, float vfov, fl
 // log_count the render zeroes and counts every vertex on), the bounce kernels are the
 // debug ones.  walk_counts (device, 3 counters, zeroed by the render) also selects
 // them and receives the box tests, triangle tests and instance visits of every walk.
+// Everything is queued on the context's stream; the caller waits for it.
 int render(lux_ctx* ctx, const lux_scene* scene, const lux_render_request& req, float* out,
            bool per_sample, float* aov_shadow = nullptr, float* aov_ng = nullptr,
            float* aov_ns = nullptr, lux_path_log_record* log = nullptr,

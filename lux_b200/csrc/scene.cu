@@ -1173,13 +1173,9 @@ int scene_update_mesh(lux_ctx* ctx, lux_scene* s, int mesh, const float* vertice
         if (view_changed) *view_changed = true;
     }
     if (!sync) return LUX_OK;
-    err = cudaStreamSynchronize(stream);
-    if (err != cudaSuccess) return cuda_fail(err, "mesh update");
     int word = 0;
-    err = cudaMemcpy(&word, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) return cuda_fail(err, "mesh update");
+    if (int st = wait_error_word(ctx, &word)) return st;
     if (word) {
-        cudaMemset(ctx->d_error, 0, sizeof(int));
         return fail(LUX_ERR_DEVICE_CHECK, "mesh update: device check failed");
     }
     return LUX_OK;

@@ -51,7 +51,6 @@ struct Runtime {
     PathPool pool[kRenderLanes];
     int* counts[kRenderLanes] = {};      // kMaxDepthSlots * kSlots per lane
     unsigned long long* rays = nullptr;  // [0] camera + extension, [1] shadow segments
-    long long last_counts[2] = {0, 0};
     int lanes = 0;                       // lanes allocated
     cudaStream_t stream[kRenderLanes] = {};   // lanes 1.. (lane 0 runs on the context's)
     cudaEvent_t ev_setup = nullptr;
@@ -305,10 +304,7 @@ void runtime_release(Runtime* rt) {
         if (rt->ev_flush[l]) cudaEventDestroy(rt->ev_flush[l]);
         if (rt->stream[l]) cudaStreamDestroy(rt->stream[l]);
     }
-    long long keep[2] = {rt->last_counts[0], rt->last_counts[1]};
     *rt = Runtime{};
-    rt->last_counts[0] = keep[0];
-    rt->last_counts[1] = keep[1];
 }
 
 }  // namespace
@@ -419,9 +415,8 @@ int select_lights(lux_ctx* ctx, const lux_scene* scene, int sampler, const float
 }
 
 int render_ray_counts(lux_ctx* ctx, int64_t* counts) {
-    pt::Runtime* rt = pt::runtime_of(ctx);
-    counts[0] = rt ? rt->last_counts[0] : 0;
-    counts[1] = rt ? rt->last_counts[1] : 0;
+    counts[0] = static_cast<int64_t>(ctx->h_words[1]);
+    counts[1] = static_cast<int64_t>(ctx->h_words[2]);
     return LUX_OK;
 }
 
@@ -564,12 +559,9 @@ int render(lux_ctx* ctx, const lux_scene* scene, const lux_render_request& req, 
         if (err == cudaSuccess) err = cudaStreamWaitEvent(s0, rt.ev_end[l], 0);
         if (err != cudaSuccess) return cuda_fail(err, "render lanes");
     }
-    unsigned long long counts[2];
-    err = cudaMemcpyAsync(counts, rt.rays, 16, cudaMemcpyDeviceToHost, s0);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(s0);
+    // The caller waits for the stream; the counts are on the host then.
+    err = cudaMemcpyAsync(ctx->h_words + 1, rt.rays, 16, cudaMemcpyDeviceToHost, s0);
     if (err != cudaSuccess) return cuda_fail(err, "render");
-    rt.last_counts[0] = static_cast<long long>(counts[0]);
-    rt.last_counts[1] = static_cast<long long>(counts[1]);
     return LUX_OK;
 }
 
