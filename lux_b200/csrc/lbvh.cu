@@ -1371,6 +1371,9 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
          sizeof(int) * static_cast<size_t>(grid_for(bvh->capacity, kClimbThreads))},
         {&bvh->codes, key * n},
         {reinterpret_cast<void**>(&bvh->root), sizeof(float) * 16},
+        // Triangles are built to be traced: their 4-wide nodes have their place from the start.
+        {reinterpret_cast<void**>(&bvh->wide),
+         bvh->kind == LUX_PRIM_TRIANGLES ? sizeof(WideNode) * inner : 0},
     };
     size_t total = 0;
     for (const auto& r : reqs) total += (r.bytes + 255) & ~size_t(255);
@@ -1385,6 +1388,8 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
         *r.ptr = base;
         base += (r.bytes + 255) & ~size_t(255);
     }
+    bvh->wide_capacity = bvh->kind == LUX_PRIM_TRIANGLES ? static_cast<int>(inner) : 0;
+    if (!bvh->wide_capacity) bvh->wide = nullptr;
     // A build's list of open subtrees ends with the build; the refits' node records are made
     // after it.
     static_assert(sizeof(int4) >= sizeof(int2), "open subtrees in the node records' place");
@@ -1395,8 +1400,8 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
 }
 
 void lbvh_free(lux_bvh* bvh) {
+    if (bvh->wide && bvh->kind != LUX_PRIM_TRIANGLES) cudaFree(bvh->wide);
     if (bvh->arena) cudaFree(bvh->arena);
-    if (bvh->wide) cudaFree(bvh->wide);
     bvh->arena = nullptr;
     bvh->wide = nullptr;
     bvh->wide_capacity = 0;
