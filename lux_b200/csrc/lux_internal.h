@@ -94,8 +94,8 @@ enum : int {
     kOccWideAny = 1,
     kOccPersistClosest = 2,
     kOccPersistAny = 3,
-    kOccExtendRefill = 4,
-    kOccShadowRefill = 5
+    kOccWalk = 4,
+    kOccWalkMany = 5
 };
 
 // Resident blocks per SM of `kernel` at `threads` threads on the context's device (at

@@ -197,6 +197,18 @@ struct Camera {  // camera/camera.h:29-38 (perspective)
     float lens_radius;
 };
 
+// Material types by the code that shades them.
+constexpr int kClasses = 5;       // Lambert, thin Lambert, GGX, dielectric, pass-through
+LUX_HD int material_class(int type) {
+    switch (type) {
+        case kLambert: return 0;
+        case kThinLambert: return 1;
+        case kGgx: return 2;
+        case kDielectric: return 3;
+        default: return 4;
+    }
+}
+
 struct SceneView {
     const Material* materials;
     int material_count;
@@ -231,6 +243,7 @@ struct SceneView {
     const int* primitive_light;      // scene triangle -> light index (-1 none, -2 several)
     bool has_two_level;
     bool has_passthrough;            // some material is an interface or transparent filter
+    bool one_class;                  // every material shades by the same code
     Camera camera;
 };
 

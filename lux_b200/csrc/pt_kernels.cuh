@@ -21,26 +21,26 @@ namespace pt {
 
 constexpr int kThreads = 256;
 constexpr int kStack = 72;
-constexpr int kClasses = 5;       // Lambert, thin Lambert, GGX, dielectric, pass-through
 constexpr int kShadowSegments = 1024;
 
-// SoA path state and queues (capacity paths, 16-byte records).
+// Path state and queues.  A path's records are read and written at places that the queues
+// pick, so what is used together lies together, in whole 32-byte sectors moved by one
+// instruction each.
+//   state   4 words of 16 bytes a path: throughput.rgb and eta scale; previous sample's
+//           position and pdf; PCG state lo/hi, depth | passthrough << 16, measure | flags << 8;
+//           pixel, sample, PCG increment lo/hi (the last does not change)
+//   ray     2: origin and t_min; direction and t_max
+//   shadow  4: origin and t_max; direction and ignored primitive (int bits); then, in a scene
+//           without pass-through surfaces, the radiance to add when the ray arrives; else
+//           contribution.rgb and MIS weight, and the throughput at the vertex
 struct PathPool {
     int capacity = 0;
-    float4* thr_eta = nullptr;      // throughput.rgb, eta scale
+    float4* state = nullptr;
+    float4* ray = nullptr;
+    float4* shadow = nullptr;
     float4* rad = nullptr;          // radiance.rgb
-    float4* prev = nullptr;         // previous sample reference position, pdf
-    int4* meta = nullptr;           // pixel, sample, depth | passthrough << 16, measure | flags << 8
-    uint4* rng = nullptr;           // PCG state lo/hi, inc lo/hi
-    float4* ray_o = nullptr;        // origin, t_min
-    float4* ray_d = nullptr;        // direction, t_max
     float4* hit = nullptr;          // t, u, v, primitive (int bits)
-    float4* sh_o = nullptr;         // origin, t_max
-    float4* sh_d = nullptr;         // direction, ignored primitive (int bits)
-    float4* sh_c = nullptr;         // contribution.rgb, mis weight
-    float4* sh_t = nullptr;         // throughput.rgb at the vertex
     int* qray[2] = {nullptr, nullptr};
-    int* qmat = nullptr;            // kClasses * capacity
     int* qshadow = nullptr;
 };
 
@@ -54,6 +54,13 @@ LUX_D unsigned lanemask_lt() {
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
+}
+
+// 32 bytes from a 32-byte aligned address that this kernel may also write.
+LUX_D void ld8(const float4* p, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z),
+                   "=f"(b.w) : "l"(p) : "memory");
 }
 
 // Warp-aggregated append: lanes with the same queue share one atomic.
@@ -269,232 +276,211 @@ LUX_D SceneHit scene_closest(const SceneView& sc, f3 o, f3 d, float tmin, float 
     return h;
 }
 
-// scene_closest as a resumable walk: step() advances by one node visit or one triangle
-// (or instance) test, followed by the pops it enables, so a kernel can interleave many
-// walks per warp and refill lanes as walks finish.  The TLAS is walked over its binary
-// nodes (a TLAS of at most kFlatTlas instances is entered leaf by leaf: init() tests every
-// leaf box and defers the passing ones in leaf order), each BLAS over its quantised 4-wide
-// nodes (lux_wide.cuh: every leaf the binary
-// walk reaches is reached in the same left-first order and accepted by the exact test of
-// its own box, the triangle's box formed from its record), so the leaves tested and the
-// best hit after each are those of scene_closest / blas_closest above and the result is
-// the same.  The stacks live apart from the scalar state, which then stays in registers.
-constexpr int kWideBlasStack = 96;   // three deferred children per 4-wide level
+// scene_closest as a resumable walk, for kernels whose warps interleave many walks.  The
+// TLAS is walked over its binary nodes (a TLAS of at most kFlatTlas instances is entered
+// leaf by leaf: its leaf boxes are tested in leaf order when the walk starts), each BLAS
+// over its quantised 4-wide nodes (lux_wide.cuh: every leaf the binary walk reaches is
+// reached in the same left-first order and accepted by the exact test of its own box, the
+// triangle's box formed from its record), so the leaves tested and the best hit after each
+// are those of scene_closest / blas_closest above and the result is the same.  (The TLAS
+// over its 4-wide nodes: 257 instances 2 % faster, Cornell 4 % and the heavy scene 6 %
+// slower, by the spills of a second node test in the kernel.)
+//
+// A walk is at a BLAS node (cur >= 0), waits at a BLAS leaf (leaf, and perhaps a second one
+// in cur), or is done with its BLAS (at_rest).  A leaf may wait while nodes are tested: node
+// tests only have to keep every leaf the reference reaches, which they do under any bound
+// not below the current one, and leaves are tested in order under the bound of their turn.
+// The world-space ray is not kept: tlas() is handed it again when a BLAS is left.  The
+// stacks live apart from the scalar state, which then stays in registers.
+constexpr int kWideStackPt = 100;     // three deferred children per 4-wide level
 constexpr int kFlatTlas = 4;          // TLAS leaves tested together when a walk starts
 
 struct WalkStacks {  // deferred (node ref, entry t bits), TLAS and BLAS
     int2 t[kStack];
-    int2 b[kWideBlasStack];
+    int2 b[kWideStackPt];
+};
+
+struct WalkRay {
+    f3 o, d;
+    float tmin, tmax;
+    int ignored;                  // scene triangle skipped, -1 none
 };
 
 struct TwoLevelWalk {
-    f3 o, d;
-    float tmin;
-    slab_ray sr;
     SceneHit hit;                 // best so far (hit.t is the current bound)
-    int ign_instance, ign_local;
-    int t_cur, t_sp;
-    unsigned t_steps;             // steps of the walk (bounded by 2n + 64 per level)
-    bool in_blas;
-    const WideNode* b_wide;
-    const TriRecord* b_tris;
-    int b_n, b_cur, b_ignored, b_first;
-    WideTop b_top;
-    unsigned b_steps;
-    f3 lo, ld;
+    // The BLAS being walked, and the ray in its space.
     slab_ray lsr;
-    unsigned lneg;                // octant of the object-space ray (wide_octant)
-    bool done;
-    bool any_hit;                 // end at the first accepted triangle (occlusion only)
+    f3 ld;
+    unsigned oct;                 // octant of the object-space ray (wide_octant)
+    const WideNode* wide;
+    const TriRecord* tris;
+    int n, ignored, first;
+    int cur, leaf;
+    unsigned steps;               // bounded by 2n + 64 per BLAS
+    WideTop top;
+    WideTop t_top;                // deferred TLAS children
 
-    LUX_D void init(const SceneView& sc, WalkStacks& k, f3 ro, f3 rd, float rtmin, float rtmax,
-                    int ignored, bool first_hit = false) {
-        any_hit = first_hit;
-        o = ro;
-        d = rd;
-        tmin = rtmin;
-        hit = SceneHit{};
-        hit.t = rtmax;
-        in_blas = false;
-        t_sp = 0;
-        t_steps = 0;
-        done = true;
-        if (!sc.has_two_level) return;
-        ign_instance = -1;
-        ign_local = -1;
-        if (ignored >= 0) {
-            float4 v1 = __ldg(&sc.tris[ignored].v1);
-            float4 v2 = __ldg(&sc.tris[ignored].v2);
-            ign_instance = __float_as_int(v1.w);
-            ign_local = __float_as_int(v2.w);
-        }
-        sr = make_slab_ray(ray3{o, tmin, d, rtmax});
-        float tn;
-        if (!slab_hit(sr, load_root(sc.tlas.root), hit.t, tn)) return;
-        t_cur = sc.tlas.n == 1 ? ~0 : 0;
-        done = false;
-        const BvhView& tl = sc.tlas;
-        if (tl.n >= 2 && tl.n <= kFlatTlas) {
-            // A TLAS of a few instances: every leaf box is tested here, in leaf order (the
-            // binary walk's left-first order), and the passing leaves after the first are
-            // deferred with their entry t as the walk defers children, so the walk enters
-            // the same instances under the same bounds without stepping through the
-            // TLAS's internal nodes (a leaf box passes under a bound exactly when every
-            // box above it does).
-            int first = -1;
-            float first_t = 0.0f;
-            for (int j = tl.n - 1; j >= 0; --j) {
-                float te;
-                if (slab_hit(sr, leaf_box(tl, j), hit.t, te)) {
-                    if (first >= 0) k.t[t_sp++] = make_int2(~first, __float_as_int(first_t));
-                    first = j;
-                    first_t = te;
-                }
-            }
-            if (first < 0) {
-                done = true;
-                return;
-            }
-            t_cur = ~first;
-        }
-    }
+    LUX_D bool at_rest() const { return cur == kNoNode && leaf == kNoNode; }
 
-    LUX_D void fail(int* error, int bit, float rtmax) {
+    LUX_D void fail(int* error, int bit) {
         atomicOr(error, bit);
         hit = SceneHit{};
-        hit.t = rtmax;
-        done = true;
+        hit.t = INFINITY;
+        cur = leaf = kNoNode;
+        top.clear();
+        t_top.clear();
+    }
+    LUX_D void stop() {  // an occlusion walk ends at its first accepted triangle
+        cur = leaf = kNoNode;
+        top.clear();
+        t_top.clear();
     }
 
-    // Resumes the deepest deferred TLAS child that still passes; false when none is left.
-    LUX_D bool pop_tlas(const WalkStacks& k) {
-        while (t_sp > 0) {
-            --t_sp;
-            const int2 e = k.t[t_sp];
-            if (!(__int_as_float(e.y) > hit.t)) {
-                t_cur = e.x;
-                return true;
+    // Goes through the TLAS, from its root (fresh) or from the last deferred child, until a
+    // BLAS is entered (true) or nothing is left (false).
+    LUX_D bool tlas(const SceneView& sc, WalkStacks& k, const WalkRay& r, bool fresh,
+                    int* error) {
+        const BvhView& tl = sc.tlas;
+        const slab_ray sr = make_slab_ray(ray3{r.o, r.tmin, r.d, r.tmax});
+        int at = kNoNode;
+        if (fresh) {
+            hit = SceneHit{};
+            hit.t = r.tmax;
+            stop();
+            if (!sc.has_two_level) return false;
+            if (tl.n <= kFlatTlas) {
+                // Every leaf box is tested here, in leaf order (the binary walk's left-first
+                // order), and the passing leaves after the first are deferred with their
+                // entry t as the walk defers children, so the walk enters the same instances
+                // under the same bounds without stepping through the TLAS's internal nodes
+                // (a leaf box passes under a bound exactly when every box above it does).
+                float at_t = 0.0f;
+                for (int j = tl.n - 1; j >= 0; --j) {
+                    float te;
+                    if (slab_hit(sr, leaf_box(tl, j), hit.t, te)) {
+                        if (at != kNoNode) t_top.push(k.t, at, at_t);
+                        at = ~j;
+                        at_t = te;
+                    }
+                }
+            } else {
+                float tn;
+                if (!slab_hit(sr, load_root(tl.root), hit.t, tn)) return false;
+                at = 0;
             }
+        } else {
+            at = t_top.pop(k.t, hit.t);
+        }
+        const unsigned bound = 2u * static_cast<unsigned>(tl.n) + 64u;
+        for (unsigned step = 0; at != kNoNode; ++step) {
+            if (step > bound || at >= tl.n - 1 || ~at >= tl.n) {
+                fail(error, kErrLoopBound);
+                return false;
+            }
+            if (at >= 0) {
+                const BvhNode nd = load_node(tl.nodes, at);
+                float ta, tb;
+                const bool hl = slab_hit(sr, node_left_box(nd), hit.t, ta);
+                const bool hr = slab_hit(sr, node_right_box(nd), hit.t, tb);
+                if (hl && hr) {
+                    if (t_top.full(kStack)) {
+                        fail(error, kErrStackOverflow);
+                        return false;
+                    }
+                    t_top.push(k.t, nd.ch.y, tb);
+                }
+                at = hl ? nd.ch.x : hr ? nd.ch.y : kNoNode;
+            } else {
+                if (enter(sc, ~at, r, sr)) return true;
+                at = kNoNode;
+            }
+            if (at == kNoNode) at = t_top.pop(k.t, hit.t);
         }
         return false;
     }
-    LUX_D bool pop_blas(const WalkStacks& k) {
-        b_cur = b_top.pop(k.b, hit.t);
-        return b_cur != kNoNode;
-    }
 
-    // One step; returns true when the walk is complete (hit holds the result).
-    LUX_D bool step(const SceneView& sc, WalkStacks& k, int* error) {
-        if (done) return true;
-        const BvhView& tl = sc.tlas;
-        if (in_blas) {
-            if (++b_steps > 2u * static_cast<unsigned>(b_n) + 64u || b_cur >= b_n - 1 ||
-                ~b_cur >= b_n) {
-                fail(error, kErrLoopBound, INFINITY);
-                return true;
-            }
-            bool pop = true;
-            if (b_cur >= 0) {
-                const WideNode w = load_wide(b_wide, b_cur);
-                float tt[4];
-                bool pp[4];
-                wide_test(w, lsr, lneg, hit.t, tt, pp);
-                if (b_top.full(kWideBlasStack)) {
-                    fail(error, kErrStackOverflow, INFINITY);
-                    return true;
-                }
-                const int next = wide_descend(w, tt, pp, k.b, b_top);
-                if (next != kNoNode) {
-                    b_cur = next;
-                    pop = false;
-                }
-            } else {
-                const float4* tp = reinterpret_cast<const float4*>(b_tris + ~b_cur);
-                const float4 p0 = __ldg(tp);
-                const int local = __float_as_int(p0.w);
-                if (local != b_ignored) {
-                    const float4 p1 = __ldg(tp + 1);
-                    const float4 p2 = __ldg(tp + 2);
-                    float tn, t, u, v;
-                    const octant_ray lorr = make_octant_ray(lsr);
-                    // The leaf's exact box (the triangle's box) under the current best t,
-                    // then the triangle.
-                    if (child_hit(triangle_box(xyz(p0), xyz(p1), xyz(p2)), lsr, lorr, hit.t, tn)
-                        && moller_trumbore(lo, ld, xyz(p0), xyz(p1), xyz(p2), t, u, v)
-                        && t > tmin && t < hit.t) {
-                        hit.prim = b_first + local;
-                        hit.t = t;
-                        hit.u = u;
-                        hit.v = v;
-                        if (any_hit) {
-                            done = true;
-                            return true;
-                        }
-                    }
-                }
-            }
-            if (pop && !pop_blas(k)) {
-                in_blas = false;
-                if (!pop_tlas(k)) done = true;
-            }
-            return done;
-        }
-        if (++t_steps > 2u * static_cast<unsigned>(tl.n) + 64u || t_cur >= tl.n - 1 ||
-            ~t_cur >= tl.n) {
-            fail(error, kErrLoopBound, INFINITY);
-            return true;
-        }
-        bool pop = true;
-        if (t_cur >= 0) {
-            BvhNode nd = load_node(tl.nodes, t_cur);
-            float a, b;
-            bool hl = slab_hit(sr, node_left_box(nd), hit.t, a);
-            bool hr = slab_hit(sr, node_right_box(nd), hit.t, b);
-            if (hl) {
-                if (hr) {
-                    if (t_sp >= kStack) {
-                        fail(error, kErrStackOverflow, INFINITY);
-                        return true;
-                    }
-                    k.t[t_sp] = make_int2(nd.ch.y, __float_as_int(b));
-                    ++t_sp;
-                }
-                t_cur = nd.ch.x;
-                pop = false;
-            } else if (hr) {
-                t_cur = nd.ch.y;
-                pop = false;
-            }
-        } else if (enter(sc)) {
-            return false;
-        }
-        if (pop && !pop_tlas(k)) done = true;
-        return done;
-    }
-
-    // Enters the instance of TLAS leaf ~t_cur: the ray in its object space and the BLAS
-    // root's test; true when the walk goes on in the BLAS.
-    LUX_D bool enter(const SceneView& sc) {
-        const int inst_id = sc.tlas_instance[sc.tlas.sorted_ids[~t_cur]];
+    // Enters the instance of TLAS leaf j: the ray in its object space and the BLAS root's
+    // test; true when the walk goes on in the BLAS.
+    LUX_D bool enter(const SceneView& sc, int j, const WalkRay& r, const slab_ray& sr) {
+        const int inst_id = sc.tlas_instance[sc.tlas.sorted_ids[j]];
         const Instance& inst = sc.instances[inst_id];
         const BvhView& b = sc.blas[inst.blas];
         if (b.n <= 0) return false;
-        lo = xform_point(inst.inv, o);
-        ld = xform_vector(inst.inv, d);
-        lsr = make_slab_ray(ray3{lo, tmin, ld, hit.t});
+        const f3 lo = xform_point(inst.inv, r.o);
+        ld = xform_vector(inst.inv, r.d);
+        if (ld.x == r.d.x && ld.y == r.d.y && ld.z == r.d.z) {
+            lsr = sr;   // a translation: the same direction, so the same reciprocals
+            lsr.o = lo;
+        } else {
+            lsr = make_slab_ray(ray3{lo, r.tmin, ld, hit.t});
+        }
         float tn;
         if (!slab_hit(lsr, load_root(b.root), hit.t, tn)) return false;
-        in_blas = true;
-        lneg = wide_octant(lsr);
-        b_wide = b.wide;
-        b_tris = b.tris;
-        b_n = b.n;
-        b_cur = b.n == 1 ? ~0 : 0;
-        b_top.clear();
-        b_steps = 0;
-        b_ignored = inst_id == ign_instance ? ign_local : -1;
-        b_first = inst.first_primitive;
+        oct = wide_octant(lsr);
+        wide = b.wide;
+        tris = b.tris;
+        n = b.n;
+        steps = 0;
+        first = inst.first_primitive;
+        ignored = -1;
+        if (r.ignored >= 0 &&
+            __float_as_int(__ldg(&sc.tris[r.ignored].v1.w)) == inst_id)
+            ignored = __float_as_int(__ldg(&sc.tris[r.ignored].v2.w));
+        top.clear();
+        cur = b.n == 1 ? kNoNode : 0;
+        leaf = b.n == 1 ? ~0 : kNoNode;
         return true;
+    }
+    // Tests BLAS node cur and moves on to the next node; a leaf on the way goes to the free
+    // place, a second one stops the walk until the first has been tested.
+    LUX_D void node_step(WalkStacks& k, int* error) {
+        if (++steps > 2u * static_cast<unsigned>(n) + 64u || cur >= n - 1) {
+            fail(error, kErrLoopBound);
+            return;
+        }
+        if (top.full(kWideStackPt)) {
+            fail(error, kErrStackOverflow);
+            return;
+        }
+        const WideNode w = load_wide(wide, cur);
+        float t[4];
+        bool p[4];
+        wide_test(w, lsr, oct, hit.t, t, p);
+        cur = wide_descend(w, t, p, k.b, top);
+        wide_move_on(cur, leaf, k.b, top, hit.t);
+    }
+
+    // Tests the waiting leaf: its exact box (the triangle's box) under the current best t,
+    // then the triangle.
+    LUX_D void leaf_step(WalkStacks& k, bool any_hit, int* error) {
+        const int j = ~leaf;
+        leaf = kNoNode;
+        if (j >= n) {
+            fail(error, kErrLoopBound);
+            return;
+        }
+        const float4* tp = reinterpret_cast<const float4*>(tris + j);
+        const float4 p0 = __ldg(tp);
+        const int local = __float_as_int(p0.w);
+        if (local != ignored) {
+            const float4 p1 = __ldg(tp + 1);
+            const float4 p2 = __ldg(tp + 2);
+            float tn, t, u, v;
+            const octant_ray lorr = make_octant_ray(lsr);
+            if (child_hit(triangle_box(xyz(p0), xyz(p1), xyz(p2)), lsr, lorr, hit.t, tn)
+                && moller_trumbore(lsr.o, ld, xyz(p0), xyz(p1), xyz(p2), t, u, v)
+                && t > lsr.tmin && t < hit.t) {
+                hit.prim = first + local;
+                hit.t = t;
+                hit.u = u;
+                hit.v = v;
+                if (any_hit) {
+                    stop();
+                    return;
+                }
+            }
+        }
+        wide_move_on(cur, leaf, k.b, top, hit.t);
     }
 };
 
@@ -917,44 +903,68 @@ struct PathState {
     float prev_pdf;
     int pixel, sample, depth, passthrough, measure;
     unsigned flags;
+    Pcg rng;
 };
 
 LUX_D PathState load_state(const PathPool& rt, int p) {
     PathState s;
-    float4 a = rt.thr_eta[p];
-    float4 b = rt.prev[p];
-    int4 m = rt.meta[p];
+    float4 a, b, c, d;
+    ld8(rt.state + 4 * static_cast<size_t>(p), a, b);
+    ld8(rt.state + 4 * static_cast<size_t>(p) + 2, c, d);
     s.thr = xyz(a);
     s.eta = a.w;
     s.prev_pos = xyz(b);
     s.prev_pdf = b.w;
-    s.pixel = m.x;
-    s.sample = m.y;
-    s.depth = m.z & 0xffff;
-    s.passthrough = (m.z >> 16) & 0xffff;
-    s.measure = m.w & 0xff;
-    s.flags = static_cast<unsigned>(m.w) >> 8;
+    s.rng.state = static_cast<uint64_t>(__float_as_uint(c.x)) |
+                  (static_cast<uint64_t>(__float_as_uint(c.y)) << 32);
+    const int depths = __float_as_int(c.z), mode = __float_as_int(c.w);
+    s.depth = depths & 0xffff;
+    s.passthrough = (depths >> 16) & 0xffff;
+    s.measure = mode & 0xff;
+    s.flags = static_cast<unsigned>(mode) >> 8;
+    s.pixel = __float_as_int(d.x);
+    s.sample = __float_as_int(d.y);
+    s.rng.inc = static_cast<uint64_t>(__float_as_uint(d.z)) |
+                (static_cast<uint64_t>(__float_as_uint(d.w)) << 32);
     return s;
 }
 
+LUX_D float4 state_word2(const PathState& s) {
+    return make_float4(__uint_as_float(static_cast<unsigned>(s.rng.state)),
+                       __uint_as_float(static_cast<unsigned>(s.rng.state >> 32)),
+                       __int_as_float(s.depth | (s.passthrough << 16)),
+                       __int_as_float(s.measure | static_cast<int>(s.flags << 8)));
+}
+LUX_D float4 state_word3(const PathState& s) {
+    return make_float4(__int_as_float(s.pixel), __int_as_float(s.sample),
+                       __uint_as_float(static_cast<unsigned>(s.rng.inc)),
+                       __uint_as_float(static_cast<unsigned>(s.rng.inc >> 32)));
+}
+
+// What changes of a path's state; store_new_state: all of it.
 LUX_D void store_state(const PathPool& rt, int p, const PathState& s) {
-    rt.thr_eta[p] = make_float4(s.thr.x, s.thr.y, s.thr.z, s.eta);
-    rt.prev[p] = make_float4(s.prev_pos.x, s.prev_pos.y, s.prev_pos.z, s.prev_pdf);
-    rt.meta[p] = make_int4(s.pixel, s.sample, s.depth | (s.passthrough << 16),
-                           s.measure | static_cast<int>(s.flags << 8));
+    float4* o = rt.state + 4 * static_cast<size_t>(p);
+    stg8(o, make_float4(s.thr.x, s.thr.y, s.thr.z, s.eta),
+         make_float4(s.prev_pos.x, s.prev_pos.y, s.prev_pos.z, s.prev_pdf));
+    o[2] = state_word2(s);
+}
+LUX_D void store_new_state(const PathPool& rt, int p, const PathState& s) {
+    float4* o = rt.state + 4 * static_cast<size_t>(p);
+    stg8(o, make_float4(s.thr.x, s.thr.y, s.thr.z, s.eta),
+         make_float4(s.prev_pos.x, s.prev_pos.y, s.prev_pos.z, s.prev_pdf));
+    stg8(o + 2, state_word2(s), state_word3(s));
 }
 
-LUX_D Pcg load_rng(const PathPool& rt, int p) {
-    uint4 r = rt.rng[p];
-    Pcg g;
-    g.state = static_cast<uint64_t>(r.x) | (static_cast<uint64_t>(r.y) << 32);
-    g.inc = static_cast<uint64_t>(r.z) | (static_cast<uint64_t>(r.w) << 32);
-    return g;
+LUX_D int path_pixel(const PathPool& rt, int p) {
+    return __float_as_int(rt.state[4 * static_cast<size_t>(p) + 3].x);
 }
 
-LUX_D void store_rng(const PathPool& rt, int p, const Pcg& g) {
-    rt.rng[p] = make_uint4(static_cast<unsigned>(g.state), static_cast<unsigned>(g.state >> 32),
-                           static_cast<unsigned>(g.inc), static_cast<unsigned>(g.inc >> 32));
+LUX_D void load_ray(const PathPool& rt, int p, float4& o, float4& d) {
+    ld8(rt.ray + 2 * static_cast<size_t>(p), o, d);
+}
+LUX_D void store_ray(const PathPool& rt, int p, f3 o, f3 d) {
+    stg8(rt.ray + 2 * static_cast<size_t>(p), make_float4(o.x, o.y, o.z, kRayEpsilon),
+         make_float4(d.x, d.y, d.z, INFINITY));
 }
 
 LUX_D void add_radiance(const PathPool& rt, int p, f3 v) {
@@ -965,27 +975,18 @@ LUX_D void add_radiance(const PathPool& rt, int p, f3 v) {
 // Moves path p's state (everything but the per-bounce hit and shadow records) from pool
 // src to slot q of pool dst.
 LUX_D void copy_path(const PathPool& src, int p, const PathPool& dst, int q) {
-    dst.thr_eta[q] = src.thr_eta[p];
+    float4 a, b;
+    for (int k = 0; k < 4; k += 2) {
+        ld8(src.state + 4 * static_cast<size_t>(p) + k, a, b);
+        stg8(dst.state + 4 * static_cast<size_t>(q) + k, a, b);
+    }
+    load_ray(src, p, a, b);
+    stg8(dst.ray + 2 * static_cast<size_t>(q), a, b);
     dst.rad[q] = src.rad[p];
-    dst.prev[q] = src.prev[p];
-    dst.meta[q] = src.meta[p];
-    dst.rng[q] = src.rng[p];
-    dst.ray_o[q] = src.ray_o[p];
-    dst.ray_d[q] = src.ray_d[p];
 }
 
 LUX_D int material_of(const SceneView& sc, int prim) {
     return __float_as_int(__ldg(&sc.tris[prim].v0.w));
-}
-
-LUX_D int material_class(int type) {
-    switch (type) {
-        case kLambert: return 0;
-        case kThinLambert: return 1;
-        case kGgx: return 2;
-        case kDielectric: return 3;
-        default: return 4;
-    }
 }
 
 // Emission seen at a hit (surface_light_le + area_light_pdf_solid_angle,
@@ -1051,118 +1052,179 @@ LUX_D void init_path(const PathPool& rt, const Camera& cam, int p, int pixel, in
     s.passthrough = 0;
     s.measure = kMeasureNone;
     s.flags = 0;
-    store_state(rt, p, s);
-    store_rng(rt, p, g);
+    s.rng = g;
+    store_new_state(rt, p, s);
     rt.rad[p] = make_float4(0, 0, 0, 0);
-    rt.ray_o[p] = make_float4(o.x, o.y, o.z, kRayEpsilon);
-    rt.ray_d[p] = make_float4(d.x, d.y, d.z, INFINITY);
+    store_ray(rt, p, o, d);
 }
 
-// Records the closest hit h of path p's ray: returns the material class of the hit, or
-// -1 after adding the environment's radiance on a miss (cpu_path_tracer.cpp:415-428).
-LUX_D int extend_finish(const PathPool& rt, const SceneView& sc, int sampler, int p,
-                        const SceneHit& h) {
-    if (h.prim >= 0) {
-        rt.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
-        return material_class(sc.materials[material_of(sc, h.prim)].type);
-    }
-    const f3 dir = xyz(rt.ray_d[p]);
+// Records the closest hit h of path p's ray (primitive -1 on a miss).
+LUX_D void store_hit(const PathPool& rt, int p, const SceneHit& h) {
+    rt.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+}
+
+// The environment's radiance along path p's ray, which hit nothing, with its weight
+// (cpu_path_tracer.cpp:415-428); false when there is none.
+LUX_D bool miss_radiance(const PathPool& rt, const SceneView& sc, int sampler, int p, f3& add_v) {
+    const f3 dir = xyz(rt.ray[2 * static_cast<size_t>(p) + 1]);
     f3 le = infinite_le(sc, dir);
-    if (max_component(le) > 0) {
-        PathState s = load_state(rt, p);
-        if (s.depth == 0 || is_delta(s.flags)) {
-            add_radiance(rt, p, s.thr * le);
-        } else if (s.measure == kMeasureSolidAngle && s.prev_pdf > 0) {
-            float w = power_heuristic(s.prev_pdf, infinite_pdf(sc, sampler, dir));
-            add_radiance(rt, p, (s.thr * le) * w);
-        }
+    if (!(max_component(le) > 0)) return false;
+    PathState s = load_state(rt, p);
+    if (s.depth == 0 || is_delta(s.flags)) {
+        add_v = s.thr * le;
+        return true;
     }
-    return -1;
+    if (s.measure == kMeasureSolidAngle && s.prev_pdf > 0) {
+        float w = power_heuristic(s.prev_pdf, infinite_pdf(sc, sampler, dir));
+        add_v = (s.thr * le) * w;
+        return true;
+    }
+    return false;
 }
 
-// Closest hit of path p's ray (one walk to completion), then extend_finish.
-LUX_D int extend_path(const PathPool& rt, const SceneView& sc, int sampler, int p, int* error) {
-    float4 a = rt.ray_o[p];
-    float4 b = rt.ray_d[p];
-    SceneHit h = scene_closest(sc, xyz(a), xyz(b), a.w, b.w, -1, error);
-    return extend_finish(rt, sc, sampler, p, h);
+// store_hit, and on a miss the environment's radiance.
+LUX_D void extend_finish(const PathPool& rt, const SceneView& sc, int sampler, int p,
+                         const SceneHit& h) {
+    store_hit(rt, p, h);
+    f3 v;
+    if (h.prim < 0 && miss_radiance(rt, sc, sampler, p, v)) add_radiance(rt, p, v);
 }
 
-// Closest hits of the paths in queue q[0, n) (q null: paths 0..n-1) by persistent warps:
-// each lane advances its walk by at most `budget` steps per round, and lanes whose walk
-// finished hand it to finish() and take the next path through one warp-aggregated
-// atomic on *next_item, so lanes do not idle behind the longest walk of a static warp.
-// tag_of(p) picks a path's scene once (view(tag) returns it); finish(p, hit) is called by
-// every lane of the warp after each round in which some lane finished, with p = -1 for
-// lanes that did not, so it may append to queues with warp-collective operations (and
-// must do nothing for p = -1).
-template <typename TagOf, typename View, typename Finish>
-LUX_D void refill_walks(const PathPool& rt, const int* q, int n, int* next_item, int budget,
-                        int* error, TagOf tag_of, View view, Finish finish) {
+// A path whose ray hit nothing, in place of shading.  (Not at the end of the walk: only the
+// shadow rays walked beside it may add to a path's radiance there.)
+LUX_D void finish_missed(const PathPool& rt, const SceneView& sc, int sampler, int p) {
+    f3 v;
+    if (miss_radiance(rt, sc, sampler, p, v)) add_radiance(rt, p, v);
+}
+
+// Material class of path p's hit, kMissed when it has none.
+constexpr int kMissed = kClasses, kNoPath = kClasses + 1;
+LUX_D int hit_class(const PathPool& rt, const SceneView& sc, int p) {
+    const int prim = __float_as_int(rt.hit[p].w);
+    return prim >= 0 ? material_class(sc.materials[material_of(sc, prim)].type) : kMissed;
+}
+
+// The block's paths (p of class cls, kNoPath: none) put in order of class, the order of
+// threads within a class; returns this thread's path, -1 for the threads left over, and its
+// class.  So the warps of a block shade one material each (all but those at the seams) and
+// the block still reads its paths' records where the queue has them side by side.  (Appended
+// to a queue per material as their walks ended, paths came out of all order, and shading
+// took 1.7 times as long.)  Called by every thread of the block.
+LUX_D int sort_by_class(int p, int& cls) {
+    constexpr int kWarps = kThreads / 32, kSorted = kNoPath;
+    __shared__ int counts[kSorted][kWarps];
+    __shared__ int path[kThreads];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = lanemask_lt();
+    int rank = 0;
+#pragma unroll
+    for (int c = 0; c < kSorted; ++c) {
+        const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+        if (cls == c) rank = __popc(m & lt);
+        if (lane == 0) counts[c][warp] = __popc(m);
+    }
+    __syncthreads();
+    int before = 0, total = 0, mine = kNoPath;
+#pragma unroll
+    for (int c = 0; c < kSorted; ++c) {
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            if (c * kWarps + w < cls * kWarps + warp) before += counts[c][w];
+            total += counts[c][w];
+        }
+        if (mine == kNoPath && static_cast<int>(threadIdx.x) < total) mine = c;
+    }
+    if (cls < kSorted) path[before + rank] = p;
+    cls = mine;
+    __syncthreads();
+    const int sorted = static_cast<int>(threadIdx.x) < total ? path[threadIdx.x] : -1;
+    __syncthreads();   // the arrays are free for the next call
+    return sorted;
+}
+
+// Closest hit of path p's ray (one walk to completion).
+LUX_D void extend_path(const PathPool& rt, const SceneView& sc, int p, int* error) {
+    float4 a, b;
+    load_ray(rt, p, a, b);
+    store_hit(rt, p, scene_closest(sc, xyz(a), xyz(b), a.w, b.w, -1, error));
+}
+
+// What path p's shadow ray adds with transmittance tr: throughput * ((contribution * tr) *
+// mis), formed at shading where tr is always 1 (whole: the record has the factors).
+LUX_D f3 shadow_value(const PathPool& rt, int p, f3 tr, bool whole) {
+    const float4* rec = rt.shadow + 4 * static_cast<size_t>(p) + 2;
+    if (!whole) return xyz(rec[0]);
+    float4 c, t;
+    ld8(rec, c, t);
+    return xyz(t) * ((xyz(c) * tr) * c.w);
+}
+
+// Walks of n items by persistent warps; item(k) names the k-th (any number from 0).  Lanes
+// without a walk take the next item through one warp-aggregated atomic on *next_item, so no
+// lane idles behind the longest walk of a static warp; and the warp takes one kind of step
+// at a time, so that most lanes execute it:
+//   * BLAS nodes are tested (at most `budget` rounds) until twice as many lanes wait at a
+//     leaf as are at a node, or kRestShare of the lanes are between BLASes;
+//   * the waiting leaves are tested;
+//   * at kRestShare, finished walks hand over their hits, items are fetched, and the TLAS is
+//     walked for all lanes that are between BLASes.  These take several dependent loads
+//     whatever their number.
+// One step of whatever kind per lane and round, all kinds one after another in every round,
+// kept 9-10 of 32 lanes active.  Measured on whole renders (Cornell 256x256 at 64 spp, the
+// heavy scene 512x512 at 16, 257 instances 401x301 at 7), that against this: 4.99, 16.41,
+// 12.85 against 4.32, 11.64, 9.55 ms.  kRestShare 12/32: 4.85, 12.66, 9.90; 16: 4.66, 12.24,
+// 9.75; 20: 4.51, 11.99, 9.62; 24: 4.43, 12.03, 9.60; 28: 4.42, 12.47, 9.97 ms.
+//
+// tag_of(p) picks an item's scene once (view(tag) returns it); ray(p) is its ray in world
+// space; any_hit(scene, p): end at the first accepted triangle.  finish(p, tag, hit) is called
+// by every lane of the warp after each round in which some lane finished, with p = -1 for
+// lanes that did not, so it may use warp-collective operations (and must do nothing for
+// p = -1); it returns true for a walk that goes on from ray(p), which it has changed.
+#ifndef LUX_WALK_REST
+#define LUX_WALK_REST 24
+#endif
+constexpr int kRestShare = LUX_WALK_REST;   // of 32
+template <typename Item, typename TagOf, typename View, typename Ray, typename AnyHit,
+          typename Finish>
+LUX_D void walk_items(Item item, int n, int* next_item, int budget, int* error, TagOf tag_of,
+                      View view, Ray ray, AnyHit any_hit, Finish finish) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
-    int p = -1;  // >= 0 active path, -1 needs one, -2 none left
+    int p = -1;  // >= 0 active item, -1 needs one, -2 none left
     int tag = 0;
+    bool fresh = false;
+    int alive = 32;             // lanes that are not out of items
     TwoLevelWalk w;
+    w.hit = SceneHit{};
+    w.n = 0;
+    w.stop();
     WalkStacks stacks;
     for (;;) {
-        const bool need = p == -1;
-        const unsigned m = __ballot_sync(0xffffffffu, need);
-        if (m) {
-            const int leader = __ffs(m) - 1;
-            int base = 0;
-            if (static_cast<int>(lane) == leader) base = atomicAdd(next_item, __popc(m));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (need) {
-                const int idx = base + __popc(m & lt);
-                if (idx >= n) {
-                    p = -2;
-                } else {
-                    p = q ? q[idx] : idx;
-                    tag = tag_of(p);
-                    const float4 a = rt.ray_o[p];
-                    const float4 b = rt.ray_d[p];
-                    w.init(view(tag), stacks, xyz(a), xyz(b), a.w, b.w, -1);
-                }
-            }
+        // Nodes
+        int on = 0, waiting = 0, resting = 0;
+        for (int s = 0; s < budget; ++s) {
+            on = __popc(__ballot_sync(0xffffffffu, w.cur >= 0));
+            waiting = __popc(__ballot_sync(0xffffffffu, w.cur < 0 && w.leaf != kNoNode));
+            resting = alive - on - waiting;
+            if (on == 0 || waiting > 2 * on || resting * 32 >= alive * kRestShare) break;
+            if (w.cur >= 0) w.node_step(stacks, error);
         }
-        if (__all_sync(0xffffffffu, p == -2)) break;
-        bool finished = false;
-        if (p >= 0) {
-            const SceneView& sc = view(tag);
-            for (int s = 0; s < budget && !finished; ++s) finished = w.step(sc, stacks, error);
+        if (waiting > 0 && resting * 32 < alive * kRestShare) {
+            if (w.leaf != kNoNode) w.leaf_step(stacks, any_hit(view(tag), p), error);
+            continue;
         }
-        // finish() is warp-collective and does nothing for lanes that did not finish, so
-        // a round in which no lane finished skips it.
-        if (__any_sync(0xffffffffu, finished)) {
+        // Lanes between BLASes: those whose walk is over hand over its hit, lanes without
+        // an item take one, and the TLAS is walked on.
+        const bool done = p >= 0 && !fresh && w.at_rest() && w.t_top.h == kNoNode;
+        if (__any_sync(0xffffffffu, done)) {
             SceneHit h = w.hit;
             if (h.prim < 0) h.t = INFINITY;
-            finish(finished ? p : -1, tag, h);
+            const bool again = finish(done ? p : -1, tag, h);
+            if (done) {
+                fresh = again;
+                if (!again) p = -1;
+            }
         }
-        if (finished) p = -1;
-    }
-}
-
-// Shadow rays of the paths in queue q[0, n) by persistent warps with refilling lanes:
-// each lane walks its ray's segments through pass-through surfaces exactly as
-// shadow_path does (the same segment loop, one resumable walk per segment) and adds the
-// NEE contribution when the ray is not blocked.  In a scene without pass-through
-// materials the first hit already blocks the ray, and a hit exists exactly when a
-// closest hit does, so the walk ends at the first accepted triangle.  deposit(p, value)
-// adds the contribution to wherever path p's radiance lives.
-template <typename TagOf, typename View, typename Deposit>
-LUX_D void refill_shadows(const PathPool& rt, const int* q, int n, int* next_item, int budget,
-                          int* error, TagOf tag_of, View view, Deposit deposit,
-                          unsigned long long& segments) {
-    const unsigned lane = threadIdx.x & 31;
-    const unsigned lt = lanemask_lt();
-    int p = -1;  // >= 0 active path, -1 needs one, -2 none left
-    int tag = 0, seg = 0;
-    f3 o, d, tr;
-    float tmax = 0;
-    TwoLevelWalk w;
-    WalkStacks stacks;
-    for (;;) {
         const bool need = p == -1;
         const unsigned m = __ballot_sync(0xffffffffu, need);
         if (m) {
@@ -1175,68 +1237,73 @@ LUX_D void refill_shadows(const PathPool& rt, const int* q, int n, int* next_ite
                 if (idx >= n) {
                     p = -2;
                 } else {
-                    p = q[idx];
+                    p = item(idx);
                     tag = tag_of(p);
-                    const float4 a = rt.sh_o[p];
-                    const float4 b = rt.sh_d[p];
-                    o = xyz(a);
-                    d = xyz(b);
-                    tmax = a.w;
-                    tr = splat(1.0f);
-                    seg = 0;
-                    ++segments;
-                    const SceneView& sv = view(tag);
-                    w.init(sv, stacks, o, d, kRayEpsilon, tmax, __float_as_int(b.w),
-                           !sv.has_passthrough);
+                    fresh = true;
                 }
             }
+            alive = __popc(__ballot_sync(0xffffffffu, p != -2));
+            if (alive == 0) break;
         }
-        if (__all_sync(0xffffffffu, p == -2)) break;
-        if (p < 0) continue;
-        const SceneView& sc = view(tag);
-        for (int s = 0; s < budget; ++s) {
-            if (!w.step(sc, stacks, error)) continue;
-            bool end = false, blocked = false;
-            const SceneHit& h = w.hit;
-            if (h.prim < 0) {
-                end = true;
-            } else {
-                const Material mat = sc.materials[material_of(sc, h.prim)];
-                if (!is_passthrough(mat)) {
-                    blocked = true;
-                    end = true;
-                } else {
-                    tr = tr * passthrough_transmittance(mat);
-                    const float adv = add(h.t, kRayEpsilon);
-                    if (max_component(tr) <= 0 || adv >= tmax) {
-                        end = true;
-                    } else if (++seg >= kShadowSegments) {
-                        atomicOr(error, kErrLoopBound);
-                        blocked = true;
-                        end = true;
-                    } else {
-                        o = o + d * adv;
-                        tmax = sub(tmax, adv);
-                        ++segments;
-                        w.init(sc, stacks, o, d, kRayEpsilon, tmax, -1);
-                    }
-                }
-            }
-            if (end) {
-                if (!blocked && max_component(tr) > 0) {
-                    const float4 c = rt.sh_c[p], t = rt.sh_t[p];
-                    deposit(p, xyz(t) * ((xyz(c) * tr) * c.w));
-                }
-                p = -1;
-                break;
-            }
+        if (p >= 0 && w.at_rest()) {
+            w.tlas(view(tag), stacks, ray(p), fresh, error);
+            fresh = false;
         }
     }
 }
 
+LUX_D WalkRay path_ray(const PathPool& rt, int p) {
+    float4 a, b;
+    load_ray(rt, p, a, b);
+    return WalkRay{xyz(a), xyz(b), a.w, b.w, -1};
+}
+LUX_D WalkRay shadow_ray(const PathPool& rt, int p) {
+    float4 a, b;
+    ld8(rt.shadow + 4 * static_cast<size_t>(p), a, b);
+    return WalkRay{xyz(a), xyz(b), kRayEpsilon, a.w, __float_as_int(b.w)};
+}
+
+// The segments of path p's shadow ray through pass-through surfaces, exactly as shadow_path
+// takes them, one walk per segment: the state of a lane's ray between its walks.  In a scene
+// without pass-through materials the first hit already blocks the ray, and a hit exists
+// exactly when a closest hit does, so the walk may end at the first accepted triangle.
+struct ShadowSegments {
+    f3 tr = splat(1.0f);
+    int seg = 0;
+    bool blocked = false;
+
+    // Takes the closest hit of a segment; true when the ray goes on (path p's shadow record is
+    // then the next segment's ray).
+    LUX_D bool go_on(const PathPool& rt, const SceneView& sc, int p, const SceneHit& h,
+                     int* error) {
+        if (h.prim < 0) return false;
+        const Material mat = sc.materials[material_of(sc, h.prim)];
+        if (!is_passthrough(mat)) {
+            blocked = true;
+            return false;
+        }
+        tr = tr * passthrough_transmittance(mat);
+        float4* rec = rt.shadow + 4 * static_cast<size_t>(p);
+        float4 a, b;
+        ld8(rec, a, b);
+        const float adv = add(h.t, kRayEpsilon);
+        if (!(max_component(tr) > 0) || adv >= a.w) return false;
+        if (++seg >= kShadowSegments) {
+            atomicOr(error, kErrLoopBound);
+            blocked = true;
+            return false;
+        }
+        const f3 o = xyz(a) + xyz(b) * adv;
+        stg8(rec, make_float4(o.x, o.y, o.z, sub(a.w, adv)),
+             make_float4(b.x, b.y, b.z, __int_as_float(-1)));
+        return true;
+    }
+    LUX_D bool arrives() const { return !blocked && max_component(tr) > 0; }
+};
+
 struct ShadeOut {
-    bool spawn = false;   // ray_o/ray_d[p] hold the next ray
-    bool shadow = false;  // sh_*[p] hold a shadow ray
+    bool spawn = false;   // the pool's ray p is the next ray
+    bool shadow = false;  // the pool's shadow record p is a shadow ray
 };
 
 // ------------------------------------------------------------------ debug images
@@ -1328,15 +1395,16 @@ LUX_D f3 encode_normal_color(f3 n) { return (normalize(n) + splat(1.0f)) * 0.5f;
 // primary_normal_debug_color for the camera ray's closest hit h of path p.
 LUX_D void aov_primary(const PathPool& rt, const SceneView& sc, int p, const SceneHit& h,
                        const DebugTargets& aov) {
-    const int4 meta = rt.meta[p];
-    if (meta.z != 0 || h.prim < 0) return;  // depth and pass-through count both zero
+    const float4 mode = rt.state[4 * static_cast<size_t>(p) + 2];
+    if (__float_as_int(mode.z) != 0 || h.prim < 0) return;  // depth and pass-through count both zero
+    const int pixel = path_pixel(rt, p);
     const SceneTri tri = sc.tris[h.prim];
     const f3 ng = triangle_normal(xyz(tri.v0), xyz(tri.v1), xyz(tri.v2));
-    if (aov.ng) aov_add(aov.ng, meta.x, encode_normal_color(ng));
+    if (aov.ng) aov_add(aov.ng, pixel, encode_normal_color(ng));
     if (aov.ns) {
         f3 ns = shading_normal(sc.shading[h.prim], ng, h.u, h.v);
         if (dot(ng, ns) < 0) ns = -ns;
-        aov_add(aov.ns, meta.x, encode_normal_color(ns));
+        aov_add(aov.ns, pixel, encode_normal_color(ns));
     }
 }
 
@@ -1363,13 +1431,15 @@ LUX_D f3 shadow_aov_color(const SceneView& sc, int source_prim, f3 ng, f3 ns, f3
 
 // Shading of the hit stored for path p (cpu_path_tracer.cpp:430-497).  With kAov, also
 // the shadow debug image's light-sample verdict at depth 0, shadow rays at depth 0 are
-// marked (sh_t.w = 1) for classification, and the vertex goes to the path log at each
+// marked (1 in the record's last word) for classification, and the vertex goes to the path log at each
 // exit evaluate_hit_kernel records one (integrator/wavefront_kernels.cu:397-555).
 template <bool kAov = false>
 LUX_D ShadeOut shade_path(const PathPool& rt, const SceneView& sc, int sampler, int max_depth,
                           int p, const DebugTargets& aov = DebugTargets{}) {
     ShadeOut out;
-    float4 ra = rt.ray_o[p], rb = rt.ray_d[p], hh = rt.hit[p];
+    float4 ra, rb;
+    load_ray(rt, p, ra, rb);
+    const float4 hh = rt.hit[p];
     f3 ro = xyz(ra), rd = xyz(rb);
     int prim = __float_as_int(hh.w);
     float t = hh.x, hu = hh.y, hv = hh.z;
@@ -1416,14 +1486,13 @@ LUX_D ShadeOut shade_path(const PathPool& rt, const SceneView& sc, int sampler, 
             log(s.thr, 0);
             s.passthrough += 1;
             f3 no = pos + rd * kRayEpsilon;
-            rt.ray_o[p] = make_float4(no.x, no.y, no.z, kRayEpsilon);
-            rt.ray_d[p] = make_float4(rd.x, rd.y, rd.z, INFINITY);
+            store_ray(rt, p, no, rd);
+            store_state(rt, p, s);
             out.spawn = true;
         } else {
             log(s.thr, max_component(s.thr) <= 0 ? LUX_PATH_END_ZERO_THROUGHPUT
                                                  : LUX_PATH_END_MAX_DEPTH);
         }
-        store_state(rt, p, s);
         return out;
     }
     if (!is_scattering(m)) {
@@ -1438,7 +1507,7 @@ LUX_D ShadeOut shade_path(const PathPool& rt, const SceneView& sc, int sampler, 
     f3 ns = shading_normal(sh, ng, hu, hv);
     if (dot(ng, ns) < 0) ns = -ns;   // make_surface_interaction
     Interaction it{pos, ng, ns, wo};
-    Pcg g = load_rng(rt, p);
+    Pcg& g = s.rng;
     if (has_direct_lighting_lobe(m)) {  // estimate_direct_light, :122-158
         float su = g.next_float();
         float cu = g.next_float();
@@ -1484,10 +1553,16 @@ LUX_D ShadeOut shade_path(const PathPool& rt, const SceneView& sc, int sampler, 
                 }
                 if (ok) {
                     out.shadow = true;
-                    rt.sh_o[p] = make_float4(so.x, so.y, so.z, smax);
-                    rt.sh_d[p] = make_float4(sd.x, sd.y, sd.z, __int_as_float(prim));
-                    rt.sh_c[p] = make_float4(contrib.x, contrib.y, contrib.z, mis);
-                    rt.sh_t[p] = make_float4(s.thr.x, s.thr.y, s.thr.z, mark ? 1.0f : 0.0f);
+                    float4* shadow = rt.shadow + 4 * static_cast<size_t>(p);
+                    stg8(shadow, make_float4(so.x, so.y, so.z, smax),
+                         make_float4(sd.x, sd.y, sd.z, __int_as_float(prim)));
+                    if (kAov || sc.has_passthrough) {
+                        stg8(shadow + 2, make_float4(contrib.x, contrib.y, contrib.z, mis),
+                             make_float4(s.thr.x, s.thr.y, s.thr.z, mark ? 1.0f : 0.0f));
+                    } else {
+                        const f3 value = s.thr * (contrib * mis);   // as shadow_value, tr = 1
+                        shadow[2] = make_float4(value.x, value.y, value.z, 0.0f);
+                    }
                 }
             }
         }
@@ -1530,13 +1605,11 @@ LUX_D ShadeOut shade_path(const PathPool& rt, const SceneView& sc, int sampler, 
             s.depth += 1;
             f3 off = dot(bs.wi, ng) >= 0 ? ng : -ng;   // spawn_scatter_ray
             f3 no = pos + off * kRayEpsilon;
-            rt.ray_o[p] = make_float4(no.x, no.y, no.z, kRayEpsilon);
-            rt.ray_d[p] = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, INFINITY);
+            store_ray(rt, p, no, bs.wi);
+            store_state(rt, p, s);
             out.spawn = true;
         }
     }
-    store_state(rt, p, s);
-    store_rng(rt, p, g);
     return out;
 }
 
@@ -1546,7 +1619,8 @@ LUX_D ShadeOut shade_path(const PathPool& rt, const SceneView& sc, int sampler, 
 template <bool kAov = false>
 LUX_D void shadow_path(const PathPool& rt, const SceneView& sc, int p, int* error,
                        unsigned long long& segments, const DebugTargets& aov = DebugTargets{}) {
-    float4 a = rt.sh_o[p], b = rt.sh_d[p];
+    float4 a, b;
+    ld8(rt.shadow + 4 * static_cast<size_t>(p), a, b);
     f3 o = xyz(a), d = xyz(b);
     float tmax = a.w;
     float tmin = kRayEpsilon;
@@ -1590,19 +1664,16 @@ LUX_D void shadow_path(const PathPool& rt, const SceneView& sc, int p, int* erro
         tmin = kRayEpsilon;
         ignored = -1;
     }
-    if (!blocked && max_component(tr) > 0) {
-        float4 c = rt.sh_c[p], t = rt.sh_t[p];
-        f3 contrib = (xyz(c) * tr) * c.w;
-        add_radiance(rt, p, xyz(t) * contrib);
-    }
-    if (kAov && aov.shadow && rt.sh_t[p].w == 1.0f) {
-        const int source = __float_as_int(rt.sh_d[p].w);
+    if (!blocked && max_component(tr) > 0)
+        add_radiance(rt, p, shadow_value(rt, p, tr, kAov || sc.has_passthrough));
+    if (kAov && aov.shadow && rt.shadow[4 * static_cast<size_t>(p) + 3].w == 1.0f) {
+        const int source = __float_as_int(b.w);
         const SceneTri tri = sc.tris[source];
         const f3 ng = triangle_normal(xyz(tri.v0), xyz(tri.v1), xyz(tri.v2));
         const float4 hh = rt.hit[p];
         f3 ns = shading_normal(sc.shading[source], ng, hh.y, hh.z);
         if (dot(ng, ns) < 0) ns = -ns;
-        aov_add(aov.shadow, rt.meta[p].x,
+        aov_add(aov.shadow, path_pixel(rt, p),
                 shadow_aov_color(sc, source, ng, ns, d, occluder, occluder_t, crossed));
     }
 }

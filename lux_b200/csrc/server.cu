@@ -9,12 +9,12 @@
 //               iteration's queue counters (single thread)
 //   k_generate  turns tickets into camera paths: ticket t -> (request, pixel, sample)
 //               through the admitted requests' ticket ranges (binary search)
-//   k_extend    closest hits of every queued path (mixed depths, requests and scenes)
-//               by persistent warps with refilling lanes; misses retire
-//   k_shade     per-material shading (the same per-path code as lux_render)
-//   k_shadow    NEE shadow rays (persistent warps with refilling lanes)
-//   k_retire    finished paths add their radiance to their request's film in 64-bit
-//               fixed point (order-independent) and count towards completion
+//   k_walk      closest hits of every queued path (mixed depths, requests and scenes) and
+//               the last iteration's NEE shadow rays, by persistent warps with refilling lanes
+//   k_retire    paths that ended in the last iteration add their radiance to their request's
+//               film in 64-bit fixed point (order-independent) and count towards completion
+//   k_shade     environment radiance on a miss, per-material shading (the same per-path code
+//               as lux_render)
 // Tickets enumerate each request's paths pixel-major (pixel = idx / spp), so the random
 // numbers of a path depend only on (request seed, pixel, sample): a request renders the
 // same whether alone or mixed.  The host worker thread admits requests by memory budget,
@@ -47,6 +47,9 @@ namespace lux {
 namespace pt {
 namespace {
 
+#ifndef LUX_SERVER_BLOCKS
+#define LUX_SERVER_BLOCKS 3
+#endif
 constexpr int kMaxRequests = 1024;
 constexpr float kFixedScale = 4294967296.0f;  // 2^32
 constexpr float kFixedMax = 1e9f;             // per-sample clamp keeps 64-bit sums exact
@@ -75,12 +78,9 @@ struct ServerState {
     long long next_ticket;
     long long ticket_limit;
     int count_ray[2];
-    int count_mat[kClasses];
-    int count_shadow;
-    int count_term;
-    int extend_next;   // refill cursor of k_extend_s
-    int shadow_next;   // refill cursor of k_shadow_s
-    int pad2;
+    int count_shadow[2];   // by the iteration's parity: its shading fills them, the next
+    int count_term[2];     // iteration's walk and retirement take them
+    int walk_next;         // refill cursor of k_walk_s
     unsigned long long rays[2];
 };
 
@@ -119,7 +119,7 @@ LUX_D const SceneView* stage_scenes(const ServerDev& d) {
 
 LUX_HD size_t scene_stage_bytes(int scene_count) { return sizeof(SceneView) * static_cast<size_t>(scene_count); }
 
-__global__ void k_plan(ServerState* st, int capacity) {
+__global__ void k_plan(ServerState* st, int capacity, int cur) {
     const int live = st->live_next;  // the previous iteration's continuing paths
     st->live = live;
     st->live_next = 0;
@@ -130,11 +130,9 @@ __global__ void k_plan(ServerState* st, int capacity) {
     st->gen_live = 0;
     st->gen_ticket = st->next_ticket;
     st->next_ticket += n;
-    for (int k = 0; k < kClasses; ++k) st->count_mat[k] = 0;
-    st->count_shadow = 0;
-    st->count_term = 0;
-    st->extend_next = 0;
-    st->shadow_next = 0;
+    st->count_shadow[cur] = 0;
+    st->count_term[cur] = 0;
+    st->walk_next = 0;
 }
 
 // Ticket t of request q is its path idx = t - ticket_start, sample-major: pixel
@@ -204,60 +202,73 @@ __global__ void __launch_bounds__(kThreads) k_generate(ServerDev d, int cur) {
     }
 }
 
-// The bounce kernels run at three resident blocks per SM (at most 80 registers, small
-// spills) rather than the two their register counts allow: config 4 went from 684 to
-// 812 Mrays/s on one B200.
-__global__ void __launch_bounds__(kThreads, 3) k_extend_s(ServerDev d, int cur, int budget) {
+// This iteration's rays and the last iteration's shadow rays, walked together (as k_walk in
+// wavefront.cu).  A shadow ray's record and request are at its path's slot of the last
+// iteration; what it brings goes to where the path lives now, or, of a path that has ended,
+// to that slot, which k_retire reads next.
+//
+// The bounce kernels run at LUX_SERVER_BLOCKS resident blocks per SM rather than the two
+// their register counts allow.
+__global__ void __launch_bounds__(kThreads, LUX_SERVER_BLOCKS) k_walk_s(ServerDev d, int cur,
+                                                                        int budget) {
     const SceneView* scenes = stage_scenes(d);
     const int n = d.st->live + d.st->gen_live;  // slots [0, n) of this iteration's pool
+    const int last = cur ^ 1;
     const PathPool& pool = d.pool[cur];
-    const int* req_of = d.req_of[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&d.st->rays[0], static_cast<unsigned long long>(n));
-    refill_walks(
-        pool, nullptr, n, &d.st->extend_next, budget, d.error,
-        [&](int p) { return req_of[p]; },
+    unsigned long long segments = 0;
+    ShadowSegments sh;
+    walk_items(
+        [&](int k) { return k < n ? 2 * k : 2 * pool.qshadow[k - n] + 1; },
+        n + d.st->count_shadow[last], &d.st->walk_next, budget, d.error,
+        [&](int i) { return d.req_of[i & 1 ? last : cur][i >> 1]; },
         [&](int rs) -> const SceneView& { return scenes[d.req[rs].scene]; },
-        [&](int p, int rs, const SceneHit& h) {
-            int cls = -1;
-            if (p >= 0) {
-                const ReqSlot& q = d.req[rs];
-                cls = extend_finish(pool, scenes[q.scene], q.light_sampler, p, h);
+        [&](int i) { return i & 1 ? shadow_ray(pool, i >> 1) : path_ray(pool, i >> 1); },
+        [](const SceneView& sc, int i) { return (i & 1) && !sc.has_passthrough; },
+        [&](int i, int rs, const SceneHit& h) {
+            if (i < 0) return false;
+            const int p = i >> 1;
+            if (!(i & 1)) {
+                store_hit(pool, p, h);
+                return false;
             }
-            const bool hit = cls >= 0;
-            const int slot = append(d.st->count_mat, hit ? cls : 0, hit);
-            if (hit) pool.qmat[cls * pool.capacity + slot] = p;
-            const int qt = append(&d.st->count_term, 0, p >= 0 && !hit);
-            if (qt >= 0) d.qterm[qt] = p;
+            const SceneView& sc = scenes[d.req[rs].scene];
+            ++segments;
+            if (sh.go_on(pool, sc, p, h, d.error)) return true;
+            if (sh.arrives()) {
+                const int dest = d.sh_dest[p];
+                add_radiance(d.pool[last ^ (dest & 1)], dest >> 1,
+                             shadow_value(pool, p, sh.tr, sc.has_passthrough));
+            }
+            sh = ShadowSegments{};
+            return false;
         });
+    warp_add(&d.st->rays[1], segments);
 }
 
 // Shading in place; a path that continues moves to the other pool at the next
 // appended slot, so the next iteration reads its paths in slot order.
-__global__ void __launch_bounds__(kThreads, 3) k_shade_s(ServerDev d, int cur) {
+__global__ void __launch_bounds__(kThreads, LUX_SERVER_BLOCKS) k_shade_s(ServerDev d, int cur) {
     const SceneView* scenes = stage_scenes(d);
     const int nxt = cur ^ 1;
     const PathPool& pool = d.pool[cur];
-    int c[kClasses];
-    int total = 0;
-    for (int k = 0; k < kClasses; ++k) {
-        c[k] = d.st->count_mat[k];
-        total += c[k];
-    }
+    const int n = d.st->live + d.st->gen_live;  // slots [0, n) of this iteration's pool
     const int stride = gridDim.x * blockDim.x;
-    const int rounds = (total + stride - 1) / stride;
-    for (int r = 0; r < rounds; ++r) {
-        const int i = r * stride + blockIdx.x * blockDim.x + threadIdx.x;
-        const bool active = i < total;
-        int cls = 0, j = i;
-        while (cls < kClasses - 1 && j >= c[cls]) j -= c[cls++];
-        const int p = active ? pool.qmat[cls * pool.capacity + j] : 0;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        const int i = base + threadIdx.x;
+        int cls = kNoPath;
+        if (i < n) cls = hit_class(pool, scenes[d.req[d.req_of[cur][i]].scene], i);
+        const int p = sort_by_class(i, cls);
+        const bool active = p >= 0;
         const int rs = active ? d.req_of[cur][p] : 0;
         ShadeOut o;
         if (active) {
             const ReqSlot& q = d.req[rs];
-            o = shade_path(pool, scenes[q.scene], q.light_sampler, q.max_depth, p);
+            const SceneView& sc = scenes[q.scene];
+            if (cls == kMissed) finish_missed(pool, sc, q.light_sampler, p);
+            else o = shade_path(pool, sc, q.light_sampler, q.max_depth, p);
         }
-        const int s = append(&d.st->count_shadow, 0, o.shadow);
+        const int s = append(&d.st->count_shadow[cur], 0, o.shadow);
         if (o.shadow) pool.qshadow[s] = p;
         const int q = append(&d.st->live_next, 0, o.spawn);
         if (o.spawn) {
@@ -265,26 +276,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_shade_s(ServerDev d, int cur) {
             d.req_of[nxt][q] = rs;
         }
         if (active) d.sh_dest[p] = o.spawn ? 2 * q + 1 : 2 * p;
-        const int t = append(&d.st->count_term, 0, active && !o.spawn);
+        const int t = append(&d.st->count_term[cur], 0, active && !o.spawn);
         if (t >= 0) d.qterm[t] = p;
     }
-}
-
-__global__ void __launch_bounds__(kThreads, 3) k_shadow_s(ServerDev d, int cur, int budget) {
-    const SceneView* scenes = stage_scenes(d);
-    const PathPool& pool = d.pool[cur];
-    const int* req_of = d.req_of[cur];
-    unsigned long long segments = 0;
-    refill_shadows(
-        pool, pool.qshadow, d.st->count_shadow, &d.st->shadow_next, budget, d.error,
-        [&](int p) { return req_of[p]; },
-        [&](int rs) -> const SceneView& { return scenes[d.req[rs].scene]; },
-        [&](int p, f3 v) {
-            const int dest = d.sh_dest[p];
-            add_radiance(d.pool[cur ^ (dest & 1)], dest >> 1, v);
-        },
-        segments);
-    warp_add(&d.st->rays[1], segments);
 }
 
 LUX_D unsigned long long to_fixed(float v) {
@@ -292,19 +286,20 @@ LUX_D unsigned long long to_fixed(float v) {
     return static_cast<unsigned long long>(__float2ll_rn(v * kFixedScale));
 }
 
-__global__ void __launch_bounds__(kThreads) k_retire(ServerDev d, int cur) {
-    const PathPool& pool = d.pool[cur];
-    const int n = d.st->count_term;
+// The paths that ended in the last iteration, whose shadow rays have been walked since.
+__global__ void __launch_bounds__(kThreads) k_retire(ServerDev d, int last) {
+    const PathPool& pool = d.pool[last];
+    const int n = d.st->count_term[last];
     const int stride = gridDim.x * blockDim.x;
     const int rounds = (n + stride - 1) / stride;
     for (int r = 0; r < rounds; ++r) {
         int i = r * stride + blockIdx.x * blockDim.x + threadIdx.x;
         bool active = i < n;
         int p = active ? d.qterm[i] : 0;
-        int rs = active ? d.req_of[cur][p] : -1;
+        int rs = active ? d.req_of[last][p] : -1;
         if (active) {
             const ReqSlot& q = d.req[rs];
-            int pixel = pool.meta[p].x;
+            int pixel = path_pixel(pool, p);
             if (!q.cancelled && pixel >= 0 && pixel < q.width * q.height) {
                 float4 rad = pool.rad[p];
                 unsigned long long* f = q.film + 3 * static_cast<size_t>(pixel);
@@ -697,23 +692,19 @@ int build_graphs(lux_server* s) {
     cudaFuncSetAttribute(k_generate, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(gen_stage));
     int grid = s->ctx->sm_count * 8;
-    int extend_blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&extend_blocks, k_extend_s, kThreads, stage);
-    const int extend_grid = s->ctx->sm_count * std::max(extend_blocks, 1);
-    int shadow_blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shadow_blocks, k_shadow_s, kThreads, stage);
-    const int shadow_grid = s->ctx->sm_count * std::max(shadow_blocks, 1);
+    int walk_blocks = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&walk_blocks, k_walk_s, kThreads, stage);
+    const int walk_grid = s->ctx->sm_count * std::max(walk_blocks, 1);
     cudaStream_t stream = s->ctx->stream;
     for (int cur = 0; cur < 2; ++cur) {
         cudaGraph_t g;
         cudaError_t err = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
         if (err != cudaSuccess) return lux::cuda_fail(err, "graph capture");
-        k_plan<<<1, 1, 0, stream>>>(s->st, s->pool[0].capacity);
+        k_plan<<<1, 1, 0, stream>>>(s->st, s->pool[0].capacity, cur);
         k_generate<<<grid, kThreads, gen_stage, stream>>>(d, cur);
-        k_extend_s<<<extend_grid, kThreads, stage, stream>>>(d, cur, s->ctx->path_budget);
+        k_walk_s<<<walk_grid, kThreads, stage, stream>>>(d, cur, s->ctx->path_budget);
+        k_retire<<<grid, kThreads, 0, stream>>>(d, cur ^ 1);
         k_shade_s<<<grid, kThreads, stage, stream>>>(d, cur);
-        k_shadow_s<<<shadow_grid, kThreads, stage, stream>>>(d, cur, s->ctx->path_budget);
-        k_retire<<<grid, kThreads, 0, stream>>>(d, cur);
         err = cudaStreamEndCapture(stream, &g);
         if (err != cudaSuccess) return lux::cuda_fail(err, "graph capture end");
         err = cudaGraphInstantiate(&s->graph[cur], g, 0);
@@ -734,8 +725,7 @@ void server_release(lux_server* s) {
     lux::pt::path_pool_free(s->pool[0]);
     const lux::pt::PathPool& p1 = s->pool[1];
     void* dev[] = {s->d_scenes, s->req_of[0], s->req_of[1], s->sh_dest, s->qterm, s->st,
-                   s->d_req, s->d_tmap, s->d_done, p1.thr_eta, p1.rad, p1.prev, p1.meta,
-                   p1.rng, p1.ray_o, p1.ray_d};
+                   s->d_req, s->d_tmap, s->d_done, p1.state, p1.ray, p1.rad};
     for (void* p : dev)
         if (p) cudaFree(p);
     if (s->h_req) cudaFreeHost(s->h_req);
@@ -814,15 +804,11 @@ int lux_server_create(int device, lux_scene* const* scenes, int32_t scene_count,
     if (!st) {
         PathPool& p1 = s->pool[1];
         p1 = s->pool[0];
-        p1.thr_eta = p1.rad = p1.prev = p1.ray_o = p1.ray_d = nullptr;
-        p1.meta = nullptr;
-        p1.rng = nullptr;
+        p1.state = p1.ray = p1.rad = nullptr;
     }
-    for (float4** a : {&s->pool[1].thr_eta, &s->pool[1].rad, &s->pool[1].prev, &s->pool[1].ray_o,
-                       &s->pool[1].ray_d})
-        dmalloc(reinterpret_cast<void**>(a), sizeof(float4) * cap);
-    dmalloc(reinterpret_cast<void**>(&s->pool[1].meta), sizeof(int4) * cap);
-    dmalloc(reinterpret_cast<void**>(&s->pool[1].rng), sizeof(uint4) * cap);
+    dmalloc(reinterpret_cast<void**>(&s->pool[1].state), 4 * sizeof(float4) * cap);
+    dmalloc(reinterpret_cast<void**>(&s->pool[1].ray), 2 * sizeof(float4) * cap);
+    dmalloc(reinterpret_cast<void**>(&s->pool[1].rad), sizeof(float4) * cap);
     dmalloc(reinterpret_cast<void**>(&s->req_of[0]), sizeof(int) * cap);
     dmalloc(reinterpret_cast<void**>(&s->req_of[1]), sizeof(int) * cap);
     dmalloc(reinterpret_cast<void**>(&s->sh_dest), sizeof(int) * cap);

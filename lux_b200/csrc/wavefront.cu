@@ -2,13 +2,12 @@
 //
 // A render is a sequence of batches; a batch holds (pixel range) x (sample range) paths,
 // pixel-major, so a pixel's samples are adjacent.  Per bounce d:
-//   k_extend   closest hit through TLAS -> BLAS for every path in ray queue d; misses
-//              add environment radiance; hits are appended to one of five material
-//              queues (warp-aggregated appends)
-//   k_shade    all material queues in one launch (warps stay on one material): emission
-//              with MIS, pass-through, NEE light sample -> shadow queue, BSDF sample,
-//              Russian roulette -> ray queue d+1
-//   k_shadow   shadow rays through pass-through surfaces; adds the NEE contribution
+//   k_walk     closest hit through TLAS -> BLAS for every path in ray queue d, and the
+//              shadow rays of bounce d - 1 through pass-through surfaces
+//   k_shade    the paths of ray queue d, each block's in order of material: environment
+//              radiance on a miss, emission with MIS, pass-through, NEE light sample ->
+//              shadow queue, BSDF sample, Russian roulette -> ray queue d+1
+// (k_extend, k_shade, k_shadow one path per thread as variant 1)
 // then k_flush adds each pixel's sample radiances to the film in sample order, which is
 // the reference CPU tracer's float accumulation order (cpu_path_tracer.cpp:543-558).
 //
@@ -30,8 +29,8 @@ namespace lux {
 namespace pt {
 namespace {
 
-constexpr int kSlots = 9;  // per-bounce counters: ray, 5 material queues, shadow, extend and
-                           // shadow cursors
+// Per-bounce counters: paths in the ray queue, shadow rays, and the walks' cursor.
+constexpr int kSlots = 4, kShadowCount = 1, kWalkNext = 2;
 
 // Depth slots of the queue counters: every max_depth the API accepts (0..1000), so the
 // counters are allocated once per runtime and a deeper request never reallocates.
@@ -75,69 +74,83 @@ __global__ void __launch_bounds__(kThreads) k_camera(PathPool rt, int* counts, S
 }
 
 __global__ void __launch_bounds__(kThreads) k_extend(PathPool rt, int* counts, SceneView sc,
-                                                     int sampler, int depth, int* error) {
-    int n = counts[depth * kSlots];
-    int* mat_counts = counts + depth * kSlots + 1;
+                                                     int depth, int* error) {
+    const int n = counts[depth * kSlots];
     const int* q = rt.qray[depth & 1];
-    int stride = gridDim.x * blockDim.x;
-    int rounds = (n + stride - 1) / stride;
-    for (int r = 0; r < rounds; ++r) {
-        int i = r * stride + blockIdx.x * blockDim.x + threadIdx.x;
-        bool active = i < n;
-        int p = active ? q[i] : 0;
-        int cls = active ? extend_path(rt, sc, sampler, p, error) : -1;
-        bool hit = cls >= 0;
-        int slot = append(mat_counts, hit ? cls : 0, hit);
-        if (hit) rt.qmat[cls * rt.capacity + slot] = p;
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        extend_path(rt, sc, q[i], error);
 }
 
-// k_extend with refilling lanes (refill_walks); the cursor is the bounce's spare slot.
-// Three resident blocks per SM (at most 80 registers, 64 bytes of spills) rather than the
-// two that 103 registers allow: latency-bound walks gain more from the extra warps (heavy
-// scene 1330 -> 1507 Mrays/s on one B200).
-__global__ void __launch_bounds__(kThreads, 3) k_extend_refill(PathPool rt, int* counts,
-                                                            SceneView sc, int sampler, int depth,
-                                                            int budget, int* error) {
+// The rays of bounce `depth` and the shadow rays of the bounce before it, walked together by
+// persistent warps with refilling lanes (walk_items): the two are independent (a path's ray
+// only records its hit, its shadow ray only adds to its radiance, before the path's next
+// shading does), and a launch of either alone ends with its longest walks on a few SMs: 257
+// instances 401x301 at 7 spp 9.55 -> 7.57 ms, 320x240 at 1 spp 1.55 -> 1.03 ms.  Item 2p is
+// path p's ray, 2p + 1 its shadow ray.
+//
+// Blocks: resident blocks per SM.  Four (64 registers, spills) for batches above
+// kManyPaths, whose walks are bound by how many are in flight (Cornell 4.43 -> 4.32 ms, the
+// heavy scene 12.03 -> 11.64 ms); three (80 registers) below, where the longest walks decide
+// (257 instances, 845,000 paths: 9.60 against 9.73 ms; 77,000 paths: 1.54 against 1.60 ms).
+constexpr long long kManyPaths = 1 << 20;
+
+template <int Blocks>
+__global__ void __launch_bounds__(kThreads, Blocks) k_walk(PathPool rt, int* counts,
+                                                           unsigned long long* rays,
+                                                           SceneView sc, int depth, int budget,
+                                                           int* error) {
     int* c = counts + depth * kSlots;
-    int* mat_counts = c + 1;
-    refill_walks(
-        rt, rt.qray[depth & 1], c[0], c + 7, budget, error, [](int) { return 0; },
+    const int n = c[0];
+    const int shadows = depth > 0 ? c[kShadowCount - kSlots] : 0;
+    const int* q = rt.qray[depth & 1];
+    unsigned long long segments = 0;
+    ShadowSegments sh;
+    walk_items(
+        [&](int k) { return k < n ? 2 * q[k] : 2 * rt.qshadow[k - n] + 1; }, n + shadows,
+        c + kWalkNext, budget, error, [](int) { return 0; },
         [&](int) -> const SceneView& { return sc; },
-        [&](int p, int, const SceneHit& h) {
-            const int cls = p >= 0 ? extend_finish(rt, sc, sampler, p, h) : -1;
-            const bool hit = cls >= 0;
-            const int slot = append(mat_counts, hit ? cls : 0, hit);
-            if (hit) rt.qmat[cls * rt.capacity + slot] = p;
+        [&](int i) { return i & 1 ? shadow_ray(rt, i >> 1) : path_ray(rt, i >> 1); },
+        [](const SceneView& scene, int i) { return (i & 1) && !scene.has_passthrough; },
+        [&](int i, int, const SceneHit& h) {
+            if (i < 0) return false;
+            const int p = i >> 1;
+            if (!(i & 1)) {
+                store_hit(rt, p, h);
+                return false;
+            }
+            ++segments;
+            if (sh.go_on(rt, sc, p, h, error)) return true;
+            if (sh.arrives())
+                add_radiance(rt, p, shadow_value(rt, p, sh.tr, sc.has_passthrough));
+            sh = ShadowSegments{};
+            return false;
         });
+    warp_add(rays + 1, segments);
 }
 
-// Three resident blocks per SM (at most 80 registers) as k_extend_refill.
-#ifndef LUX_SHADE_BLOCKS
-#define LUX_SHADE_BLOCKS 3
-#endif
-__global__ void __launch_bounds__(kThreads, LUX_SHADE_BLOCKS) k_shade(PathPool rt, int* counts, SceneView sc,
-                                                    int sampler, int depth, int max_depth) {
-    const int* mc = counts + depth * kSlots + 1;
+// Blocks as k_walk's.
+template <int Blocks>
+__global__ void __launch_bounds__(kThreads, Blocks) k_shade(PathPool rt, int* counts,
+                                                            SceneView sc, int sampler, int depth,
+                                                            int max_depth) {
+    const int n = counts[depth * kSlots];
     int* next_count = counts + (depth + 1) * kSlots;
-    int* shadow_count = counts + depth * kSlots + 6;
-    int c[kClasses];
-    int total = 0;
-    for (int k = 0; k < kClasses; ++k) {
-        c[k] = mc[k];
-        total += c[k];
-    }
+    int* shadow_count = counts + depth * kSlots + kShadowCount;
+    const int* q = rt.qray[depth & 1];
     int* qnext = rt.qray[(depth + 1) & 1];
-    int stride = gridDim.x * blockDim.x;
-    int rounds = (total + stride - 1) / stride;
-    for (int r = 0; r < rounds; ++r) {
-        int i = r * stride + blockIdx.x * blockDim.x + threadIdx.x;
-        bool active = i < total;
-        int cls = 0, j = i;
-        while (cls < kClasses - 1 && j >= c[cls]) j -= c[cls++];
-        int p = active ? rt.qmat[cls * rt.capacity + j] : 0;
+    const int stride = gridDim.x * blockDim.x;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        const int i = base + threadIdx.x;
+        int p = i < n ? q[i] : -1;
+        int cls = kNoPath;
+        if (p >= 0) {
+            if (!sc.one_class) cls = hit_class(rt, sc, p);
+            else cls = __float_as_int(rt.hit[p].w) >= 0 ? 0 : kMissed;
+        }
+        if (!sc.one_class) p = sort_by_class(p, cls);
         ShadeOut o;
-        if (active) o = shade_path(rt, sc, sampler, max_depth, p);
+        if (cls < kMissed) o = shade_path(rt, sc, sampler, max_depth, p);
+        else if (cls == kMissed) finish_missed(rt, sc, sampler, p);
         int slot = append(shadow_count, 0, o.shadow);
         if (o.shadow) rt.qshadow[slot] = p;
         slot = append(next_count, 0, o.spawn);
@@ -148,24 +161,10 @@ __global__ void __launch_bounds__(kThreads, LUX_SHADE_BLOCKS) k_shade(PathPool r
 __global__ void __launch_bounds__(kThreads) k_shadow(PathPool rt, int* counts,
                                                      unsigned long long* rays, SceneView sc,
                                                      int depth, int* error) {
-    int n = counts[depth * kSlots + 6];
+    int n = counts[depth * kSlots + kShadowCount];
     unsigned long long segments = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         shadow_path(rt, sc, rt.qshadow[i], error, segments);
-    warp_add(rays + 1, segments);
-}
-
-// k_shadow with refilling lanes (refill_shadows); the cursor is the bounce's slot 8.
-__global__ void __launch_bounds__(kThreads, 3) k_shadow_refill(PathPool rt, int* counts,
-                                                            unsigned long long* rays,
-                                                            SceneView sc, int depth, int budget,
-                                                            int* error) {
-    int* c = counts + depth * kSlots;
-    unsigned long long segments = 0;
-    refill_shadows(
-        rt, rt.qshadow, c[6], c + 8, budget, error, [](int) { return 0; },
-        [&](int) -> const SceneView& { return sc; },
-        [&](int p, f3 v) { add_radiance(rt, p, v); }, segments);
     warp_add(rays + 1, segments);
 }
 
@@ -175,55 +174,41 @@ __global__ void __launch_bounds__(kThreads) k_extend_aov(PathPool rt, int* count
                                                          int sampler, int depth, int* error,
                                                          DebugTargets aov) {
     int n = counts[depth * kSlots];
-    int* mat_counts = counts + depth * kSlots + 1;
     const int* q = rt.qray[depth & 1];
-    int stride = gridDim.x * blockDim.x;
-    int rounds = (n + stride - 1) / stride;
-    for (int r = 0; r < rounds; ++r) {
-        int i = r * stride + blockIdx.x * blockDim.x + threadIdx.x;
-        bool active = i < n;
-        int p = active ? q[i] : 0;
-        int cls = -1;
-        if (active) {
-            const float4 a = rt.ray_o[p], b = rt.ray_d[p];
-            SceneHit h;
-            if (aov.walk_counts) {
-                WalkCounts wc;
-                h = scene_closest<true>(sc, xyz(a), xyz(b), a.w, b.w, -1, error, &wc);
-                atomicAdd(aov.walk_counts, wc.boxes);
-                atomicAdd(aov.walk_counts + 1, wc.tris);
-                atomicAdd(aov.walk_counts + 2, wc.instances);
-            } else {
-                h = scene_closest(sc, xyz(a), xyz(b), a.w, b.w, -1, error);
-            }
-            if (depth == 0) aov_primary(rt, sc, p, h, aov);
-            cls = extend_finish(rt, sc, sampler, p, h);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int p = q[i];
+        float4 a, b;
+        load_ray(rt, p, a, b);
+        SceneHit h;
+        if (aov.walk_counts) {
+            WalkCounts wc;
+            h = scene_closest<true>(sc, xyz(a), xyz(b), a.w, b.w, -1, error, &wc);
+            atomicAdd(aov.walk_counts, wc.boxes);
+            atomicAdd(aov.walk_counts + 1, wc.tris);
+            atomicAdd(aov.walk_counts + 2, wc.instances);
+        } else {
+            h = scene_closest(sc, xyz(a), xyz(b), a.w, b.w, -1, error);
         }
-        bool hit = cls >= 0;
-        int slot = append(mat_counts, hit ? cls : 0, hit);
-        if (hit) rt.qmat[cls * rt.capacity + slot] = p;
+        if (depth == 0) aov_primary(rt, sc, p, h, aov);
+        extend_finish(rt, sc, sampler, p, h);
     }
 }
 
 __global__ void __launch_bounds__(kThreads) k_shade_aov(PathPool rt, int* counts, SceneView sc,
                                                         int sampler, int depth, int max_depth,
                                                         DebugTargets aov) {
-    const int* mc = counts + depth * kSlots + 1;
+    const int n = counts[depth * kSlots];
     int* next_count = counts + (depth + 1) * kSlots;
-    int* shadow_count = counts + depth * kSlots + 6;
-    int total = 0;
-    for (int k = 0; k < kClasses; ++k) total += mc[k];
+    int* shadow_count = counts + depth * kSlots + kShadowCount;
+    const int* q = rt.qray[depth & 1];
     int* qnext = rt.qray[(depth + 1) & 1];
-    int stride = gridDim.x * blockDim.x;
-    int rounds = (total + stride - 1) / stride;
-    for (int r = 0; r < rounds; ++r) {
-        int i = r * stride + blockIdx.x * blockDim.x + threadIdx.x;
-        bool active = i < total;
-        int cls = 0, j = i;
-        while (cls < kClasses - 1 && j >= mc[cls]) j -= mc[cls++];
-        int p = active ? rt.qmat[cls * rt.capacity + j] : 0;
+    const int stride = gridDim.x * blockDim.x;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        const int i = base + threadIdx.x;
+        const int p = i < n ? q[i] : 0;
         ShadeOut o;
-        if (active) o = shade_path<true>(rt, sc, sampler, max_depth, p, aov);
+        if (i < n && __float_as_int(rt.hit[p].w) >= 0)
+            o = shade_path<true>(rt, sc, sampler, max_depth, p, aov);
         int slot = append(shadow_count, 0, o.shadow);
         if (o.shadow) rt.qshadow[slot] = p;
         slot = append(next_count, 0, o.spawn);
@@ -234,7 +219,7 @@ __global__ void __launch_bounds__(kThreads) k_shade_aov(PathPool rt, int* counts
 __global__ void __launch_bounds__(kThreads) k_shadow_aov(PathPool rt, int* counts,
                                                          unsigned long long* rays, SceneView sc,
                                                          int depth, int* error, DebugTargets aov) {
-    int n = counts[depth * kSlots + 6];
+    int n = counts[depth * kSlots + kShadowCount];
     unsigned long long segments = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         shadow_path<true>(rt, sc, rt.qshadow[i], error, segments, aov);
@@ -310,8 +295,7 @@ void runtime_release(Runtime* rt) {
 }  // namespace
 
 void path_pool_free(PathPool& p) {
-    void* ptrs[] = {p.thr_eta, p.rad, p.prev, p.meta, p.rng, p.ray_o, p.ray_d, p.hit, p.sh_o,
-                    p.sh_d, p.sh_c, p.sh_t, p.qray[0], p.qray[1], p.qmat, p.qshadow};
+    void* ptrs[] = {p.state, p.ray, p.shadow, p.rad, p.hit, p.qray[0], p.qray[1], p.qshadow};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     p = PathPool{};
@@ -324,14 +308,10 @@ int path_pool_alloc(PathPool& p, int capacity) {
         void** ptr;
         size_t bytes;
     } reqs[] = {
-        {reinterpret_cast<void**>(&p.thr_eta), 16 * c}, {reinterpret_cast<void**>(&p.rad), 16 * c},
-        {reinterpret_cast<void**>(&p.prev), 16 * c}, {reinterpret_cast<void**>(&p.meta), 16 * c},
-        {reinterpret_cast<void**>(&p.rng), 16 * c}, {reinterpret_cast<void**>(&p.ray_o), 16 * c},
-        {reinterpret_cast<void**>(&p.ray_d), 16 * c}, {reinterpret_cast<void**>(&p.hit), 16 * c},
-        {reinterpret_cast<void**>(&p.sh_o), 16 * c}, {reinterpret_cast<void**>(&p.sh_d), 16 * c},
-        {reinterpret_cast<void**>(&p.sh_c), 16 * c}, {reinterpret_cast<void**>(&p.sh_t), 16 * c},
+        {reinterpret_cast<void**>(&p.state), 64 * c}, {reinterpret_cast<void**>(&p.ray), 32 * c},
+        {reinterpret_cast<void**>(&p.shadow), 64 * c}, {reinterpret_cast<void**>(&p.rad), 16 * c},
+        {reinterpret_cast<void**>(&p.hit), 16 * c},
         {reinterpret_cast<void**>(&p.qray[0]), 4 * c}, {reinterpret_cast<void**>(&p.qray[1]), 4 * c},
-        {reinterpret_cast<void**>(&p.qmat), 4 * c * kClasses},
         {reinterpret_cast<void**>(&p.qshadow), 4 * c},
     };
     for (auto& r : reqs) {
@@ -461,14 +441,14 @@ int render(lux_ctx* ctx, const lux_scene* scene, const lux_render_request& req, 
     int grid = ctx->sm_count * 8;
     // Persistent grids of the refilling kernels: blocks per SM up to what fits, or the
     // context's LUX_OPT_REFILL_BLOCKS when it asks for fewer.
-    const int refill_fit = occupancy_blocks(ctx, kOccExtendRefill, k_extend_refill, kThreads);
-    const int shadow_fit = occupancy_blocks(ctx, kOccShadowRefill, k_shadow_refill, kThreads);
-    const int refill_grid =
-        ctx->sm_count * (ctx->refill_blocks > 0 ? std::min(ctx->refill_blocks, refill_fit)
-                                                : refill_fit);
-    const int shadow_grid =
-        ctx->sm_count * (ctx->refill_blocks > 0 ? std::min(ctx->refill_blocks, shadow_fit)
-                                                : shadow_fit);
+    const bool many = capacity > kManyPaths;
+    const int walk_fit = many ? occupancy_blocks(ctx, kOccWalkMany, k_walk<4>, kThreads)
+                              : occupancy_blocks(ctx, kOccWalk, k_walk<3>, kThreads);
+    auto* walk = many ? k_walk<4> : k_walk<3>;
+    auto* shade = many ? k_shade<4> : k_shade<3>;
+    const int walk_grid =
+        ctx->sm_count *
+        (ctx->refill_blocks > 0 ? std::min(ctx->refill_blocks, walk_fit) : walk_fit);
     cudaError_t err = cudaMemsetAsync(rt.rays, 0, 16, s);
     if (!per_sample && err == cudaSuccess)
         err = cudaMemsetAsync(out, 0, sizeof(float) * 3 * size_t(pixels), s);
@@ -522,23 +502,20 @@ int render(lux_ctx* ctx, const lux_scene* scene, const lux_render_request& req, 
                     continue;
                 }
                 if (ctx->trace_variant == kTraceStatic) {
-                    k_extend<<<grid, kThreads, 0, s>>>(pool, counts, sc, req.light_sampler,
-                                                       d, ctx->d_error);
-                } else {
-                    k_extend_refill<<<refill_grid, kThreads, 0, s>>>(
-                        pool, counts, sc, req.light_sampler, d, ctx->path_budget,
-                        ctx->d_error);
-                }
-                k_shade<<<grid, kThreads, 0, s>>>(pool, counts, sc, req.light_sampler, d,
-                                                  req.max_depth);
-                if (ctx->trace_variant == kTraceStatic) {
+                    k_extend<<<grid, kThreads, 0, s>>>(pool, counts, sc, d, ctx->d_error);
+                    shade<<<grid, kThreads, 0, s>>>(pool, counts, sc, req.light_sampler, d,
+                                                    req.max_depth);
                     k_shadow<<<grid, kThreads, 0, s>>>(pool, counts, rt.rays, sc, d,
                                                        ctx->d_error);
-                } else {
-                    k_shadow_refill<<<shadow_grid, kThreads, 0, s>>>(
-                        pool, counts, rt.rays, sc, d, ctx->path_budget, ctx->d_error);
+                    ctx->launches += 3;
+                    continue;
                 }
-                ctx->launches += 3;
+                // The last bounce casts no shadow rays: its shading ends every path.
+                walk<<<walk_grid, kThreads, 0, s>>>(pool, counts, rt.rays, sc, d,
+                                                    ctx->path_budget, ctx->d_error);
+                shade<<<grid, kThreads, 0, s>>>(pool, counts, sc, req.light_sampler, d,
+                                                req.max_depth);
+                ctx->launches += 2;
             }
             k_count_rays<<<1, 1, 0, s>>>(counts, rt.rays, req.max_depth + 1);
             int fgrid = std::max(1, std::min(grid, (b.pixels + kThreads - 1) / kThreads));
