@@ -1104,42 +1104,101 @@ LUX_D int hit_class(const PathPool& rt, const SceneView& sc, int p) {
     return prim >= 0 ? material_class(sc.materials[material_of(sc, prim)].type) : kMissed;
 }
 
-// The block's paths (p of class cls, kNoPath: none) put in order of class, the order of
-// threads within a class; returns this thread's path, -1 for the threads left over, and its
-// class.  So the warps of a block shade one material each (all but those at the seams) and
-// the block still reads its paths' records where the queue has them side by side.  (Appended
-// to a queue per material as their walks ended, paths came out of all order, and shading
-// took 1.7 times as long.)  Called by every thread of the block.
-LUX_D int sort_by_class(int p, int& cls) {
-    constexpr int kWarps = kThreads / 32, kSorted = kNoPath;
-    __shared__ int counts[kSorted][kWarps];
-    __shared__ int path[kThreads];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned lt = lanemask_lt();
-    int rank = 0;
+// A block's paths in order of class, the order of their places within a class, so that its
+// warps shade one material each (all but those at the seams) and the block still reads its
+// paths' records where the queue has them side by side.  (Appended to a queue per material
+// as their walks ended, paths came out of all order, and shading took 1.7 times as long.)
+// The block sorts up to kSortRounds paths a thread at a time and its warps take 32 of them
+// after 32 as they come free: with one path a thread and a warp for each 32, the warps waited
+// for the slowest a third of the time (the heavy scene's 512x512, 16 spp: 10.29 -> 9.82 ms).
+constexpr int kSortRounds = 4;
+constexpr int kBlockWarps = kThreads / 32;
+
+struct ClassSort {
+    int place[kNoPath * kSortRounds * kBlockWarps];   // by class, then by round and warp
+    int path[kSortRounds * kThreads];
+    int total, taken;
+
+    // Sorts path_of(0 .. rounds * kThreads - 1) (-1: none) by class_of(path).  Called by
+    // every thread of the block.
+    template <typename PathOf, typename ClassOf>
+    LUX_D void sort(int rounds, PathOf path_of, ClassOf class_of) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const unsigned lt = lanemask_lt();
+        int p[kSortRounds], cls[kSortRounds], rank[kSortRounds];
 #pragma unroll
-    for (int c = 0; c < kSorted; ++c) {
-        const unsigned m = __ballot_sync(0xffffffffu, cls == c);
-        if (cls == c) rank = __popc(m & lt);
-        if (lane == 0) counts[c][warp] = __popc(m);
-    }
-    __syncthreads();
-    int before = 0, total = 0, mine = kNoPath;
+        for (int r = 0; r < kSortRounds; ++r)
+            p[r] = r < rounds ? path_of(r * kThreads + static_cast<int>(threadIdx.x)) : -1;
 #pragma unroll
-    for (int c = 0; c < kSorted; ++c) {
+        for (int r = 0; r < kSortRounds; ++r) cls[r] = p[r] >= 0 ? class_of(p[r]) : kNoPath;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            if (c * kWarps + w < cls * kWarps + warp) before += counts[c][w];
-            total += counts[c][w];
+        for (int r = 0; r < kSortRounds; ++r) {
+            rank[r] = 0;
+#pragma unroll
+            for (int c = 0; c < kNoPath; ++c) {
+                const unsigned m = __ballot_sync(0xffffffffu, cls[r] == c);
+                if (cls[r] == c) rank[r] = __popc(m & lt);
+                if (lane == 0) place[(c * kSortRounds + r) * kBlockWarps + warp] = __popc(m);
+            }
         }
-        if (mine == kNoPath && static_cast<int>(threadIdx.x) < total) mine = c;
+        if (threadIdx.x == 0) taken = 0;
+        __syncthreads();
+        if (warp == 0) {   // exclusive sums of the counts
+            constexpr int kEach = kNoPath * kSortRounds * kBlockWarps / 32;
+            static_assert(kEach * 32 == kNoPath * kSortRounds * kBlockWarps, "counts per lane");
+            int v[kEach], sum = 0;
+#pragma unroll
+            for (int k = 0; k < kEach; ++k) {
+                v[k] = place[lane * kEach + k];
+                sum += v[k];
+            }
+            int incl = sum;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int o = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off) incl += o;
+            }
+            int run = incl - sum;
+#pragma unroll
+            for (int k = 0; k < kEach; ++k) {
+                place[lane * kEach + k] = run;
+                run += v[k];
+            }
+            if (lane == 31) total = incl;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSortRounds; ++r)
+            if (cls[r] < kNoPath)
+                path[place[(cls[r] * kSortRounds + r) * kBlockWarps + warp] + rank[r]] = p[r];
+        __syncthreads();
     }
-    if (cls < kSorted) path[before + rank] = p;
-    cls = mine;
-    __syncthreads();
-    const int sorted = static_cast<int>(threadIdx.x) < total ? path[threadIdx.x] : -1;
-    __syncthreads();   // the arrays are free for the next call
-    return sorted;
+
+    // The next 32 paths for the calling warp: its lane's path and class (-1 and kNoPath past
+    // the last); false when none are left.
+    LUX_D bool next(int& p, int& cls) {
+        const int lane = threadIdx.x & 31;
+        int g = 0;
+        if (lane == 0) g = atomicAdd(&taken, 1);
+        g = __shfl_sync(0xffffffffu, g, 0);
+        if (32 * g >= total) return false;
+        const int k = 32 * g + lane;
+        p = -1;
+        cls = kNoPath;
+        if (k < total) {
+            p = path[k];
+            cls = 0;
+#pragma unroll
+            for (int c = 1; c < kNoPath; ++c)
+                if (k >= place[c * kSortRounds * kBlockWarps]) cls = c;
+        }
+        return true;
+    }
+};
+
+// Paths a thread for a sort: as many as leave every block something to do.
+LUX_D int sort_rounds(int n) {
+    return max(1, min(kSortRounds, n / static_cast<int>(kThreads * gridDim.x)));
 }
 
 // Closest hit of path p's ray (one walk to completion).

@@ -138,23 +138,32 @@ __global__ void __launch_bounds__(kThreads, Blocks) k_shade(PathPool rt, int* co
     int* shadow_count = counts + depth * kSlots + kShadowCount;
     const int* q = rt.qray[depth & 1];
     int* qnext = rt.qray[(depth + 1) & 1];
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int i = base + threadIdx.x;
-        int p = i < n ? q[i] : -1;
-        int cls = kNoPath;
-        if (p >= 0) {
-            if (!sc.one_class) cls = hit_class(rt, sc, p);
-            else cls = __float_as_int(rt.hit[p].w) >= 0 ? 0 : kMissed;
+    __shared__ ClassSort order;
+    // Paths of one class need no order: the block takes one a thread at a time.
+    const int rounds = sc.one_class ? 1 : sort_rounds(n);
+    const int per = kThreads * rounds;
+    for (int base = blockIdx.x * per; base < n; base += gridDim.x * per) {
+        if (!sc.one_class)
+            order.sort(
+                rounds, [&](int k) { return base + k < n ? q[base + k] : -1; },
+                [&](int p) { return hit_class(rt, sc, p); });
+        for (bool more = true; more; more = !sc.one_class) {
+            int p = -1, cls = kNoPath;
+            if (!sc.one_class) {
+                if (!order.next(p, cls)) break;
+            } else if (const int i = base + static_cast<int>(threadIdx.x); i < n) {
+                p = q[i];
+                cls = __float_as_int(rt.hit[p].w) >= 0 ? 0 : kMissed;
+            }
+            ShadeOut o;
+            if (cls < kMissed) o = shade_path(rt, sc, sampler, max_depth, p);
+            else if (cls == kMissed) finish_missed(rt, sc, sampler, p);
+            int slot = append(shadow_count, 0, o.shadow);
+            if (o.shadow) rt.qshadow[slot] = p;
+            slot = append(next_count, 0, o.spawn);
+            if (o.spawn) qnext[slot] = p;
         }
-        if (!sc.one_class) p = sort_by_class(p, cls);
-        ShadeOut o;
-        if (cls < kMissed) o = shade_path(rt, sc, sampler, max_depth, p);
-        else if (cls == kMissed) finish_missed(rt, sc, sampler, p);
-        int slot = append(shadow_count, 0, o.shadow);
-        if (o.shadow) rt.qshadow[slot] = p;
-        slot = append(next_count, 0, o.spawn);
-        if (o.spawn) qnext[slot] = p;
+        if (!sc.one_class) __syncthreads();   // the order's memory is free again
     }
 }
 
