@@ -7,12 +7,12 @@
 //   3. radix sort      stable LSD sort of (code, input index), 8-bit digits: one
 //                      k_onesweep launch per digit (local ranking, then the tile's digit
 //                      offsets by a decoupled look-back over the earlier tiles)
-//      k_sort_small    1 to 3 in one block, for few primitives
 //   4. k_climb         leaf boxes + triangle records in sorted order, then one bottom-up
 //                      climb per leaf through the binary radix tree of the codes (Karras's
 //                      hierarchy and node numbers), each node written once with both its
 //                      child boxes: within a block's own leaves through shared memory
 //      k_climb_top     the levels above the blocks, through global memory
+//      k_build_small   1 to 3 in one block for few primitives, all of it for fewer
 // A refit (k_refit) climbs the known hierarchy with new geometry.
 //
 // Reference counterparts (src/): bvh/gpu_bvh.cu:135-149 (codes), 582-584 (sort),
@@ -443,151 +443,6 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const Key* keys_in,
     }
 }
 
-// Root box, Morton codes and their stable sort by one block, for up to kSmallSort
-// primitives: the keys and (16-bit) input indices stay in shared memory over all passes.
-// A chain of kernels over so few keys is launch and look-back latency and nothing else: it
-// takes about 40 us whatever their number, this kernel 15 us for 1,000, 29 us for 5,000 and
-// 44 us for 8,192 (hence the line at 6,144).
-constexpr int kSmallSort = 6144;
-constexpr int kSmallThreads = 1024;
-
-template <typename Key>
-constexpr int small_sort_smem() {
-    return 2 * kSmallSort * static_cast<int>(sizeof(Key) + sizeof(unsigned short)) +
-           (kSmallThreads / 32) * kRadix * static_cast<int>(sizeof(unsigned));
-}
-
-template <int Kind, typename Key>
-__global__ void __launch_bounds__(kSmallThreads) k_sort_small(const float* prims, int n,
-                                                              Key* codes, int* sorted_ids) {
-    constexpr int kWarps = kSmallThreads / 32;
-    constexpr int kPasses = sizeof(Key) == 4 ? 4 : 8;
-    extern __shared__ __align__(16) unsigned char sort_smem[];
-    Key* keys[2];
-    unsigned short* ids[2];
-    keys[0] = reinterpret_cast<Key*>(sort_smem);
-    keys[1] = keys[0] + kSmallSort;
-    unsigned (*wcount)[kRadix] = reinterpret_cast<unsigned (*)[kRadix]>(keys[1] + kSmallSort);
-    ids[0] = reinterpret_cast<unsigned short*>(wcount + kWarps);
-    ids[1] = ids[0] + kSmallSort;
-    __shared__ float part[kWarps][6];
-    __shared__ unsigned loff[kRadix], warp_sums[kRadix / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // The scene box (min and max are order-free).
-    float lo[3] = {INFINITY, INFINITY, INFINITY};
-    float hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
-        f3 v0, v1, v2;
-        box3 b;
-        load_prim<Kind>(prims, i, v0, v1, v2, b);
-        lo[0] = fminf(lo[0], b.lo.x); lo[1] = fminf(lo[1], b.lo.y); lo[2] = fminf(lo[2], b.lo.z);
-        hi[0] = fmaxf(hi[0], b.hi.x); hi[1] = fmaxf(hi[1], b.hi.y); hi[2] = fmaxf(hi[2], b.hi.z);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
-        }
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            part[warp][a] = lo[a];
-            part[warp][3 + a] = hi[a];
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        lo[a] = part[lane][a];
-        hi[a] = part[lane][3 + a];
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
-        }
-    }
-    const box3 root{make_f3(lo[0], lo[1], lo[2]), make_f3(hi[0], hi[1], hi[2])};
-    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
-        f3 v0, v1, v2;
-        box3 b;
-        load_prim<Kind>(prims, i, v0, v1, v2, b);
-        keys[0][i] = sizeof(Key) == 4 ? static_cast<Key>(morton30(b, root))
-                                      : static_cast<Key>(morton63(b, root));
-        ids[0][i] = static_cast<unsigned short>(i);
-    }
-    // Each warp ranks a run of `rounds` * 32 consecutive keys, as k_onesweep's warps do.
-    const unsigned lt = lanemask_lt();
-    const int rounds = (n + kSmallThreads - 1) / kSmallThreads;
-    const int base = warp * rounds * 32;
-    int cur = 0;
-    for (int p = 0; p < kPasses; ++p) {
-        const int shift = 8 * p;
-        for (int i = threadIdx.x; i < kWarps * kRadix; i += kSmallThreads) (&wcount[0][0])[i] = 0;
-        __syncthreads();
-        unsigned rank[kSmallSort / kSmallThreads];
-#pragma unroll
-        for (int j = 0; j < kSmallSort / kSmallThreads; ++j) {
-            if (j >= rounds) break;
-            const int idx = base + j * 32 + lane;
-            const bool valid = idx < n;
-            const unsigned d = valid ? digit_of(keys[cur][idx], shift) : 0u;
-            const unsigned peers = digit_peers(d, valid);
-            const unsigned before = valid ? wcount[warp][d] : 0u;
-            __syncwarp();
-            if (valid && lane == __ffs(peers) - 1) wcount[warp][d] = before + __popc(peers);
-            __syncwarp();
-            rank[j] = before + __popc(peers & lt);
-        }
-        __syncthreads();
-        unsigned total = 0, incl = 0;
-        if (threadIdx.x < kRadix) {
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const unsigned c = wcount[w][threadIdx.x];
-                wcount[w][threadIdx.x] = total;
-                total += c;
-            }
-            incl = total;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
-                if (lane >= off) incl += o;
-            }
-            if (lane == 31) warp_sums[warp] = incl;
-        }
-        __syncthreads();
-        if (threadIdx.x < kRadix) {
-            unsigned before = 0;
-            for (int w = 0; w < warp; ++w) before += warp_sums[w];
-            loff[threadIdx.x] = before + incl - total;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < kSmallSort / kSmallThreads; ++j) {
-            if (j >= rounds) break;
-            const int idx = base + j * 32 + lane;
-            if (idx >= n) break;
-            const Key key = keys[cur][idx];
-            const unsigned d = digit_of(key, shift);
-            const unsigned at = loff[d] + wcount[warp][d] + rank[j];   // < n
-            keys[cur ^ 1][at] = key;
-            ids[cur ^ 1][at] = ids[cur][idx];
-        }
-        cur ^= 1;
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
-        codes[i] = keys[cur][i];
-        sorted_ids[i] = ids[cur][i];
-    }
-}
-
 // Per-tile digit counts, stored digit-major: hist[d * tiles + tile].
 template <typename Key>
 __global__ void __launch_bounds__(kThreads) k_sort_upsweep(const Key* keys, int n, int shift,
@@ -789,6 +644,248 @@ LUX_D Subtree join(const Subtree& left, const Subtree& right, BvhNode* nodes, in
 LUX_D void store_root(float* root, const box3& b) {
     root[0] = b.lo.x; root[1] = b.lo.y; root[2] = b.lo.z;
     root[3] = b.hi.x; root[4] = b.hi.y; root[5] = b.hi.z;
+}
+
+// Few primitives, by one block: scene box, Morton codes and their stable sort with the keys
+// and (16-bit) input indices in shared memory over all passes; and, up to kWholeBuild, the
+// hierarchy too (Whole).  A chain of kernels over so few keys is launch, look-back and atomic
+// latency and nothing else: the chain took 33 us for 257 triangles, 38 us for 1,000 and 49 us
+// for 2,000, the whole build by one block takes 16, 28 and 46 us.  It climbs with one SM's
+// issue slots, 18 us per 1,024 leaves, so beyond that k_climb's many blocks are faster (4,000
+// triangles: 61 against 84 us), and one SM's sort is faster than the chain of sort kernels up
+// to kSmallSort (4,000: 61 against 67 us, with 63-bit codes 76 against 99; 6,144: 74 against
+// 74, 96 against 104).
+constexpr int kWholeBuild = 2048;
+constexpr int kSmallSort = 6144;
+constexpr int kSmallThreads = 1024;
+
+template <typename Key, bool Whole>
+constexpr int small_build_smem() {
+    constexpr int kMax = Whole ? kWholeBuild : kSmallSort;
+    const int sort = 2 * kMax * static_cast<int>(sizeof(Key) + sizeof(unsigned short)) +
+                     (kSmallThreads / 32) * kRadix * static_cast<int>(sizeof(unsigned));
+    const int climb = kWholeBuild * static_cast<int>(6 * sizeof(float) + sizeof(unsigned) +
+                                                     sizeof(unsigned short));
+    return sort > climb || !Whole ? sort : climb;
+}
+
+template <int Kind, typename Key, bool Whole>
+__global__ void __launch_bounds__(kSmallThreads) k_build_small(
+        const float* prims, int n, Key* codes, int* sorted_ids, TriRecord* tris, BvhNode* nodes,
+        int* leaf_parent, int* node_parent, float* root_box) {
+    constexpr int kWarps = kSmallThreads / 32;
+    constexpr int kPasses = sizeof(Key) == 4 ? 4 : 8;
+    constexpr int kMax = Whole ? kWholeBuild : kSmallSort;
+    constexpr int kEach = kMax / kSmallThreads;
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    Key* keys[2];
+    unsigned short* ids[2];
+    keys[0] = reinterpret_cast<Key*>(small_smem);
+    keys[1] = keys[0] + kMax;
+    unsigned (*wcount)[kRadix] = reinterpret_cast<unsigned (*)[kRadix]>(keys[1] + kMax);
+    ids[0] = reinterpret_cast<unsigned short*>(wcount + kWarps);
+    ids[1] = ids[0] + kMax;
+    __shared__ float part[kWarps][6];
+    __shared__ unsigned loff[kRadix], warp_sums[kRadix / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // The scene box (min and max are order-free).
+    float lo[3] = {INFINITY, INFINITY, INFINITY};
+    float hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        f3 v0, v1, v2;
+        box3 b;
+        load_prim<Kind>(prims, i, v0, v1, v2, b);
+        lo[0] = fminf(lo[0], b.lo.x); lo[1] = fminf(lo[1], b.lo.y); lo[2] = fminf(lo[2], b.lo.z);
+        hi[0] = fmaxf(hi[0], b.hi.x); hi[1] = fmaxf(hi[1], b.hi.y); hi[2] = fmaxf(hi[2], b.hi.z);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+        }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            part[warp][a] = lo[a];
+            part[warp][3 + a] = hi[a];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = part[lane][a];
+        hi[a] = part[lane][3 + a];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+        }
+    }
+    const box3 root{make_f3(lo[0], lo[1], lo[2]), make_f3(hi[0], hi[1], hi[2])};
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        f3 v0, v1, v2;
+        box3 b;
+        load_prim<Kind>(prims, i, v0, v1, v2, b);
+        keys[0][i] = sizeof(Key) == 4 ? static_cast<Key>(morton30(b, root))
+                                      : static_cast<Key>(morton63(b, root));
+        ids[0][i] = static_cast<unsigned short>(i);
+    }
+    // Each warp ranks a run of `rounds` * 32 consecutive keys, as k_onesweep's warps do.
+    const unsigned lt = lanemask_lt();
+    const int rounds = (n + kSmallThreads - 1) / kSmallThreads;
+    const int base = warp * rounds * 32;
+    int cur = 0;
+    for (int p = 0; p < kPasses; ++p) {
+        const int shift = 8 * p;
+        for (int i = threadIdx.x; i < kWarps * kRadix; i += kSmallThreads) (&wcount[0][0])[i] = 0;
+        __syncthreads();
+        unsigned rank[kEach];
+#pragma unroll
+        for (int j = 0; j < kEach; ++j) {
+            if (j >= rounds) break;
+            const int idx = base + j * 32 + lane;
+            const bool valid = idx < n;
+            const unsigned d = valid ? digit_of(keys[cur][idx], shift) : 0u;
+            const unsigned peers = digit_peers(d, valid);
+            const unsigned before = valid ? wcount[warp][d] : 0u;
+            __syncwarp();
+            if (valid && lane == __ffs(peers) - 1) wcount[warp][d] = before + __popc(peers);
+            __syncwarp();
+            rank[j] = before + __popc(peers & lt);
+        }
+        __syncthreads();
+        unsigned total = 0, incl = 0;
+        if (threadIdx.x < kRadix) {
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+                const unsigned c = wcount[w][threadIdx.x];
+                wcount[w][threadIdx.x] = total;
+                total += c;
+            }
+            incl = total;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off) incl += o;
+            }
+            if (lane == 31) warp_sums[warp] = incl;
+        }
+        __syncthreads();
+        if (threadIdx.x < kRadix) {
+            unsigned before = 0;
+            for (int w = 0; w < warp; ++w) before += warp_sums[w];
+            loff[threadIdx.x] = before + incl - total;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kEach; ++j) {
+            if (j >= rounds) break;
+            const int idx = base + j * 32 + lane;
+            if (idx >= n) break;
+            const Key key = keys[cur][idx];
+            const unsigned d = digit_of(key, shift);
+            const unsigned at = loff[d] + wcount[warp][d] + rank[j];   // < n
+            keys[cur ^ 1][at] = key;
+            ids[cur ^ 1][at] = ids[cur][idx];
+        }
+        cur ^= 1;
+        __syncthreads();
+    }
+    if (!Whole) {
+        for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+            codes[i] = keys[cur][i];
+            sorted_ids[i] = ids[cur][i];
+        }
+        return;
+    }
+    // The hierarchy, as k_climb's blocks build it, of all leaves.  What it needs of the sort
+    // is kept in registers (its ids) and in place (the prefix lengths), the rest of the shared
+    // memory is taken anew.
+    __shared__ signed char sdelta[Whole ? kMax + 1 : 1];   // prefix length of leaves j - 1 and j
+    int pid[kEach];
+#pragma unroll
+    for (int r = 0; r < kEach; ++r) {
+        const int k = r * kSmallThreads + static_cast<int>(threadIdx.x);
+        pid[r] = -1;
+        if (k < n) {
+            pid[r] = ids[cur][k];
+            codes[k] = keys[cur][k];
+            sorted_ids[k] = pid[r];
+            sdelta[k] = static_cast<signed char>(k > 0 ? delta(keys[cur], k - 1, k) : -1);
+        }
+    }
+    if (threadIdx.x == 0) sdelta[n] = -1;
+    __syncthreads();
+    float* sbox = reinterpret_cast<float*>(small_smem);                   // [6][kMax]
+    unsigned* sflag = reinterpret_cast<unsigned*>(sbox + 6 * kMax);   // per split
+    unsigned short* send = reinterpret_cast<unsigned short*>(sflag + kMax);
+    auto put_box = [&](int j, const box3& b) {
+        sbox[j] = b.lo.x; sbox[kMax + j] = b.lo.y; sbox[2 * kMax + j] = b.lo.z;
+        sbox[3 * kMax + j] = b.hi.x; sbox[4 * kMax + j] = b.hi.y;
+        sbox[5 * kMax + j] = b.hi.z;
+    };
+    auto get_box = [&](int j) {
+        return box3{make_f3(sbox[j], sbox[kMax + j], sbox[2 * kMax + j]),
+                    make_f3(sbox[3 * kMax + j], sbox[4 * kMax + j],
+                            sbox[5 * kMax + j])};
+    };
+#pragma unroll
+    for (int r = 0; r < kEach; ++r) {
+        const int k = r * kSmallThreads + static_cast<int>(threadIdx.x);
+        if (pid[r] < 0) continue;
+        f3 v0, v1, v2;
+        box3 b;
+        load_prim<Kind>(prims, pid[r], v0, v1, v2, b);
+        if (Kind == LUX_PRIM_TRIANGLES) {
+            TriRecord t;
+            t.p0 = make_float4(v0.x, v0.y, v0.z, __int_as_float(pid[r]));
+            t.p1 = make_float4(v1.x, v1.y, v1.z, 0.0f);
+            t.p2 = make_float4(v2.x, v2.y, v2.z, 0.0f);
+            tris[k] = t;
+        }
+        put_box(k, b);
+        send[k] = static_cast<unsigned short>(k);
+        sflag[k] = 0;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = threadIdx.x; k < n; k += kSmallThreads) {
+        Subtree t;
+        t.b = get_box(k);
+        t.first = t.last = k;
+        t.dl = sdelta[k];
+        t.dr = sdelta[k + 1];
+        for (;;) {   // at most n - 1 joins in all
+            if (t.is_root()) {
+                store_root(root_box, t.b);
+                break;
+            }
+            const bool left = t.is_left();
+            const int s = left ? t.last : t.first - 1;
+            const int own = left ? s : s + 1, sib = left ? s + 1 : s;
+            if (t.first != t.last) {
+                put_box(own, t.b);
+                send[own] = static_cast<unsigned short>(left ? t.first : t.last);
+            }
+            __threadfence_block();
+            if (atomicAdd(&sflag[s], 1u) == 0) break;   // the sibling joins them
+            __threadfence_block();
+            Subtree o;
+            o.b = get_box(sib);
+            o.first = left ? sib : send[sib];
+            o.last = left ? send[sib] : sib;
+            o.dl = left ? t.dr : sdelta[o.first];
+            o.dr = left ? sdelta[o.last + 1] : t.dl;
+            t = left ? join(t, o, nodes, leaf_parent, node_parent)
+                     : join(o, t, nodes, leaf_parent, node_parent);
+        }
+    }
 }
 
 // Hierarchy and boxes in one bottom-up pass over the sorted codes, in two kernels.  The tree
@@ -1326,12 +1423,16 @@ int build_typed(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
         err = cudaMemsetAsync(bvh->leaf_parent, 0xff, sizeof(int), ctx->stream);
     if (err != cudaSuccess) return cuda_fail(err, "memset leaf parent");
     if (n <= kSmallSort) {
-        err = allow_smem(k_sort_small<Kind, Key>, small_sort_smem<Key>());
+        const bool whole = n <= kWholeBuild;
+        const auto kernel = whole ? k_build_small<Kind, Key, true> : k_build_small<Kind, Key, false>;
+        const int smem = whole ? small_build_smem<Key, true>() : small_build_smem<Key, false>();
+        err = allow_smem(kernel, smem);
         if (err == cudaSuccess)
-            err = chain_launch(ctx, k_sort_small<Kind, Key>, 1, kSmallThreads,
-                               small_sort_smem<Key>(), prims, n, codes, bvh->sorted_ids);
-        if (err != cudaSuccess) return cuda_fail(err, "k_sort_small");
-        return climb<Kind, Key>(ctx, bvh, prims);
+            err = chain_launch(ctx, kernel, 1, kSmallThreads, smem, prims, n, codes,
+                               bvh->sorted_ids, bvh->tris, bvh->nodes, bvh->leaf_parent,
+                               bvh->node_parent, bvh->root);
+        if (err != cudaSuccess) return cuda_fail(err, "k_build_small");
+        return whole ? LUX_OK : climb<Kind, Key>(ctx, bvh, prims);
     }
     unsigned* root_ord = nullptr;
     if (int st = reset_sort_scratch<Key>(ctx, n, &root_ord)) return st;

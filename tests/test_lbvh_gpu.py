@@ -461,9 +461,11 @@ def test_wide_walk_exact_on_leaf_chains_at_any_scale(ctx, oracle, scale, speed):
     assert np.array_equal(got_id, want_id) and np.array_equal(got_t, want_t)
 
 
-# The climb's 256-leaf blocks, one leaf more and one less, and a tree of a chain whose
-# subtrees leave their block one leaf at a time; then a refit of each.
-@pytest.mark.parametrize("n", [3, 255, 256, 257, 511, 769, 6144, 6145])
+# The edges of the one-block build (1,024 threads, up to 2,048 leaves), of the climb's 256-leaf
+# blocks and of the one-block sort, and a tree of a chain whose subtrees leave their block one
+# leaf at a time; then a refit of each.
+@pytest.mark.parametrize("n", [3, 255, 256, 257, 511, 769, 1024, 1025, 2047, 2048, 2049, 2304,
+                               2305, 6144, 6145])
 @pytest.mark.parametrize("kind", [lux_b200.PRIM_TRIANGLES, lux_b200.PRIM_AABBS])
 @pytest.mark.parametrize("chain", [False, True])
 def test_climb_blocks_match_oracle(ctx, oracle, n, kind, chain):
@@ -476,6 +478,7 @@ def test_climb_blocks_match_oracle(ctx, oracle, n, kind, chain):
     bvh = ctx.build_lbvh(prims, kind=kind)
     got = bvh.download()
     _assert_tree_equal(got, oracle.build(boxes))
+    _assert_tree_equal(ctx.build_lbvh(prims, kind, 63).download(), oracle.build(boxes, 63))
     for _ in range(2):                            # the arrival counters are left at zero
         bvh.refit(moved_prims)
         after = bvh.download()
