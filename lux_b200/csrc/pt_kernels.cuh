@@ -1222,8 +1222,8 @@ LUX_D f3 shadow_value(const PathPool& rt, int p, f3 tr, bool whole) {
 // without a walk take the next item through one warp-aggregated atomic on *next_item, so no
 // lane idles behind the longest walk of a static warp; and the warp takes one kind of step
 // at a time, so that most lanes execute it:
-//   * BLAS nodes are tested (at most `budget` rounds) until twice as many lanes wait at a
-//     leaf as are at a node, or kRestShare of the lanes are between BLASes;
+//   * BLAS nodes are tested (at most `budget` rounds) until more lanes wait at a leaf than
+//     are at a node, or kRestShare of the lanes are between BLASes;
 //   * the waiting leaves are tested;
 //   * at kRestShare, finished walks hand over their hits, items are fetched, and the TLAS is
 //     walked for all lanes that are between BLASes.  These take several dependent loads
@@ -1232,7 +1232,9 @@ LUX_D f3 shadow_value(const PathPool& rt, int p, f3 tr, bool whole) {
 // kept 9-10 of 32 lanes active.  Measured on whole renders (Cornell 256x256 at 64 spp, the
 // heavy scene 512x512 at 16, 257 instances 401x301 at 7), that against this: 4.99, 16.41,
 // 12.85 against 4.32, 11.64, 9.55 ms.  kRestShare 12/32: 4.85, 12.66, 9.90; 16: 4.66, 12.24,
-// 9.75; 20: 4.51, 11.99, 9.62; 24: 4.43, 12.03, 9.60; 28: 4.42, 12.47, 9.97 ms.
+// 9.75; 20: 4.51, 11.99, 9.62; 24: 4.43, 12.03, 9.60; 28: 4.42, 12.47, 9.97 ms.  Leaves once
+// waiting lanes are more than 3, 2, 1, 1/2 times those at nodes (in a later build): 4.15,
+// 9.96, 7.66; 4.15, 9.79, 7.64; 4.16, 9.64, 7.40; 4.22, 9.65, 7.34 ms.
 //
 // tag_of(p) picks an item's scene once (view(tag) returns it); ray(p) is its ray in world
 // space; any_hit(scene, p): end at the first accepted triangle.  finish(p, tag, hit) is called
@@ -1265,7 +1267,7 @@ LUX_D void walk_items(Item item, int n, int* next_item, int budget, int* error, 
             on = __popc(__ballot_sync(0xffffffffu, w.cur >= 0));
             waiting = __popc(__ballot_sync(0xffffffffu, w.cur < 0 && w.leaf != kNoNode));
             resting = alive - on - waiting;
-            if (on == 0 || waiting > 2 * on || resting * 32 >= alive * kRestShare) break;
+            if (on == 0 || waiting > on || resting * 32 >= alive * kRestShare) break;
             if (w.cur >= 0) w.node_step(stacks, error);
         }
         if (waiting > 0 && resting * 32 < alive * kRestShare) {
