@@ -197,6 +197,23 @@ def test_small_tlas_walks_render_as_the_binary_walk(ctx, extra):
     assert np.array_equal(got, want)
 
 
+# One path, fewer paths than a warp has lanes, one per warp and fewer, and some per warp of a
+# persistent grid: the walks spread over all warps.
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (5, 3, 1), (61, 53, 1), (97, 89, 2)])
+def test_spread_walks_render_as_one_thread_per_path(ctx, w, h, spp):
+    sc = S.Scene(ctx, S.make_cornell_scene(w, h))
+    req = S.request(w, h, spp, 5, 17)
+    old = ctx.get_option(lux_b200.OPT_TRACE_VARIANT)
+    try:
+        ctx.set_option(lux_b200.OPT_TRACE_VARIANT, 1)
+        want = S.render(ctx, sc, req)
+        ctx.set_option(lux_b200.OPT_TRACE_VARIANT, 0)
+        got = S.render(ctx, sc, req)
+    finally:
+        ctx.set_option(lux_b200.OPT_TRACE_VARIANT, old)
+    assert np.array_equal(got, want)
+
+
 def test_sample_offset_and_frame_index_continue_the_sequence(ctx):
     """RenderSettings::sample_offset (integrator/render_context.h:52): two halves of the
     samples rendered separately equal the full render's samples."""
