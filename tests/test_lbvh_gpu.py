@@ -431,6 +431,18 @@ def test_few_rays_match_oracle(ctx, oracle, count):
     assert np.array_equal(bvh.trace_any(rays) >= 0, want_id >= 0)
 
 
+# Nodes are fetched ahead up to 14 rays a warp of 16 on each of the 148 SMs.
+@pytest.mark.parametrize("count", [33152, 33153])
+def test_walks_that_fetch_ahead_match_oracle(ctx, oracle, count):
+    tris = W.soup_triangles(16384, seed=43, median_len=0.02)
+    rays = W.uniform_rays(count, seed=44)
+    want_id, want_t = oracle.trace(tris, oracle.build(oracle.triangle_bounds(tris)), rays)
+    bvh = ctx.build_lbvh(tris)
+    got_id, got_t = bvh.trace_closest(rays)
+    assert np.array_equal(got_id, want_id) and np.array_equal(got_t, want_t)
+    assert np.array_equal(bvh.trace_any(rays) >= 0, want_id >= 0)
+
+
 # Triangles at distances that halve towards a corner: a hierarchy of leaf-and-node pairs,
 # whose wide nodes open the node side twice, over many scales in one scene; at scales where
 # a node's grid fits, just fits and does not fit, and for directions whose reciprocals are
