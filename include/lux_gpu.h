@@ -73,10 +73,11 @@ int lux_ctx_launch_count(lux_ctx* ctx, int64_t* count);
  *   LUX_OPT_TRACE_VARIANT  0 auto (4), 1 one thread per ray, 2 persistent warps with
  *                          refill, 3 one thread per ray over 4-wide nodes, 4 persistent
  *                          warps with refill over 4-wide nodes
- *   LUX_OPT_TRACE_BUDGET   traversal steps per refill round of the persistent kernel
+ *   LUX_OPT_TRACE_BUDGET   node steps of the persistent kernel before waiting leaves are
+ *                          tested and idle lanes take new rays, at most
  *   LUX_OPT_RENDER_BATCH   paths in flight per wavefront batch (device memory ~200 B each)
- *   LUX_OPT_PATH_BUDGET    traversal steps per refill round of the path tracer's extension and
- *                          shadow kernels (variant 1 uses one thread per path instead)
+ *   LUX_OPT_PATH_BUDGET    the same of the path tracer's walks (variant 1 uses one thread
+ *                          per path instead)
  *   LUX_OPT_REFILL_BLOCKS  resident 256-thread blocks per SM of those refilling kernels'
  *                          persistent grids (0: as many as fit, else 1..3)
  * Read only (lux_ctx_get_option), the device memory the context holds for reuse:

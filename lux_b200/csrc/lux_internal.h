@@ -20,8 +20,8 @@ struct lux_ctx {
     unsigned long long* h_words = nullptr;
     // Tunables (lux_ctx_set_option).
     int trace_variant = 0;           // lux::kTrace* (auto: wide persistent)
-    int trace_budget = 16;           // traversal steps per refill round (ray queries)
-    int path_budget = 32;            // traversal steps per refill round (path tracer)
+    int trace_budget = 16;           // node steps per round (ray queries)
+    int path_budget = 32;            // node steps per round (path tracer)
     int render_batch = 1 << 22;      // paths in flight per wavefront batch
     int refill_blocks = 0;           // blocks per SM of the refilling kernels (0: max)
     void* render_runtime = nullptr;  // wavefront buffers, grown on demand
