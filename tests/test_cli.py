@@ -55,6 +55,7 @@ def _read_pfm(path):
 
 
 @pytest.mark.gpu
+@pytest.mark.skipif(not Ref.available(), reason="reference harness not built")
 def test_cli_cornell_matches_reference_cpu_tracer(cli, tmp_path):
     """`lux-render -gpu` on the Cornell box (seed 0, as the reference CLI) against the
     reference's own CPU tracer at the same settings: per-pixel means within noise."""
@@ -93,6 +94,7 @@ def test_cli_renders_every_code_defined_scene(cli, tmp_path, scene, sampler):
 
 
 @pytest.mark.gpu
+@pytest.mark.skipif(not Ref.available(), reason="reference harness not built")
 def test_film_encoders_match_the_reference_writers(ctx, tmp_path):
     """lux_film_encode's PPM bytes, linear-debug bytes and PFM floats against the
     reference's write_ppm / write_debug_ppm_linear / write_pfm on the same film."""
