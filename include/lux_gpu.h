@@ -597,7 +597,8 @@ int lux_server_wait_all(lux_server* server, int64_t timeout_us);
 /* Queued requests are dropped; running ones stop contributing and finish early. */
 int lux_server_cancel(lux_server* server, int64_t request_id);
 /* New vertex positions for one mesh of one resident scene: applied between pool
- * iterations as a refit (lux_scene_update_mesh), so later paths see the new frame. */
+ * iterations as a refit (lux_scene_update_mesh), so later rays see the new frame; a light
+ * sample is tested against the frame that its vertex was shaded on. */
 int lux_server_update_mesh(lux_server* server, int32_t scene, int32_t mesh,
                            const float* vertices);
 /* Host timestamps (steady clock, ns) of submission, admission and completion. */

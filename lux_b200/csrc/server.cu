@@ -20,7 +20,8 @@
 // same whether alone or mixed.  The host worker thread admits requests by memory budget,
 // uploads request slots and ticket ranges between launches (stream order), keeps two
 // iterations in flight, and delivers films when a request's retired-path count reaches
-// its path count.
+// its path count.  Before it applies mesh updates it has the queued shadow rays walked, so
+// that no light sample is tested against another frame than its vertex's.
 // No reference counterpart: the reference renders one request per call with a host
 // loop over batches and bounces (integrator/wavefront_scheduler.cu:73-131).
 
@@ -205,14 +206,16 @@ __global__ void __launch_bounds__(kThreads) k_generate(ServerDev d, int cur) {
 // This iteration's rays and the last iteration's shadow rays, walked together (as k_walk in
 // wavefront.cu).  A shadow ray's record and request are at its path's slot of the last
 // iteration; what it brings goes to where the path lives now, or, of a path that has ended,
-// to that slot, which k_retire reads next.
+// to that slot, which k_retire reads next.  rays false: the shadow rays alone
+// (drain_shadows).
 //
 // The bounce kernels run at LUX_SERVER_BLOCKS resident blocks per SM: eight requests over
 // four scenes in a pool of 2^21 paths take 33.8 ms at four (64 registers), 34.8 at three.
 __global__ void __launch_bounds__(kThreads, LUX_SERVER_BLOCKS) k_walk_s(ServerDev d, int cur,
-                                                                        int budget) {
+                                                                        bool rays, int budget) {
     const SceneView* scenes = stage_scenes(d);
-    const int n = d.st->live + d.st->gen_live;  // slots [0, n) of this iteration's pool
+    // Slots [0, n) of this iteration's pool.
+    const int n = rays ? d.st->live + d.st->gen_live : 0;
     const int last = cur ^ 1;
     const PathPool& pool = d.pool[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&d.st->rays[0], static_cast<unsigned long long>(n));
@@ -368,6 +371,8 @@ struct lux_server_request {
 
 struct lux_server {
     lux_ctx* ctx = nullptr;
+    lux::pt::ServerDev dev{};       // what the kernels are given
+    int walk_grid = 0;
     std::vector<lux_scene*> scenes;
     lux::pt::SceneView* d_scenes = nullptr;
     lux::pt::PathPool pool[2];      // pool[1] owns only its path-state arrays
@@ -571,6 +576,23 @@ void fail_all(lux_server* s, int status) {
     s->finished.notify_all();
 }
 
+// Walks the shadow rays that the last launched iteration queued, which the next one would
+// walk: a mesh is about to move, and a light sample is tested against the geometry that it
+// was drawn on.
+cudaError_t drain_shadows(lux_server* s) {
+    using namespace lux::pt;
+    if (s->launched == 0) return cudaSuccess;
+    const int cur = static_cast<int>(s->launched & 1);   // the next iteration's parity
+    cudaStream_t stream = s->ctx->stream;
+    cudaError_t err = cudaMemsetAsync(&s->st->walk_next, 0, sizeof(int), stream);
+    if (err != cudaSuccess) return err;
+    k_walk_s<<<s->walk_grid, kThreads, scene_stage_bytes(s->dev.scene_count), stream>>>(
+        s->dev, cur, false, s->ctx->path_budget);
+    err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
+    return cudaMemsetAsync(&s->st->count_shadow[cur ^ 1], 0, sizeof(int), stream);
+}
+
 void worker_main(lux_server* s) {
     cudaSetDevice(s->ctx->device);
     std::unique_lock<std::mutex> lk(s->mu);
@@ -591,6 +613,11 @@ void worker_main(lux_server* s) {
             batch.swap(s->updates);
             lk.unlock();
             int64_t applied = 0;
+            if (drain_shadows(s) != cudaSuccess) {
+                lk.lock();
+                fail_all(s, LUX_ERR_CUDA);
+                continue;
+            }
             for (size_t k = 0; k < batch.size(); ++k) {
                 bool superseded = false;
                 for (size_t j = k + 1; j < batch.size() && !superseded; ++j)
@@ -680,7 +707,7 @@ void worker_main(lux_server* s) {
 
 int build_graphs(lux_server* s) {
     using namespace lux::pt;
-    ServerDev d;
+    ServerDev& d = s->dev;
     for (int k = 0; k < 2; ++k) {
         d.pool[k] = s->pool[k];
         d.req_of[k] = s->req_of[k];
@@ -701,7 +728,7 @@ int build_graphs(lux_server* s) {
     int grid = s->ctx->sm_count * 8;
     int walk_blocks = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&walk_blocks, k_walk_s, kThreads, stage);
-    const int walk_grid = s->ctx->sm_count * std::max(walk_blocks, 1);
+    s->walk_grid = s->ctx->sm_count * std::max(walk_blocks, 1);
     cudaStream_t stream = s->ctx->stream;
     for (int cur = 0; cur < 2; ++cur) {
         cudaGraph_t g;
@@ -709,7 +736,7 @@ int build_graphs(lux_server* s) {
         if (err != cudaSuccess) return lux::cuda_fail(err, "graph capture");
         k_plan<<<1, 1, 0, stream>>>(s->st, s->pool[0].capacity, cur);
         k_generate<<<grid, kThreads, gen_stage, stream>>>(d, cur);
-        k_walk_s<<<walk_grid, kThreads, stage, stream>>>(d, cur, s->ctx->path_budget);
+        k_walk_s<<<s->walk_grid, kThreads, stage, stream>>>(d, cur, true, s->ctx->path_budget);
         k_retire<<<grid, kThreads, 0, stream>>>(d, cur ^ 1);
         k_shade_s<<<grid, kThreads, stage, stream>>>(d, cur);
         err = cudaStreamEndCapture(stream, &g);

@@ -155,6 +155,36 @@ def test_refits_faster_than_iterations_do_not_starve_requests(ctx):
         assert 1 <= refits <= pushed
 
 
+def test_refits_under_a_request_keep_each_light_sample_on_its_frame(ctx):
+    """A floor with a second one below it jumps between two heights under a distant light while
+    a request runs: in either frame alone nothing is in shadow, and every sample has the same
+    value.  A shadow ray from the low floor that is tested against the raised one meets its
+    underside."""
+    b = S.SceneBuilder()
+    grey = b.add_material(S.lambert((0.5, 0.5, 0.5)))
+    quad = np.array([[-9, 0, -9], [-9, 0, 9], [9, 0, 9], [9, 0, -9]], np.float32)
+    low = np.concatenate([quad, quad - np.float32([0, 1, 0])])
+    high = low + np.float32([0, 2, 0])
+    mesh = b.add_mesh(S.Mesh(low, np.array([[0, 1, 2], [0, 2, 3], [4, 5, 6], [4, 6, 7]], np.uint32),
+                             np.full(4, grey, np.int32)))
+    b.add_instance(mesh)
+    b.add_distant_light((0.0, 1.0, 0.0), (1.0, 1.0, 1.0))
+    b.set_pinhole_camera((0.0, 6.0, 0.1), (0.0, 0.0, 0.0), 40.0, 1.0)
+    req = S.request(64, 64, 512, 1, 3)
+    want = S.render(ctx, S.Scene(ctx, b), req)
+    assert want.min() > 0 and np.ptp(want) <= 1e-4 * want.max()
+    with SV.Server([S.Scene(ctx, b)], pool_paths=1 << 13) as srv:
+        rid, film = srv.submit(0, req)
+        k = 0
+        while srv.poll(rid) in (SV.QUEUED, SV.RUNNING):
+            srv.update_mesh(0, mesh, high if k % 2 == 0 else low)
+            k += 1
+            time.sleep(2e-4)
+        assert srv.poll(rid) == SV.DONE
+        assert srv.stats()["refits"] >= 8
+    assert _close(film, want)
+
+
 def test_mixed_batch_over_the_four_resident_scenes_matches_single_renders(ctx):
     """A mix over the four resident scenes of the batched and served workloads (Cornell,
     the displaced icosphere with glass, the 2,097,152-triangle soup and the 256-instance
