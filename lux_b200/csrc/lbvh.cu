@@ -1451,7 +1451,6 @@ size_t lbvh_scratch_bytes(int n, int morton_bits) {
 }
 
 int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
-    (void)ctx;
     bvh->capacity = std::max(bvh->capacity, std::max(bvh->n, 1));
     const size_t n = static_cast<size_t>(bvh->capacity);
     const size_t inner = std::max<size_t>(n - 1, 1);
@@ -1495,8 +1494,11 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
     // after it.
     static_assert(sizeof(int4) >= sizeof(int2), "open subtrees in the node records' place");
     bvh->open = reinterpret_cast<int2*>(bvh->node_info);
-    cudaError_t err = cudaMemset(bvh->flags, 0, sizeof(unsigned) * inner);
-    if (err == cudaSuccess) err = cudaMemset(bvh->leaf_parent, 0xff, sizeof(int) * n);
+    // On the context's stream: one on the default stream has no order with the build that
+    // follows on a non-blocking stream.
+    cudaError_t err = cudaMemsetAsync(bvh->flags, 0, sizeof(unsigned) * inner, ctx->stream);
+    if (err == cudaSuccess)
+        err = cudaMemsetAsync(bvh->leaf_parent, 0xff, sizeof(int) * n, ctx->stream);
     return cuda_fail(err, "lbvh init");
 }
 

@@ -1,0 +1,71 @@
+"""The library's host code against a CUDA runtime without a GPU (fake_cudart.c, preloaded):
+what it allocates, clears and launches, on which stream, and what it does when memory runs
+out.  No kernel runs."""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+PRELUDE = """
+import ctypes, json, re, sys
+import numpy as np
+import lux_b200 as L
+
+fake = ctypes.CDLL(None)
+fake.fake_log.restype = ctypes.c_char_p
+fake.fake_used.restype = ctypes.c_size_t
+fake.fake_set_limit.argtypes = [ctypes.c_size_t]
+
+
+def log(clear=True):
+    text = fake.fake_log().decode()
+    if clear:
+        fake.fake_clear_log()
+    return text.splitlines()
+
+
+def launched(lines):
+    # Kernel names of the launches: the k_... part of the mangled name.
+    return [re.search(r"(k_[a-z_]*[a-z])", s).group(1) for s in lines if s.startswith("launch")]
+
+
+def triangles(n, seed=0):
+    return np.random.default_rng(seed).random((n, 9), np.float32)
+
+
+ctx = L.Context(0)
+"""
+
+
+@pytest.fixture(scope="session")
+def run(tmp_path_factory):
+    """run(code): code's result (its variable `out`) in a process with the fake runtime."""
+    lib = tmp_path_factory.mktemp("fake") / "fake_cudart.so"
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-o", str(lib),
+                    os.path.join(HERE, "fake_cudart.c"), "-lpthread"], check=True)
+
+    def call(code):
+        env = dict(os.environ, LD_PRELOAD=str(lib), PYTHONPATH=ROOT)
+        res = subprocess.run([sys.executable, "-c", PRELUDE + code + "\nprint(json.dumps(out))"],
+                             env=env, capture_output=True, text=True, timeout=120)
+        assert res.returncode == 0, res.stderr
+        return json.loads(res.stdout.splitlines()[-1])
+
+    return call
+
+
+def test_a_new_bvh_is_cleared_in_stream_order(run):
+    """What a build relies on finding cleared is cleared on the context's stream: a memset on
+    the default stream has no order with a build on a non-blocking one."""
+    lines = run("""
+log()
+bvh = ctx.build_lbvh(triangles(5000))
+out = log()
+""")
+    memsets = [s for s in lines if s.startswith("memset")]
+    assert len(memsets) >= 2 and not any("default" in s for s in memsets), memsets
