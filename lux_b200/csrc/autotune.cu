@@ -53,12 +53,8 @@ int time_candidate(lux_ctx* ctx, int repeats, Run run, float* best_ms) {
 
 int check_error_word(lux_ctx* ctx) {
     int word = 0;
-    cudaError_t err = cudaMemcpy(&word, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) return lux::cuda_fail(err, "error word read");
-    if (word) {
-        cudaMemset(ctx->d_error, 0, sizeof(int));
-        return lux::fail(LUX_ERR_DEVICE_CHECK, "device check failed during tuning");
-    }
+    if (int st = lux::wait_error_word(ctx, &word)) return st;
+    if (word) return lux::fail(LUX_ERR_DEVICE_CHECK, "device check failed during tuning");
     return LUX_OK;
 }
 

@@ -281,7 +281,10 @@ int wait_error_word(lux_ctx* ctx, int* word) {
     if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
     if (err != cudaSuccess) return cuda_fail(err, "stream synchronize");
     *word = static_cast<int>(ctx->h_words[0] & 0xffffffffu);
-    if (*word) cudaMemset(ctx->d_error, 0, sizeof(int));
+    // On the stream too, ahead of the next call's kernels.
+    if (*word)
+        return cuda_fail(cudaMemsetAsync(ctx->d_error, 0, sizeof(int), ctx->stream),
+                         "error word reset");
     return LUX_OK;
 }
 
@@ -318,9 +321,11 @@ int lux_ctx_create(lux_ctx** out, int device, void* stream) {
         ctx->stream = ctx->own_stream;
     }
     err = cudaMalloc(&ctx->d_error, sizeof(int));
-    if (err == cudaSuccess) err = cudaMemset(ctx->d_error, 0, sizeof(int));
+    if (err == cudaSuccess) err = cudaMemsetAsync(ctx->d_error, 0, sizeof(int), ctx->stream);
     if (err == cudaSuccess) err = cudaMalloc(&ctx->d_counter, 64);
-    if (err == cudaSuccess) err = cudaMemset(ctx->d_counter, 0, 64);
+    if (err == cudaSuccess) err = cudaMemsetAsync(ctx->d_counter, 0, 64, ctx->stream);
+    // Before the caller may choose another stream.
+    if (err == cudaSuccess && ctx->own_stream) err = cudaStreamSynchronize(ctx->own_stream);
     if (err == cudaSuccess)
         err = cudaMallocHost(reinterpret_cast<void**>(&ctx->h_words), 64);
     if (err == cudaSuccess) std::memset(ctx->h_words, 0, 64);

@@ -694,7 +694,7 @@ void worker_main(lux_server* s) {
             s->rays[0] = s->h_state[parity]->rays[0];
             s->rays[1] = s->h_state[parity]->rays[1];
             if (err_word) {
-                cudaMemset(s->ctx->d_error, 0, sizeof(int));
+                cudaMemsetAsync(s->ctx->d_error, 0, sizeof(int), s->ctx->stream);
                 fail_all(s, LUX_ERR_DEVICE_CHECK);
                 continue;
             }

@@ -69,3 +69,24 @@ out = log()
 """)
     memsets = [s for s in lines if s.startswith("memset")]
     assert len(memsets) >= 2 and not any("default" in s for s in memsets), memsets
+
+
+def test_the_error_word_is_cleared_in_stream_order(run):
+    """The context's words and a reported error word are cleared on the context's stream: a
+    clear on the default stream can land after the next call's kernels and lose their errors."""
+    out = run("""
+start = log()
+word = ctypes.c_int.from_address(int(re.match(r"malloc 4 (0x[0-9a-f]+)", next(
+    s for s in start if s.startswith("malloc 4 "))).group(1), 16))
+word.value = 4
+try:
+    ctx.synchronize()
+    status = 0
+except L.LuxError as e:
+    status = e.status
+ctx.synchronize()
+out = [start + log(), status, word.value]
+""")
+    memsets = [s for s in out[0] if s.startswith("memset")]
+    assert out[1] == 5 and out[2] == 0
+    assert len(memsets) == 3 and not any("default" in s for s in memsets), memsets
