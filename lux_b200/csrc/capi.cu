@@ -472,7 +472,6 @@ int lux_lbvh_rebuild(lux_ctx* ctx, lux_bvh* bvh, const float* prims, int32_t n) 
     if (n > bvh->capacity) {
         cudaStreamSynchronize(ctx->stream);
         lux::lbvh_free(bvh);
-        bvh->capacity = 0;
         bvh->n = n;
         if (int st = lux::lbvh_alloc(ctx, bvh)) {
             bvh->n = 0;

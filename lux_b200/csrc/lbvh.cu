@@ -1451,8 +1451,8 @@ size_t lbvh_scratch_bytes(int n, int morton_bits) {
 }
 
 int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
-    bvh->capacity = std::max(bvh->capacity, std::max(bvh->n, 1));
-    const size_t n = static_cast<size_t>(bvh->capacity);
+    const int capacity = std::max(bvh->capacity, std::max(bvh->n, 1));
+    const size_t n = static_cast<size_t>(capacity);
     const size_t inner = std::max<size_t>(n - 1, 1);
     const size_t key = bvh->morton_bits == 63 ? 8 : 4;
     // One allocation for every array (each cudaMalloc of a build is time on the host).
@@ -1468,7 +1468,7 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
         {reinterpret_cast<void**>(&bvh->node_info), sizeof(int4) * inner},
         {reinterpret_cast<void**>(&bvh->flags), sizeof(unsigned) * inner},
         {reinterpret_cast<void**>(&bvh->open_count),
-         sizeof(int) * static_cast<size_t>(grid_for(bvh->capacity, kClimbThreads))},
+         sizeof(int) * static_cast<size_t>(grid_for(capacity, kClimbThreads))},
         {&bvh->codes, key * n},
         {reinterpret_cast<void**>(&bvh->root), sizeof(float) * 16},
         // Triangles are built to be traced: their 4-wide nodes have their place from the start.
@@ -1484,6 +1484,7 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
         return fail(LUX_ERR_OUT_OF_MEMORY, "lbvh allocation failed");
     }
     bvh->arena = base;
+    bvh->capacity = capacity;   // only now: a BVH without arrays has room for nothing
     for (const auto& r : reqs) {
         *r.ptr = base;
         base += (r.bytes + 255) & ~size_t(255);
@@ -1499,6 +1500,7 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
     cudaError_t err = cudaMemsetAsync(bvh->flags, 0, sizeof(unsigned) * inner, ctx->stream);
     if (err == cudaSuccess)
         err = cudaMemsetAsync(bvh->leaf_parent, 0xff, sizeof(int) * n, ctx->stream);
+    if (err != cudaSuccess) lbvh_free(bvh);
     return cuda_fail(err, "lbvh init");
 }
 
@@ -1506,6 +1508,7 @@ void lbvh_free(lux_bvh* bvh) {
     if (bvh->wide && bvh->kind != LUX_PRIM_TRIANGLES) cudaFree(bvh->wide);
     if (bvh->arena) cudaFree(bvh->arena);
     bvh->arena = nullptr;
+    bvh->capacity = 0;
     bvh->wide = nullptr;
     bvh->wide_capacity = 0;
     bvh->wide_current = false;

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_persistent(
         unsigned* ray_counter, int budget, int* error) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt_u();
-    const box3 root = load_root(bvh.root);
+    const box3 root = bvh.n > 0 ? load_root(bvh.root) : box3{};
     const unsigned bound = 2u * static_cast<unsigned>(bvh.n) + 64u;  // n <= 2^30
 
     int ray_idx = -1;   // >= 0 active ray, -1 needs a ray, -2 no rays left

@@ -90,3 +90,26 @@ out = [start + log(), status, word.value]
     memsets = [s for s in out[0] if s.startswith("memset")]
     assert out[1] == 5 and out[2] == 0
     assert len(memsets) == 3 and not any("default" in s for s in memsets), memsets
+
+
+def test_a_rebuild_that_found_no_memory_leaves_an_empty_bvh(run):
+    """After a rebuild that was refused its memory the BVH holds nothing: the next smaller
+    rebuild allocates anew instead of launching on arrays that are gone."""
+    out = run("""
+bvh = ctx.build_lbvh(triangles(1000))
+fake.fake_set_limit(fake.fake_used() + (1 << 20))
+log()
+try:
+    bvh.rebuild(triangles(100000))
+    status = 0
+except L.LuxError as e:
+    status = e.status
+refused = log()
+bvh.rebuild(triangles(2000))
+out = [status, refused, log()]
+""")
+    status, refused, again = out
+    assert status == 3 and not any(s.startswith("launch") for s in refused)
+    first_launch = next(i for i, s in enumerate(again) if s.startswith("launch"))
+    sizes = [int(s.split()[1]) for s in again[:first_launch] if s.startswith("malloc")]
+    assert max(sizes, default=0) > 100 * 2000, again
