@@ -1471,14 +1471,20 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
          sizeof(int) * static_cast<size_t>(grid_for(capacity, kClimbThreads))},
         {&bvh->codes, key * n},
         {reinterpret_cast<void**>(&bvh->root), sizeof(float) * 16},
-        // Triangles are built to be traced: their 4-wide nodes have their place from the start.
-        {reinterpret_cast<void**>(&bvh->wide),
-         bvh->kind == LUX_PRIM_TRIANGLES ? sizeof(WideNode) * inner : 0},
     };
     size_t total = 0;
     for (const auto& r : reqs) total += (r.bytes + 255) & ~size_t(255);
+    // Triangles are built to be traced: their 4-wide nodes have their place from the start,
+    // unless only the other arrays fit (the first ray query then asks for it).
+    size_t wide_bytes = bvh->kind == LUX_PRIM_TRIANGLES ? sizeof(WideNode) * inner : 0;
     char* base = nullptr;
-    if (cudaMalloc(reinterpret_cast<void**>(&base), total) != cudaSuccess) {
+    cudaError_t got = cudaMalloc(reinterpret_cast<void**>(&base), total + wide_bytes);
+    if (got != cudaSuccess && wide_bytes) {
+        cudaGetLastError();
+        wide_bytes = 0;
+        got = cudaMalloc(reinterpret_cast<void**>(&base), total);
+    }
+    if (got != cudaSuccess) {
         cudaGetLastError();
         lbvh_free(bvh);
         return fail(LUX_ERR_OUT_OF_MEMORY, "lbvh allocation failed");
@@ -1489,8 +1495,11 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
         *r.ptr = base;
         base += (r.bytes + 255) & ~size_t(255);
     }
-    bvh->wide_capacity = bvh->kind == LUX_PRIM_TRIANGLES ? static_cast<int>(inner) : 0;
-    if (!bvh->wide_capacity) bvh->wide = nullptr;
+    if (wide_bytes) {
+        bvh->wide = reinterpret_cast<WideNode*>(base);
+        bvh->wide_capacity = static_cast<int>(inner);
+        bvh->wide_in_arena = true;
+    }
     // A build's list of open subtrees ends with the build; the refits' node records are made
     // after it.
     static_assert(sizeof(int4) >= sizeof(int2), "open subtrees in the node records' place");
@@ -1505,12 +1514,13 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
 }
 
 void lbvh_free(lux_bvh* bvh) {
-    if (bvh->wide && bvh->kind != LUX_PRIM_TRIANGLES) cudaFree(bvh->wide);
+    if (bvh->wide && !bvh->wide_in_arena) cudaFree(bvh->wide);
     if (bvh->arena) cudaFree(bvh->arena);
     bvh->arena = nullptr;
     bvh->capacity = 0;
     bvh->wide = nullptr;
     bvh->wide_capacity = 0;
+    bvh->wide_in_arena = false;
     bvh->wide_current = false;
     bvh->info_current = false;
     bvh->nodes = nullptr;
@@ -1734,6 +1744,7 @@ int lbvh_ensure_wide(lux_ctx* ctx, lux_bvh* bvh) {
     if (bvh->wide_current || bvh->n <= 1) return LUX_OK;
     int need = std::max(bvh->capacity - 1, 1);
     if (bvh->wide_capacity < need) {
+        // Nodes in the arena have its capacity: what is freed here is an allocation of its own.
         if (bvh->wide) cudaFree(bvh->wide);
         bvh->wide = nullptr;
         bvh->wide_capacity = 0;

@@ -61,9 +61,10 @@ struct lux_bvh {
     int* open_count = nullptr;          // their number, per climb block
     void* codes = nullptr;              // n sorted codes (uint32 or uint64)
     float* root = nullptr;              // 6
-    lux::WideNode* wide = nullptr;      // capacity - 1, built on demand for ray queries
+    lux::WideNode* wide = nullptr;      // capacity - 1, made on demand for ray queries
     bool wide_current = false;          // wide matches nodes (cleared by build/refit)
     int wide_capacity = 0;              // wide nodes allocated
+    bool wide_in_arena = false;         // in the arena, not an allocation of their own
     lux::BvhView view() const {
         lux::BvhView v;
         v.nodes = nodes;

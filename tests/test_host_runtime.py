@@ -113,3 +113,33 @@ out = [status, refused, log()]
     first_launch = next(i for i, s in enumerate(again) if s.startswith("launch"))
     sizes = [int(s.split()[1]) for s in again[:first_launch] if s.startswith("malloc")]
     assert max(sizes, default=0) > 100 * 2000, again
+
+
+def test_a_build_needs_no_room_for_the_wide_nodes(run):
+    """Where a triangle BVH's 4-wide nodes do not fit beside its other arrays, the build still
+    succeeds, as it does for a BVH that is only refitted or downloaded; the first ray query asks
+    for them again."""
+    out = run("""
+n = 200000
+bvh = ctx.build_lbvh(triangles(n))           # grows the context's scratch and staging
+bvh.close()
+rays = np.zeros((64, 8), np.float32)
+used = fake.fake_used()
+log()
+fake.fake_set_limit(used + 160 * n)
+bvh = ctx.build_lbvh(triangles(n))
+bvh.refit(triangles(n))
+built = log()
+try:
+    bvh.trace_closest(rays)
+    status = 0
+except L.LuxError as e:
+    status = e.status
+fake.fake_set_limit(used + 400 * n)
+bvh.trace_closest(rays)
+bvh.close()
+out = [status, launched(built), fake.fake_used() - used, log()]
+""")
+    status, kernels, left, rest = out
+    assert "k_climb" in kernels and status == 3
+    assert left == 0 and not any("unknown" in s for s in rest)
