@@ -44,8 +44,9 @@ struct PathPool {
     int* qshadow = nullptr;
 };
 
-// Device buffers of a pool (wavefront.cu).
-int path_pool_alloc(PathPool& pool, int capacity);
+// Device buffers of a pool (wavefront.cu), without the ray queues if the paths need no order
+// of their own; adds what they take to *bytes.
+int path_pool_alloc(PathPool& pool, int capacity, bool ray_queues, int64_t* bytes = nullptr);
 void path_pool_free(PathPool& pool);
 
 namespace {

@@ -398,7 +398,7 @@ struct lux_server {
     int max_requests = 256;
     int64_t budget = 0;
     int64_t used = 0;
-    int64_t pool_bytes = 0;
+    int64_t pool_bytes = 0;         // of the two pools and the queues beside them
     long long ticket_limit = 0;
     // host state
     std::mutex mu;
@@ -823,7 +823,7 @@ int lux_server_create(int device, lux_scene* const* scenes, int32_t scene_count,
     s->max_requests = max_requests;
     s->budget = opt.memory_budget_bytes > 0 ? opt.memory_budget_bytes : (int64_t(120) << 30);
     int cap = static_cast<int>(pool_paths);
-    st = path_pool_alloc(s->pool[0], cap);
+    st = path_pool_alloc(s->pool[0], cap, false, &s->pool_bytes);
     std::vector<SceneView> views;
     for (lux_scene* sc : s->scenes) views.push_back(sc->view);
     auto dmalloc = [&](void** p, size_t bytes) {
@@ -840,13 +840,16 @@ int lux_server_create(int device, lux_scene* const* scenes, int32_t scene_count,
         p1 = s->pool[0];
         p1.state = p1.ray = p1.rad = nullptr;
     }
-    dmalloc(reinterpret_cast<void**>(&s->pool[1].state), 4 * sizeof(float4) * cap);
-    dmalloc(reinterpret_cast<void**>(&s->pool[1].ray), 2 * sizeof(float4) * cap);
-    dmalloc(reinterpret_cast<void**>(&s->pool[1].rad), sizeof(float4) * cap);
-    dmalloc(reinterpret_cast<void**>(&s->req_of[0]), sizeof(int) * cap);
-    dmalloc(reinterpret_cast<void**>(&s->req_of[1]), sizeof(int) * cap);
-    dmalloc(reinterpret_cast<void**>(&s->sh_dest), sizeof(int) * cap);
-    dmalloc(reinterpret_cast<void**>(&s->qterm), sizeof(int) * cap);
+    // Arrays of `per` bytes a path, part of what the pool is charged against the budget.
+    auto per_path = [&](auto** p, size_t per) {
+        dmalloc(reinterpret_cast<void**>(p), per * static_cast<size_t>(cap));
+        s->pool_bytes += static_cast<int64_t>(per) * cap;
+    };
+    per_path(&s->pool[1].state, 4 * sizeof(float4));
+    per_path(&s->pool[1].ray, 2 * sizeof(float4));
+    per_path(&s->pool[1].rad, sizeof(float4));
+    for (int** p : {&s->req_of[0], &s->req_of[1], &s->sh_dest, &s->qterm})
+        per_path(p, sizeof(int));
     dmalloc(reinterpret_cast<void**>(&s->st), sizeof(ServerState));
     dmalloc(reinterpret_cast<void**>(&s->d_req), sizeof(ReqSlot) * max_requests);
     dmalloc(reinterpret_cast<void**>(&s->d_tmap), sizeof(TicketMap));
@@ -885,8 +888,6 @@ int lux_server_create(int device, lux_scene* const* scenes, int32_t scene_count,
         delete s;
         return st;
     }
-    // Pool, queues and records, plus the second pool's path state and request slots.
-    s->pool_bytes = static_cast<int64_t>(cap) * (16 * 12 + 4 * 7 + 4 * kClasses + 16 * 7 + 4 + 4);
     s->used = s->pool_bytes;
     for (int k = max_requests - 1; k >= 0; --k) s->free_slots.push_back(k);
     s->worker = std::thread(worker_main, s);

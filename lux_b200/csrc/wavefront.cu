@@ -311,8 +311,8 @@ void path_pool_free(PathPool& p) {
 }
 
 // Shared by the server: device buffers of a path pool of `capacity` paths.
-int path_pool_alloc(PathPool& p, int capacity) {
-    size_t c = static_cast<size_t>(capacity);
+int path_pool_alloc(PathPool& p, int capacity, bool ray_queues, int64_t* bytes) {
+    const size_t c = static_cast<size_t>(capacity), q = ray_queues ? 4 * c : 0;
     struct Req {
         void** ptr;
         size_t bytes;
@@ -320,11 +320,13 @@ int path_pool_alloc(PathPool& p, int capacity) {
         {reinterpret_cast<void**>(&p.state), 64 * c}, {reinterpret_cast<void**>(&p.ray), 32 * c},
         {reinterpret_cast<void**>(&p.shadow), 64 * c}, {reinterpret_cast<void**>(&p.rad), 16 * c},
         {reinterpret_cast<void**>(&p.hit), 16 * c},
-        {reinterpret_cast<void**>(&p.qray[0]), 4 * c}, {reinterpret_cast<void**>(&p.qray[1]), 4 * c},
+        {reinterpret_cast<void**>(&p.qray[0]), q}, {reinterpret_cast<void**>(&p.qray[1]), q},
         {reinterpret_cast<void**>(&p.qshadow), 4 * c},
     };
     for (auto& r : reqs) {
+        if (r.bytes == 0) continue;
         cudaError_t err = cudaMalloc(r.ptr, r.bytes);
+        if (bytes) *bytes += static_cast<int64_t>(r.bytes);
         if (err != cudaSuccess) {
             cudaGetLastError();
             return fail(LUX_ERR_OUT_OF_MEMORY, "path pool allocation failed");
@@ -358,7 +360,7 @@ int runtime_reserve(lux_ctx* ctx, int capacity, int max_depth, int lanes) {
     int st = LUX_OK;
     cudaError_t err = cudaSuccess;
     for (int l = 0; l < lanes && !st && err == cudaSuccess; ++l) {
-        st = path_pool_alloc(rt->pool[l], capacity);
+        st = path_pool_alloc(rt->pool[l], capacity, true);
         if (!st) err = cudaMalloc(&rt->counts[l], sizeof(int) * kSlots * kMaxDepthSlots);
     }
     if (!st && err == cudaSuccess) err = cudaMalloc(&rt->rays, 16);

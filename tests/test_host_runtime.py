@@ -143,3 +143,24 @@ out = [status, launched(built), fake.fake_used() - used, log()]
     status, kernels, left, rest = out
     assert "k_climb" in kernels and status == 3
     assert left == 0 and not any("unknown" in s for s in rest)
+
+
+def test_a_server_accounts_for_the_pools_it_allocates(run):
+    """bytes_in_use of an idle server is what its path pools took, and none of their arrays is
+    a per-path array that only single renders use."""
+    out = run("""
+from lux_b200 import scene as S, server as SV
+scene = S.Scene(ctx, S.make_cornell_scene(32, 32))
+out = []
+for paths in (1 << 14, 1 << 15):
+    log()
+    with SV.Server([scene], pool_paths=paths) as srv:
+        out.append([srv.stats()["bytes_in_use"],
+                    [int(s.split()[1]) for s in log() if s.startswith("malloc")]])
+""")
+    (small, a), (large, b) = out
+    per_path = [y - x for x, y in zip(a, b)]         # what grows with the pool
+    assert large - small == sum(per_path) and small == sum(per_path), (small, sum(per_path))
+    # state, ray, radiance and request of two pools; shadow, hit, shadow queue, where a shadow
+    # ray's path went, ended paths
+    assert small == (1 << 14) * (2 * (64 + 32 + 16 + 4) + 64 + 16 + 4 + 4 + 4)
