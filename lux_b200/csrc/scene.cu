@@ -1079,7 +1079,7 @@ int blocks_for(lux_ctx* ctx, int64_t items) {
 }
 
 // First update of a mesh: device vertex/index buffers and its instance/TLAS-entry lists.
-int prepare_refit(lux_scene* s, int mesh) {
+int prepare_refit(lux_ctx* ctx, lux_scene* s, int mesh) {
     if (s->refit.size() < s->blas.size()) s->refit.resize(s->blas.size());
     lux_scene::MeshRefit& r = s->refit[mesh];
     if (r.vertices) return LUX_OK;
@@ -1096,12 +1096,13 @@ int prepare_refit(lux_scene* s, int mesh) {
         err = cudaMalloc(&r.indices, sizeof(uint32_t) * std::max<size_t>(1, idx.size()));
     if (err == cudaSuccess)
         err = cudaMalloc(&r.instances, sizeof(int) * std::max<size_t>(1, lists.size()));
+    // From pageable memory, so staged before the calls return, in order before the kernels.
     if (err == cudaSuccess && !idx.empty())
-        err = cudaMemcpy(r.indices, idx.data(), sizeof(uint32_t) * idx.size(),
-                         cudaMemcpyHostToDevice);
+        err = cudaMemcpyAsync(r.indices, idx.data(), sizeof(uint32_t) * idx.size(),
+                              cudaMemcpyHostToDevice, ctx->stream);
     if (err == cudaSuccess && !lists.empty())
-        err = cudaMemcpy(r.instances, lists.data(), sizeof(int) * lists.size(),
-                         cudaMemcpyHostToDevice);
+        err = cudaMemcpyAsync(r.instances, lists.data(), sizeof(int) * lists.size(),
+                              cudaMemcpyHostToDevice, ctx->stream);
     if (err != cudaSuccess) {
         cudaFree(r.vertices);
         cudaFree(r.indices);
@@ -1121,7 +1122,7 @@ int scene_update_mesh(lux_ctx* ctx, lux_scene* s, int mesh, const float* vertice
     if (view_changed) *view_changed = false;
     if (mesh < 0 || mesh >= static_cast<int>(s->blas.size()))
         return fail(LUX_ERR_INVALID_ARGUMENT, "mesh out of range");
-    if (int st = prepare_refit(s, mesh)) return st;
+    if (int st = prepare_refit(ctx, s, mesh)) return st;
     std::vector<float>& verts = s->mesh_vertices[mesh];
     std::memcpy(verts.data(), vertices, sizeof(float) * verts.size());
     const lux_scene::MeshRefit& r = s->refit[mesh];

@@ -164,3 +164,18 @@ for paths in (1 << 14, 1 << 15):
     # state, ray, radiance and request of two pools; shadow, hit, shadow queue, where a shadow
     # ray's path went, ended paths
     assert small == (1 << 14) * (2 * (64 + 32 + 16 + 4) + 64 + 16 + 4 + 4 + 4)
+
+
+def test_a_mesh_update_uploads_in_stream_order(run):
+    """Everything a mesh's first update uploads goes through the context's stream, on which its
+    kernels read it: a pageable copy on the default stream may still be on its way when they
+    start."""
+    lines = run("""
+from lux_b200 import scene as S
+scene = S.Scene(ctx, S.make_cornell_scene(32, 32))
+log()
+scene.update_mesh(0, np.zeros((36, 3), np.float32))
+out = log()
+""")
+    copies = [s for s in lines if s.startswith("memcpy")]
+    assert len(copies) >= 3 and not any("default" in s for s in copies), copies
