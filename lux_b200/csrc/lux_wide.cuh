@@ -18,7 +18,11 @@
 
 namespace lux {
 
-constexpr int kWideStack = 116;  // three deferred children per wide level
+// Deferred children of the deepest walk.  A path has at most 93 binary nodes (prefix lengths
+// 1 to 63 of 63-bit codes, then 30 more of up to 2^30 equal ones' indices), a wide node takes
+// two or more of them and defers at most three: 47 * 3 = 141.  (Room that is not used costs
+// nothing: 2,048 to 4,194,304 rays of a 1M-triangle tree take the same at 116, 144 and 160.)
+constexpr int kWideStack = 144;
 
 LUX_D WideNode load_wide(const WideNode* wide, int i) {
     WideNode w;

@@ -293,7 +293,7 @@ LUX_D SceneHit scene_closest(const SceneView& sc, f3 o, f3 d, float tmin, float 
 // not below the current one, and leaves are tested in order under the bound of their turn.
 // The world-space ray is not kept: tlas() is handed it again when a BLAS is left.  The
 // stacks live apart from the scalar state, which then stays in registers.
-constexpr int kWideStackPt = 100;     // three deferred children per 4-wide level
+constexpr int kWideStackPt = 100;     // as kWideStack, of 30-bit codes: 60 nodes, 30 * 3 = 90
 constexpr int kFlatTlas = 4;          // TLAS leaves tested together when a walk starts
 
 struct WalkStacks {  // deferred (node ref, entry t bits), TLAS and BLAS

@@ -502,3 +502,49 @@ def test_climb_blocks_match_oracle(ctx, oracle, n, kind, chain):
         assert bvh.validate()[0]
     bvh.rebuild(moved_prims)
     _assert_tree_equal(bvh.download(), oracle.build(moved_boxes))
+
+
+def deep_boxes(equal=1 << 15):
+    """Boxes around one corner whose 63-bit hierarchy is as deep as its codes allow on the side
+    that a walk takes first: at each of the 63 levels one box or two (in turn, the two with the
+    larger area) leave the path, and `equal` boxes with the same code end it."""
+    c = []
+    for k in range(20, -1, -1):
+        for a in range(3):
+            at = np.full(3, 0.25)
+            if (3 * (20 - k) + a) % 2 == 0:
+                at[a] = 2.0 ** k
+                c.append(at)
+                continue
+            for step in (1.0, 1.5):
+                if k > 0:
+                    at = np.array([2.0 ** k * (0.98 if x < a else 1.98) for x in range(3)])
+                at[a] = 2.0 ** k * step
+                c.append(np.minimum(at, 2.0 ** 20) if k == 20 else at.copy())
+    c = np.array(c + [np.full(3, 0.25)] * equal)
+    return np.concatenate([np.zeros_like(c), 2 * c], 1).astype(np.float32)
+
+
+# A ray into the corner passes every box: the walk defers up to three children at each of its
+# nodes, 114 in all before the last of them.
+@pytest.mark.parametrize("variant", [1, 2, 3, 4])
+def test_walks_of_the_deepest_hierarchies_match_oracle(ctx, oracle, variant):
+    boxes = deep_boxes()
+    n = len(boxes)
+    tris = np.tile(np.float32([0.5, 0, 0, 0, 0.5, 0, 0, 0, 0.5]), (n, 1))
+    rays = np.zeros((40, 8), np.float32)
+    rays[:, 0:3] = -1.0 - np.arange(40)[:, None] * 0.01
+    rays[:, 4:7] = 1.0
+    rays[:, 7] = np.inf
+    rays[::2, 7] = 1.0                      # ends in the corner, before any triangle
+    want_id, want_t = oracle.trace(tris, oracle.build(boxes, 63), rays)
+    assert (want_id >= 0).sum() == 20
+    bvh = ctx.build_lbvh(boxes, lux_b200.PRIM_AABBS, 63)
+    bvh.attach_triangles(tris)
+
+    def check():
+        got_id, got_t = bvh.trace_closest(rays)
+        assert np.array_equal(got_id, want_id) and np.array_equal(got_t, want_t)
+        assert np.array_equal(bvh.trace_any(rays) >= 0, want_id >= 0)
+
+    _with_variant(ctx, variant, check)
