@@ -613,11 +613,11 @@ struct Subtree {
     LUX_D int id() const { return is_root() ? 0 : is_left() ? last : first; }
 };
 
-// Joins left = [.., s] and right = [s + 1, ..] and writes the new node's record, parent
-// links included.  ch.z, ch.w of the record: the other end of its leaves and the prefix
-// length beyond it, which the sibling that meets this node in global memory reads.
-LUX_D Subtree join(const Subtree& left, const Subtree& right, BvhNode* nodes, int* leaf_parent,
-                   int* node_parent) {
+// Joins left = [.., s] and right = [s + 1, ..] and writes the new node's record and its
+// children's parent links.  ch.z, ch.w of the record: the other end of its leaves and, until
+// the node is joined itself, the prefix length beyond it, which the sibling that meets this
+// node in global memory reads; then its parent link (-1 for the root, as its prefix length).
+LUX_D Subtree join(const Subtree& left, const Subtree& right, BvhNode* nodes, int* leaf_parent) {
     Subtree t;
     t.b = box_union(left.b, right.b);
     t.first = left.first;
@@ -635,9 +635,8 @@ LUX_D Subtree join(const Subtree& left, const Subtree& right, BvhNode* nodes, in
          make_float4(__int_as_float(ll ? ~s : s), __int_as_float(rl ? ~(s + 1) : s + 1),
                      __int_as_float(side ? t.first : t.last),
                      __int_as_float(side ? t.dl : t.dr)));
-    (ll ? leaf_parent : node_parent)[s] = id << 1;
-    (rl ? leaf_parent : node_parent)[s + 1] = (id << 1) | 1;
-    if (t.is_root()) node_parent[0] = -1;
+    *(ll ? leaf_parent + s : &nodes[s].ch.w) = id << 1;
+    *(rl ? leaf_parent + s + 1 : &nodes[s + 1].ch.w) = (id << 1) | 1;
     return t;
 }
 
@@ -672,7 +671,7 @@ constexpr int small_build_smem() {
 template <int Kind, typename Key, bool Whole>
 __global__ void __launch_bounds__(kSmallThreads) k_build_small(
         const float* prims, int n, Key* codes, int* sorted_ids, TriRecord* tris, BvhNode* nodes,
-        int* leaf_parent, int* node_parent, float* root_box) {
+        int* leaf_parent, float* root_box) {
     constexpr int kWarps = kSmallThreads / 32;
     constexpr int kPasses = sizeof(Key) == 4 ? 4 : 8;
     constexpr int kMax = Whole ? kWholeBuild : kSmallSort;
@@ -882,8 +881,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(
             o.last = left ? send[sib] : sib;
             o.dl = left ? t.dr : sdelta[o.first];
             o.dr = left ? sdelta[o.last + 1] : t.dl;
-            t = left ? join(t, o, nodes, leaf_parent, node_parent)
-                     : join(o, t, nodes, leaf_parent, node_parent);
+            t = left ? join(t, o, nodes, leaf_parent) : join(o, t, nodes, leaf_parent);
         }
     }
 }
@@ -904,8 +902,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(
 template <int Kind, typename Key>
 __global__ void __launch_bounds__(kClimbThreads, LUX_CLIMB_BLOCKS) k_climb(
         const float* prims, int n, const Key* codes, const int* sorted_ids, TriRecord* tris,
-        BvhNode* nodes, int* leaf_parent, int* node_parent, int2* open, int* open_count,
-        float* root, int* error) {
+        BvhNode* nodes, int* leaf_parent, int2* open, int* open_count, float* root,
+        int* error) {
     constexpr int T = kClimbThreads;
     // By the subtree's number within the block (a left child: its last leaf, a right child:
     // its first): box and other end.  The number is free again once the sibling has read it.
@@ -980,13 +978,13 @@ __global__ void __launch_bounds__(kClimbThreads, LUX_CLIMB_BLOCKS) k_climb(
             o.last = send[sib];
             o.dl = t.dr;
             o.dr = sdelta[o.last + 1 - lo];
-            t = join(t, o, nodes, leaf_parent, node_parent);
+            t = join(t, o, nodes, leaf_parent);
         } else {
             o.first = send[sib];
             o.last = lo + s;
             o.dl = sdelta[o.first - lo];
             o.dr = t.dl;
-            t = join(o, t, nodes, leaf_parent, node_parent);
+            t = join(o, t, nodes, leaf_parent);
         }
     }
     __syncthreads();
@@ -1028,9 +1026,8 @@ constexpr int kTopThreads = 256;
 template <int Kind, typename Key>
 __global__ void __launch_bounds__(kTopThreads) k_climb_top(
         const float* prims, int n, const Key* codes, const int* sorted_ids,
-        const TriRecord* tris, BvhNode* nodes, int* leaf_parent, int* node_parent,
-        const int2* open, const int* open_count, int blocks, unsigned* flags, float* root,
-        int* error) {
+        const TriRecord* tris, BvhNode* nodes, int* leaf_parent, const int2* open,
+        const int* open_count, int blocks, unsigned* flags, float* root, int* error) {
     const int block = (blockIdx.x * kTopThreads + threadIdx.x) >> 5;
     if (block >= blocks) return;
     const int count = min(open_count[block], kClimbThreads);
@@ -1074,13 +1071,13 @@ __global__ void __launch_bounds__(kTopThreads) k_climb_top(
                 o.last = end;
                 o.dl = t.dr;
                 o.dr = !leaf ? ch.w : sib + 1 < n ? delta(codes, sib, sib + 1) : -1;
-                t = join(t, o, nodes, leaf_parent, node_parent);
+                t = join(t, o, nodes, leaf_parent);
             } else {
                 o.first = end;
                 o.last = sib;
                 o.dl = !leaf ? ch.w : sib > 0 ? delta(codes, sib - 1, sib) : -1;
                 o.dr = t.dl;
-                t = join(o, t, nodes, leaf_parent, node_parent);
+                t = join(o, t, nodes, leaf_parent);
             }
             if (t.is_root()) {
                 store_root(root, t.b);
@@ -1113,19 +1110,6 @@ LUX_D box3 load_slot_cg(const BvhNode* node, int slot) {
     return box3{make_f3(a.x, a.y, b.x), make_f3(b.y, b.z, b.w)};
 }
 
-// What a refit's climb reads of a node in one load: its first and last sorted leaf and its
-// parent's code (the node is numbered by one end of its leaves, ch.z is the other).  Made on
-// the first refit of a hierarchy: stored while the nodes are joined, the word more per node
-// takes a build 3 % longer.
-__global__ void __launch_bounds__(kThreads) k_node_info(const BvhNode* nodes,
-                                                        const int* node_parent, int n,
-                                                        int4* node_info) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    const int end = nodes[i].ch.z;
-    node_info[i] = make_int4(min(i, end), max(i, end), node_parent[i], 0);
-}
-
 // Refit: one thread per sorted leaf.  The leaf box (and, for triangles, the sorted triangle
 // record) is written; then the thread climbs: it hands its box to the parent, and the
 // second of the two children to arrive (a counter) unions both and continues upward, so
@@ -1135,15 +1119,15 @@ __global__ void __launch_bounds__(kThreads) k_node_info(const BvhNode* nodes,
 // that range too (a Karras node is numbered by one end of its range), so the hand-over
 // goes through shared memory; above that through the node's slot in global memory with
 // an acquire-release counter, which the second arrival resets to zero.  One 16-byte load
-// of node_info per level gives the node's range and its parent link.  The topology being
-// known, this is one kernel (117 us for 1,048,576 triangles, 22 us for 5,000), where a
-// build's climb and its top take 122 and 27 us.
+// per level, of the last words of the node's record, gives its range and its parent link
+// (from a table of their own 113 us instead of 105 for 1,048,576 triangles, and 15 us to make
+// it after every build).  The topology being known, this is one kernel (105 us for 1,048,576
+// triangles, 20 us for 5,000), where a build's climb and its top take 124 and 30 us.
 template <int Kind>
 __global__ void __launch_bounds__(kClimbThreads) k_refit(const float* prims, int n,
                                                               const int* sorted_ids,
                                                               TriRecord* tris, BvhNode* nodes,
                                                               const int* leaf_parent,
-                                                              const int4* node_info,
                                                               unsigned* flags, float* root,
                                                               int* error) {
     // Per node of the block: each child's box (three float2) and an arrival counter.
@@ -1158,8 +1142,8 @@ __global__ void __launch_bounds__(kClimbThreads) k_refit(const float* prims, int
     // primitive, so the two dependent chains overlap.
     const int pid = sorted_ids[k];
     int code = n > 1 ? leaf_parent[k] : -1;
-    int4 info = make_int4(0, -1, -1, 0);
-    if (code >= 0 && (code >> 1) < n - 1) info = node_info[code >> 1];
+    int4 info = make_int4(0, 0, -1, -1);   // the last words of the parent's record
+    if (code >= 0 && (code >> 1) < n - 1) info = nodes[code >> 1].ch;
     if (pid < 0 || pid >= n) {  // cannot happen for a consistent sort
         atomicOr(error, kErrLoopBound);
         return;
@@ -1185,11 +1169,12 @@ __global__ void __launch_bounds__(kClimbThreads) k_refit(const float* prims, int
         if (code < 0 || p >= n - 1) break;  // parent links out of range: report below
         // The grandparent's record is requested now, before the hand-over, so its load
         // overlaps this level's (for the half of the threads that go on).
-        const int up = info.z;
-        int4 next = make_int4(0, -1, -1, 0);
-        if (up >= 0 && (up >> 1) < n - 1) next = node_info[up >> 1];
-        const int s = p - lo;
-        if (info.x >= lo && info.y < lo + kClimbThreads && s >= 0 && s < kClimbThreads) {
+        const int up = info.w;
+        int4 next = make_int4(0, 0, -1, -1);
+        if (up >= 0 && (up >> 1) < n - 1) next = nodes[up >> 1].ch;
+        // Both ends of the node's leaves: its number and ch.z.
+        const int s = p - lo, other = info.z - lo;
+        if (s >= 0 && s < kClimbThreads && other >= 0 && other < kClimbThreads) {
             // The block fences order the box's stores before the counter's add, and the
             // add before the sibling's box is read (they are also compiler barriers).
             float2* mine = &sbox[s][slot][0];
@@ -1388,29 +1373,23 @@ int climb(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
     const Key* codes = static_cast<const Key*>(bvh->codes);
     cudaError_t err = chain_launch(ctx, k_climb<Kind, Key>, blocks, kClimbThreads, 0, prims,
                                    bvh->n, codes, bvh->sorted_ids, bvh->tris, bvh->nodes,
-                                   bvh->leaf_parent, bvh->node_parent, bvh->open,
-                                   bvh->open_count, bvh->root, ctx->d_error);
+                                   bvh->leaf_parent, bvh->open, bvh->open_count, bvh->root,
+                                   ctx->d_error);
     if (err == cudaSuccess && blocks > 1)
         err = chain_launch(ctx, k_climb_top<Kind, Key>, grid_for(blocks, kTopThreads / 32),
                            kTopThreads, 0, prims, bvh->n, codes, bvh->sorted_ids, bvh->tris,
-                           bvh->nodes, bvh->leaf_parent, bvh->node_parent, bvh->open,
-                           bvh->open_count, blocks, bvh->flags, bvh->root, ctx->d_error);
+                           bvh->nodes, bvh->leaf_parent, bvh->open, bvh->open_count, blocks,
+                           bvh->flags, bvh->root, ctx->d_error);
     return cuda_fail(err, "climb");
 }
 
 template <int Kind>
 int refit(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
-    cudaError_t err = cudaSuccess;
-    if (!bvh->info_current && bvh->n > 1)
-        err = chain_launch(ctx, k_node_info, grid_for(bvh->n - 1), kThreads, 0, bvh->nodes,
-                           bvh->node_parent, bvh->n, bvh->node_info);
-    if (err == cudaSuccess)
-        err = chain_launch(ctx, k_refit<Kind>, grid_for(bvh->n, kClimbThreads), kClimbThreads, 0,
-                           prims, bvh->n, bvh->sorted_ids, bvh->tris, bvh->nodes,
-                           bvh->leaf_parent, bvh->node_info, bvh->flags, bvh->root,
-                           ctx->d_error);
-    if (err == cudaSuccess) bvh->info_current = true;
-    return cuda_fail(err, "refit");
+    return cuda_fail(chain_launch(ctx, k_refit<Kind>, grid_for(bvh->n, kClimbThreads),
+                                  kClimbThreads, 0, prims, bvh->n, bvh->sorted_ids, bvh->tris,
+                                  bvh->nodes, bvh->leaf_parent, bvh->flags, bvh->root,
+                                  ctx->d_error),
+                     "refit");
 }
 
 template <int Kind, typename Key>
@@ -1430,7 +1409,7 @@ int build_typed(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
         if (err == cudaSuccess)
             err = chain_launch(ctx, kernel, 1, kSmallThreads, smem, prims, n, codes,
                                bvh->sorted_ids, bvh->tris, bvh->nodes, bvh->leaf_parent,
-                               bvh->node_parent, bvh->root);
+                               bvh->root);
         if (err != cudaSuccess) return cuda_fail(err, "k_build_small");
         return whole ? LUX_OK : climb<Kind, Key>(ctx, bvh, prims);
     }
@@ -1464,9 +1443,8 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
         {reinterpret_cast<void**>(&bvh->tris), sizeof(TriRecord) * n},
         {reinterpret_cast<void**>(&bvh->sorted_ids), sizeof(int) * n},
         {reinterpret_cast<void**>(&bvh->leaf_parent), sizeof(int) * n},
-        {reinterpret_cast<void**>(&bvh->node_parent), sizeof(int) * inner},
-        {reinterpret_cast<void**>(&bvh->node_info), sizeof(int4) * inner},
         {reinterpret_cast<void**>(&bvh->flags), sizeof(unsigned) * inner},
+        {reinterpret_cast<void**>(&bvh->open), sizeof(int2) * n},
         {reinterpret_cast<void**>(&bvh->open_count),
          sizeof(int) * static_cast<size_t>(grid_for(capacity, kClimbThreads))},
         {&bvh->codes, key * n},
@@ -1500,10 +1478,6 @@ int lbvh_alloc(lux_ctx* ctx, lux_bvh* bvh) {
         bvh->wide_capacity = static_cast<int>(inner);
         bvh->wide_in_arena = true;
     }
-    // A build's list of open subtrees ends with the build; the refits' node records are made
-    // after it.
-    static_assert(sizeof(int4) >= sizeof(int2), "open subtrees in the node records' place");
-    bvh->open = reinterpret_cast<int2*>(bvh->node_info);
     // On the context's stream: one on the default stream has no order with the build that
     // follows on a non-blocking stream.
     cudaError_t err = cudaMemsetAsync(bvh->flags, 0, sizeof(unsigned) * inner, ctx->stream);
@@ -1522,13 +1496,10 @@ void lbvh_free(lux_bvh* bvh) {
     bvh->wide_capacity = 0;
     bvh->wide_in_arena = false;
     bvh->wide_current = false;
-    bvh->info_current = false;
     bvh->nodes = nullptr;
     bvh->tris = nullptr;
     bvh->sorted_ids = nullptr;
     bvh->leaf_parent = nullptr;
-    bvh->node_parent = nullptr;
-    bvh->node_info = nullptr;
     bvh->flags = nullptr;
     bvh->open = nullptr;
     bvh->open_count = nullptr;
@@ -1538,7 +1509,6 @@ void lbvh_free(lux_bvh* bvh) {
 
 int lbvh_build(lux_ctx* ctx, lux_bvh* bvh, const float* prims) {
     bvh->wide_current = false;
-    bvh->info_current = false;
     if (bvh->n <= 0) return LUX_OK;
     bool wide = bvh->morton_bits == 63;
     if (bvh->kind == LUX_PRIM_TRIANGLES) {

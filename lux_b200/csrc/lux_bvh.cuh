@@ -32,7 +32,9 @@ struct alignas(32) BvhNode {
     float4 a;  // left.lo.x  left.lo.y  left.lo.z  left.hi.x
     float4 b;  // left.hi.y  left.hi.z  right.lo.x right.lo.y
     float4 c;  // right.lo.z right.hi.x right.hi.y right.hi.z
-    int4 ch;   // left handle, right handle, unused, unused
+    // Left handle, right handle; the other end of the node's leaves (its number is one); its
+    // parent link as leaf_parent's.
+    int4 ch;
 };
 static_assert(sizeof(BvhNode) == 64, "one node is one 64-byte record");
 

@@ -52,12 +52,8 @@ struct lux_bvh {
     lux::TriRecord* tris = nullptr;     // n (triangle BVHs)
     int* sorted_ids = nullptr;          // n
     int* leaf_parent = nullptr;         // n
-    int* node_parent = nullptr;         // n - 1: parent code
-    int4* node_info = nullptr;          // n - 1: first and last sorted leaf, parent code
-    bool info_current = false;          // node_info matches the hierarchy (cleared by builds)
     unsigned* flags = nullptr;          // n - 1, zero between passes
     int2* open = nullptr;               // n: leaf ranges of the subtrees a climb block leaves
-                                        // (in node_info's memory)
     int* open_count = nullptr;          // their number, per climb block
     void* codes = nullptr;              // n sorted codes (uint32 or uint64)
     float* root = nullptr;              // 6

@@ -77,12 +77,14 @@ int download(lux_ctx* ctx, const lux_bvh* bvh, Downloaded& d) {
     float root[6];
     cudaError_t err = cudaMemcpy(d.leaf_parent.data(), bvh->leaf_parent, sizeof(int) * n,
                                  cudaMemcpyDeviceToHost);
+    std::vector<lux::BvhNode> nodes(std::max(n - 1, 0));
     if (err == cudaSuccess && n > 1)
-        err = cudaMemcpy(d.node_parent.data(), bvh->node_parent, sizeof(int) * (n - 1),
+        err = cudaMemcpy(nodes.data(), bvh->nodes, sizeof(lux::BvhNode) * nodes.size(),
                          cudaMemcpyDeviceToHost);
     if (err == cudaSuccess)
         err = cudaMemcpy(root, bvh->root, sizeof(root), cudaMemcpyDeviceToHost);
     if (err != cudaSuccess) return lux::cuda_fail(err, "validator download");
+    for (int i = 0; i < n - 1; ++i) d.node_parent[i] = nodes[i].ch.w;
     d.root = box_at(root);
     return LUX_OK;
 }

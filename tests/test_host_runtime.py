@@ -179,3 +179,17 @@ out = log()
 """)
     copies = [s for s in lines if s.startswith("memcpy")]
     assert len(copies) >= 3 and not any("default" in s for s in copies), copies
+
+
+def test_the_first_refit_after_a_build_is_one_launch(run):
+    """The build leaves all that a refit reads: no pass of its own over the nodes."""
+    out = run("""
+out = []
+for n in (1000, 5000, 20000):
+    bvh = ctx.build_lbvh(triangles(n))
+    for again in range(2):
+        log()
+        bvh.refit(triangles(n, 1))
+        out.append(launched(log()))
+""")
+    assert out == [["k_refit"]] * 6, out
