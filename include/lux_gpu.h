@@ -79,7 +79,8 @@ int lux_ctx_launch_count(lux_ctx* ctx, int64_t* count);
  *   LUX_OPT_PATH_BUDGET    the same of the path tracer's walks (variant 1 uses one thread
  *                          per path instead)
  *   LUX_OPT_REFILL_BLOCKS  resident 256-thread blocks per SM of those refilling kernels'
- *                          persistent grids (0: as many as fit, else 1..3)
+ *                          persistent grids (0: as many as fit, three for batches of up
+ *                          to 2^20 paths, four for larger ones; else at most 1..3)
  * Read only (lux_ctx_get_option), the device memory the context holds for reuse:
  *   LUX_OPT_SCRATCH_BYTES  growable scratch of builds and queries
  *   LUX_OPT_STAGING_BYTES  growable staging of host arguments */

@@ -176,7 +176,8 @@ extern "C" int lux_autotune_render(lux_ctx* ctx, const lux_scene* scene,
     // warps, more cache and shared bandwidth each).
     int tried = static_cast<int>(cands.size());
     if (!st && best.variant != lux::kTraceStatic) {
-        for (int blocks : {1, 2}) {
+        const int fit = std::min<long long>(best.batch, paths) > lux::kManyPaths ? 4 : 3;
+        for (int blocks = 1; blocks < fit; ++blocks) {
             Candidate c = best;
             c.blocks = blocks;
             float ms = 0;

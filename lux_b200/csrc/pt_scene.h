@@ -98,6 +98,10 @@ int scene_update_mesh(lux_ctx* ctx, lux_scene* scene, int mesh, const float* ver
 int camera_perspective(const float* origin, const float* look_at, float vfov, float aspect,
                        float lens_radius, float focal_distance, lux_camera_desc* out);
 
+// Paths in a batch above which the bounce kernels run at four blocks per SM instead of three
+// (the measurements stand at k_walk).
+constexpr long long kManyPaths = 1 << 20;
+
 // Wavefront renderer (wavefront.cu).  out is a device pointer: film sums (width*height*3)
 // or, when per_sample, every sample's radiance ((pixel*spp + s)*3).  Non-null aov_*
 // (device, width*height*3) receive the debug images' per-pixel sums.

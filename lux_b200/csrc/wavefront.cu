@@ -92,8 +92,6 @@ __global__ void __launch_bounds__(kThreads) k_extend(PathPool rt, int* counts, S
 // kManyPaths, whose walks are bound by how many are in flight (Cornell 4.43 -> 4.32 ms, the
 // heavy scene 12.03 -> 11.64 ms); three (80 registers) below, where the longest walks decide
 // (257 instances, 845,000 paths: 9.60 against 9.73 ms; 77,000 paths: 1.54 against 1.60 ms).
-constexpr long long kManyPaths = 1 << 20;
-
 template <int Blocks>
 __global__ void __launch_bounds__(kThreads, Blocks) k_walk(PathPool rt, int* counts,
                                                            unsigned long long* rays,

@@ -193,3 +193,20 @@ for n in (1000, 5000, 20000):
         out.append(launched(log()))
 """)
     assert out == [["k_refit"]] * 6, out
+
+
+def test_the_autotuner_tries_every_smaller_grid(run):
+    """Resident blocks per SM below those that fit: three fit batches of up to 2^20 paths, four
+    larger ones."""
+    out = run("""
+from lux_b200 import autotune as A, scene as S
+scene = S.Scene(ctx, S.make_cornell_scene(32, 32))
+out = []
+for spp in (4, 2048):
+    log()
+    A.autotune_render(ctx, scene, S.request(32, 32, spp, 0))
+    sm = 148
+    grids = [int(s.split(" grid ")[1].split()[0]) for s in log() if "k_walk" in s]
+    out.append(sorted({g // sm for g in grids}))
+""")
+    assert out == [[1, 2, 4], [1, 2, 3, 4]], out    # (the stand-in says that four blocks fit)
