@@ -1276,20 +1276,24 @@ struct SortScratch {
 };
 
 // Keys per thread of a k_onesweep block: the more the fewer tiles look back, but the longer
-// each tile's chain of ranking rounds.
-constexpr int kFewKeys = 1 << 20, kFewestKeys = 1 << 19;
+// each tile's chain of ranking rounds.  Builds with 4, 8 and 16 keys a thread, in us, of 30-bit
+// codes: 262,144 triangles 118, 118, 134; 393,216 139, 139, 147; 524,288 158, 150, 160; 1,048,576
+// 235, 219, 218; 1,310,720 276, 266, 270; 4,194,304 722, 681, 696; of 63-bit codes: 262,144 159,
+// 176, 198; 393,216 188, 189, 217; 524,288 219, 205, 235; 1,048,576 337, 296, 302; 4,194,304 1035,
+// 897, 941.
+constexpr int kFewKeys = 3 << 17;
 int sort_items(int n) {
 #ifdef LUX_SORT_ITEMS
     return LUX_SORT_ITEMS;
 #endif
-    return n > kFewKeys ? 16 : n > kFewestKeys ? 8 : 4;
+    return n > kFewKeys ? 8 : 4;
 }
 
 SortScratch sort_scratch(int n, size_t key_size, int passes) {
     // Tiles of any count up to n (a smaller one may take smaller tiles), so that a rebuild of
     // fewer primitives never needs more room.
     size_t tiles = 0;
-    for (int m : {n, std::min(n, kFewKeys), std::min(n, kFewestKeys)}) {
+    for (int m : {n, std::min(n, kFewKeys)}) {
         const int tile = kSortThreads * sort_items(m);
         tiles = std::max(tiles, static_cast<size_t>((m + tile - 1) / tile));
     }
@@ -1338,9 +1342,7 @@ int morton_and_sort(lux_ctx* ctx, const float* prims, Key* codes, int* vals, int
                                    vin, kout, vout, n, 8 * p, hist + p * kRadix, words,
                                    counters + p, ctx->d_error);
         };
-        if (items == 16)
-            pass(k_onesweep<Key, true, 16>, k_onesweep<Key, false, 16>, onesweep_smem<Key, 16>());
-        else if (items == 8)
+        if (items == 8)
             pass(k_onesweep<Key, true, 8>, k_onesweep<Key, false, 8>, onesweep_smem<Key, 8>());
         else
             pass(k_onesweep<Key, true, 4>, k_onesweep<Key, false, 4>, onesweep_smem<Key, 4>());

@@ -41,11 +41,12 @@ def test_trace_matches_reference_fixtures(ctx, golden_lbvh):
         assert np.array_equal(aid >= 0, hid >= 0), name
 
 
-# Sizes at the climb's 256-leaf blocks and the sort's 8192-key tiles, at the 4096-key
-# tiles of the allocation-free sort, and well above them.
+# Sizes at the climb's 256-leaf blocks, at multiples of the sort's 2048-key tiles and well
+# above them; then at the size from which its tiles have 4096 keys, and at a last tile of three.
 @pytest.mark.parametrize("n,seed", [(1, 1), (2, 2), (5, 3), (256, 8), (257, 9), (4095, 4),
                                     (4096, 5), (4097, 6), (8191, 10), (8192, 11), (8193, 12),
-                                    (16385, 13), (100_000, 7)])
+                                    (16385, 13), (100_000, 7), (393_216, 14), (393_217, 15),
+                                    (256 * 4096 + 3, 16)])
 @pytest.mark.parametrize("bits", [30, 63])
 def test_build_matches_oracle(ctx, oracle, n, seed, bits):
     tris = W.soup_triangles(n, seed=seed)
