@@ -127,6 +127,55 @@ def test_film_encoders_match_the_reference_writers(ctx, tmp_path):
                                pfm.ctypes.data) == lux_b200.LUX_ERR_INVALID_ARGUMENT
 
 
+def _encoded(film, spp, fmt):
+    """The encoder's arithmetic in numpy: the linear and float forms in float32, exactly; the
+    gamma form's power in 64 bits."""
+    inv = np.float32(1.0) / np.float32(spp)
+    c = film * inv
+    if fmt == 2:
+        return c[::-1].reshape(-1)
+    if fmt == 1:
+        return (np.float32(255.999) * np.clip(c, 0, 1)).astype(np.uint8).reshape(-1)
+    v = np.clip(c / (np.float32(1.0) + c), 0, 1).astype(np.float64)
+    return (np.float32(255.999) * (v ** np.float64(np.float32(1 / 2.2)))).astype(np.uint8).reshape(-1)
+
+
+# The film and the output each on the host or on the device: what is on the host goes through
+# the context's scratch, which a build of more than 6,144 triangles shares.
+@pytest.mark.gpu
+@pytest.mark.parametrize("in_dev", [False, True])
+@pytest.mark.parametrize("out_dev", [False, True])
+def test_film_encoder_matches_its_arithmetic(in_dev, out_dev):
+    import torch
+
+    from lux_b200 import workloads as W
+    ctx = lux_b200.Context(0)
+    rng = np.random.default_rng(6)
+    tris = W.soup_triangles(7000, seed=3)
+    for h, w, spp in ((1, 1, 1), (37, 53, 16), (301, 503, 7), (5, 3, 2)):
+        film = (rng.gamma(0.7, 3.0, (h, w, 3)) * spp).astype(np.float32)
+        film[0, 0] = [0.0, np.float32(1e9), np.float32(0.25 * spp)]
+        for fmt in (0, 1, 2):
+            out = np.zeros(h * w * 3, np.float32 if fmt == 2 else np.uint8)
+            src = torch.from_numpy(film).cuda() if in_dev else film
+            dst = torch.from_numpy(out).cuda() if out_dev else out
+            torch.cuda.synchronize()
+            lux_b200._check(ctx._lib.lux_film_encode(ctx.handle, lux_b200._ptr(src), w, h, spp, fmt,
+                                                     lux_b200._ptr(dst)))
+            got = dst.cpu().numpy() if out_dev else out
+            want = _encoded(film, spp, fmt)
+            if fmt:
+                assert np.array_equal(got, want)
+            else:   # a byte may differ where the value lies within powf's error of a step
+                diff = np.abs(got.astype(int) - want.astype(int))
+                assert diff.max() <= 1 and np.mean(diff > 0) < 1e-3
+        bvh = ctx.build_lbvh(tris)
+        assert bvh.validate(tris) == (True, "")
+    assert ctx._lib.lux_film_encode(ctx.handle, lux_b200._ptr(film), 3, 5, 2, 7,
+                                    lux_b200._ptr(film)) == lux_b200.LUX_ERR_INVALID_ARGUMENT
+    ctx.close()
+
+
 @pytest.mark.gpu
 def test_cli_writes_debug_images(cli, ctx, tmp_path):
     """`-debug-aov shadow,ng,ns` writes <prefix>_shadow / _ng / _ns next to the image (PFM

@@ -549,3 +549,31 @@ def test_walks_of_the_deepest_hierarchies_match_oracle(ctx, oracle, variant):
         assert np.array_equal(bvh.trace_any(rays) >= 0, want_id >= 0)
 
     _with_variant(ctx, variant, check)
+
+
+# One BVH through the lines at which a build takes another form (one block up to 2,048, one
+# block's sort up to 6,144, four keys a thread up to 393,216), down and up again, a refit after
+# each rebuild.
+@pytest.mark.parametrize("bits", [30, 63])
+@pytest.mark.parametrize("kind", [lux_b200.PRIM_TRIANGLES, lux_b200.PRIM_AABBS])
+def test_rebuilds_across_the_forms_of_a_build_then_refits(ctx, oracle, bits, kind):
+    tris = W.soup_triangles(393_217, seed=61)
+    moved = W.jitter_triangles(tris, seed=62, sigma=1e-3)
+    boxes, moved_boxes = oracle.triangle_bounds(tris), oracle.triangle_bounds(moved)
+    own, own_moved = ((tris, moved) if kind == lux_b200.PRIM_TRIANGLES else (boxes, moved_boxes))
+    bvh = ctx.build_lbvh(own[:100], kind, bits)
+    for n in (393_217, 6_145, 2_048, 393_216, 2, 6_144, 1, 2_049):
+        bvh.rebuild(own[:n])
+        got = bvh.download()
+        _assert_tree_equal(got, oracle.build(boxes[:n], bits))
+        for again in range(2):
+            bvh.refit(own_moved[:n])
+            after = bvh.download()
+            nb = after.node_bounds
+            assert np.array_equal(after.node_left, got.node_left)
+            assert np.array_equal(after.sorted_ids, got.sorted_ids)
+            assert np.array_equal(nb[n - 1:], moved_boxes[after.sorted_ids])
+            left, right = after.node_left[:n - 1], after.node_right[:n - 1]
+            assert np.array_equal(nb[:n - 1, :3], np.minimum(nb[left, :3], nb[right, :3]))
+            assert np.array_equal(nb[:n - 1, 3:], np.maximum(nb[left, 3:], nb[right, 3:]))
+        assert bvh.validate(own_moved[:n]) == (True, "")

@@ -610,3 +610,22 @@ def test_image_emission_matches_reference(ctx, sampler, with_env):
     assert np.isfinite(gpu).all() and gpu.mean() > 0
     assert _agreement(gpu, ref) >= 0.97
     assert _z_fraction(gpu, ref) <= 0.01
+
+
+def test_large_batches_sample_as_small_ones_do(ctx):
+    """Two million paths in one batch (four blocks per SM, several paths a thread for each sort
+    of the shading blocks) against batches of 2^16 (three blocks, one path a thread) and against
+    one path per thread: the same radiance, sample for sample."""
+    from lux_b200 import scenes as SC
+    sc = S.Scene(ctx, SC.heavy_render_scene(256, 256))
+    req = S.request(256, 256, 32, 6, 11)
+    saved = [ctx.get_option(o) for o in (lux_b200.OPT_TRACE_VARIANT, lux_b200.OPT_RENDER_BATCH)]
+    want = S.render_samples(ctx, sc, req)
+    try:
+        for variant, batch in ((0, 1 << 16), (1, 1 << 16)):
+            ctx.set_option(lux_b200.OPT_TRACE_VARIANT, variant)
+            ctx.set_option(lux_b200.OPT_RENDER_BATCH, batch)
+            assert np.array_equal(S.render_samples(ctx, sc, req), want)
+    finally:
+        for o, v in zip((lux_b200.OPT_TRACE_VARIANT, lux_b200.OPT_RENDER_BATCH), saved):
+            ctx.set_option(o, v)

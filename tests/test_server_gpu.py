@@ -210,3 +210,19 @@ def test_mixed_batch_over_the_four_resident_scenes_matches_single_renders(ctx):
         rid, alone = srv.submit(*mix[3])
         srv.wait_all(timeout_s=300)
     assert np.array_equal(alone, out[3][1])
+
+
+def test_large_pools_render_as_small_ones_do(ctx):
+    """A pool of two million paths, whose shading blocks sort several paths a thread, against one
+    of 2^15: the same films, bit for bit (they sum in fixed point, so in any order)."""
+    from lux_b200 import scenes as SC
+    resident = [S.Scene(ctx, SC.heavy_render_scene(256, 256)), S.Scene(ctx, _zoo())]
+    reqs = [(0, S.request(256, 256, 24, 6, 21)), (1, S.request(64, 64, 64, 5, 22))]
+    films = []
+    for paths in (1 << 21, 1 << 15):
+        with SV.Server(resident, pool_paths=paths) as srv:
+            out = [srv.submit(s, r) for s, r in reqs]
+            srv.wait_all(timeout_s=120)
+            assert all(srv.poll(i) == SV.DONE for i, _ in out)
+            films.append([f for _, f in out])
+    assert all(np.array_equal(a, b) for a, b in zip(*films))
