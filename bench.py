@@ -41,7 +41,7 @@ METRIC = "Mrays/s"
 # Algorithmic bytes (per unit) used for the roofline: build 120 B/tri, refit 104 B/tri,
 # traversal 32 B ray + 8 B hit + 32 B per box test + 36 B per triangle test.
 BUILD_BYTES_PER_TRI = 120
-TRACE_DRAM_BYTES_PER_RAY = (0.7169208e9 + 0.0557215e9) / 1048576
+TRACE_DRAM_BYTES_PER_RAY = (618.541312e6 + 36.832256e6) / 1048576
 REFIT_BYTES_PER_TRI = 104
 
 
@@ -315,9 +315,11 @@ def run_lux(args) -> None:
     phase_ms = {p: float(np.mean(v)) for p, v in per_phase.items()}
 
     # Roofline of the dominant kernel (the traversal: one launch per trace phase).
-    # DRAM traffic per ray of k_trace_wide_persistent from one ncu capture of this
-    # generator at 1,048,576 triangles and 1,048,576 rays (0.717 GB read + 0.056 GB
-    # written, 737 B per ray), scaled by the ray count.
+    # The algorithmic bytes, counted in the reference's visit order, come mostly from L1 and
+    # L2, so their rate may exceed the DRAM copy rate; the DRAM traffic is about a tenth of
+    # that rate.  Traffic per ray of k_trace_wide_persistent: one ncu capture of this
+    # generator at 1,048,576 triangles and 1,048,576 rays (0.619 GB read + 0.037 GB written,
+    # 625 B per ray, profiles/walk_build_and_trace_kernels.md), scaled by the ray count.
     box_tests, tri_tests = bvh.trace_stats(d_rays)
     trace_bytes = N_RAYS * (32 + 8) + 32 * box_tests + 36 * tri_tests
     peak, peak_kind = measured_peaks()
@@ -359,9 +361,13 @@ def run_lux(args) -> None:
         "refit_mtri_s": N_TRIS / (phase_ms["refit"] * 1e-3) / 1e6,
         "hits": hits, "overlap_pairs": found_count,
         "roofline": {"bound": "hbm",
+                     "note": "the counted bytes come mostly from L1 and L2; the walk is bound "
+                             "by issue and node-load latency" if dominant == "trace" else None,
                      "kernel": "k_trace_wide_persistent" if dominant == "trace" else dominant,
                      "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
                      "unit": "GB/s", "frac": achieved / peak, "traffic": trace_traffic,
+                     "traffic_frac": trace_traffic / (phase_ms["trace"] * 1e-3) / 1e9 / peak
+                                     if trace_traffic else None,
                      "traffic_source": "ncu dram__bytes_read+write of k_trace_wide_persistent "
                                        "at 1,048,576 rays, scaled by rays",
                      "algorithmic_bytes_per_launch": alg,
@@ -552,9 +558,9 @@ RAY_BYTES = 40
 PATH_STATE_BYTES_PER_BOUNCE = 2 * 68
 FILM_BYTES_PER_PATH = 12
 # The Cornell render's kernels run from L1 (a 71-node BLAS): its bound is instruction
-# issue, measured by ncu as the issue-active fraction of the dominant bounce kernel
-# (profiles/render_kernels_cornell_c1.md).
-CORNELL_ISSUE_ACTIVE = None
+# issue, measured by ncu as the issue-active fraction of the dominant bounce kernel, k_walk
+# (profiles/walk_build_and_trace_kernels.md).
+CORNELL_ISSUE_ACTIVE = 0.81
 
 
 def render_roofline(stats: dict, paths: int, seconds: float, scale: float = 1.0,

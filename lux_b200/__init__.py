@@ -41,8 +41,8 @@ PRIM_TRIANGLES = 0
 PRIM_AABBS = 1
 
 OPT_TRACE_VARIANT = 1   # 0 auto, 1 one thread per ray, 2/4 persistent (binary/4-wide), 3 4-wide
-OPT_TRACE_BUDGET = 2    # traversal steps per refill round (ray queries)
-OPT_PATH_BUDGET = 4     # traversal steps per refill round (path tracer)
+OPT_TRACE_BUDGET = 2    # node steps of a warp before waiting leaves and new rays (ray queries)
+OPT_PATH_BUDGET = 4     # the same of the path tracer's walks
 OPT_SCRATCH_BYTES = 5   # read only: the context's reusable device scratch
 OPT_STAGING_BYTES = 6   # read only: the context's reusable device staging
 OPT_REFILL_BLOCKS = 7   # blocks per SM of the refilling path-tracer kernels (0: max)

@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_persistent(
 // but a coherent view of a terrain takes 5 % longer at 5/6 than at 2/3.
 //
 // Few rays are spread over the SMs, `lanes` of a warp taking one each (launch_trace): 2,048
-// rays take 192 us there, and took 335 us in 64 full warps.
+// rays take 212 us instead of 276 us in 64 full warps, and 179 us fetched ahead.
 constexpr int kNodeShareNum = 2, kNodeShareDen = 3;
 
 // Starts bringing 4-wide node `ref` near, if ref is one: an asynchronous 16-byte copy of each
@@ -599,8 +599,9 @@ int launch_trace(lux_ctx* ctx, const lux_bvh* bvh, const float* rays, int nrays,
                                          k_trace_wide_persistent<AnyHit, false>, kTraceThreads);
         // Up to kSpreadWarps warps per SM a warp takes only as many rays as give each SM its
         // share: rays that do not wait for others' steps end sooner.  With more warps than
-        // that (four per scheduler) full ones are better: 65,536 rays take 376 us at 16,
-        // 393 us at 24, 419 us at 32.
+        // that (four per scheduler) fuller ones are better.  Rays of a 1M-triangle tree in us
+        // at 8, 16, 24, 32 warps: 4,096 190, 178, 179, 199; 16,384 240, 252, 243, 278; 32,768
+        // 299, 278, 300, 362; 65,536 329, 333, 340, 384.
         const int spread = ctx->sm_count * kSpreadWarps;
         const int lanes = std::max(1, std::min(32, nrays / spread + (nrays % spread != 0)));
         const int per_block = lanes * (kTraceThreads / 32);
@@ -609,10 +610,12 @@ int launch_trace(lux_ctx* ctx, const lux_bvh* bvh, const float* rays, int nrays,
             cudaError_t err = cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream);
             if (err != cudaSuccess) return cuda_fail(err, "ray counter reset");
         }
-        // Ahead, in microseconds without and with it: 1,024 rays of 1M triangles 183, 148, of
-        // 5,000 triangles 33, 28; 4,096 rays 214, 186 and 39, 36; 32,768 rays 285, 269 and 48,
-        // 47.  At 28 lanes a warp the requests cost what they save (65,536 rays: 316, 321 and
-        // 53, 56), at full warps far more (4,194,304 rays: 4,981, 7,699).
+        // Ahead, in us without and with it, at 1, 7, 14, 18, 28 rays a warp: 1M triangles 216,
+        // 184; 265, 238; 291, 281; 286, 283; 332, 322; a terrain of 131,072 117, 106 at 14 and
+        // 124, 114 at 28; 5,000 triangles 29.3, 26.9; 33.0, 33.0; 37.1, 37.1; 39.2, 41.0; 40.5,
+        // 43.3.  The line is where the smallest tree, whose nodes are near anyway, stops
+        // gaining; once warps are full and refill the requests cost far more than they save
+        // (4,194,304 rays: 4,981, 7,699).
         const bool ahead = lanes <= kAheadLanes;
         const auto kernel = ahead ? k_trace_wide_persistent<AnyHit, true>
                                   : k_trace_wide_persistent<AnyHit, false>;
