@@ -92,20 +92,7 @@ struct Staging {
             return lux::fail(LUX_ERR_INVALID_ARGUMENT,
                              "a device pointer belongs to another GPU than the context's");
         if (items.empty()) return LUX_OK;
-        if (total > ctx->staging_bytes) {
-            if (ctx->staging) {
-                cudaStreamSynchronize(ctx->stream);
-                cudaFree(ctx->staging);
-                ctx->staging = nullptr;
-                ctx->staging_bytes = 0;
-            }
-            cudaError_t err = cudaMalloc(&ctx->staging, total);
-            if (err != cudaSuccess) {
-                cudaGetLastError();
-                return lux::fail(LUX_ERR_OUT_OF_MEMORY, "staging allocation failed");
-            }
-            ctx->staging_bytes = total;
-        }
+        if (int st = lux::ensure_staging(ctx, total)) return st;
         char* base = static_cast<char*>(ctx->staging);
         for (Item& it : items) {
             *it.device = base + it.offset;
@@ -272,6 +259,23 @@ int ensure_scratch(lux_ctx* ctx, size_t bytes) {
         return fail(LUX_ERR_OUT_OF_MEMORY, "scratch allocation failed");
     }
     ctx->scratch_bytes = want;
+    return LUX_OK;
+}
+
+int ensure_staging(lux_ctx* ctx, size_t bytes) {
+    if (bytes <= ctx->staging_bytes) return LUX_OK;
+    if (ctx->staging) {
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(ctx->staging);
+        ctx->staging = nullptr;
+        ctx->staging_bytes = 0;
+    }
+    cudaError_t err = cudaMalloc(&ctx->staging, bytes);
+    if (err != cudaSuccess) {
+        cudaGetLastError();
+        return fail(LUX_ERR_OUT_OF_MEMORY, "staging allocation failed");
+    }
+    ctx->staging_bytes = bytes;
     return LUX_OK;
 }
 

@@ -76,15 +76,16 @@ extern "C" int lux_film_encode(lux_ctx* ctx, const float* film_sum, int32_t widt
         return dev;
     };
     const bool in_dev = on_device(film_sum), out_dev = on_device(out);
-    void* d_in = const_cast<float*>(film_sum);  // replaced by scratch when on the host
+    void* d_in = const_cast<float*>(film_sum);  // replaced by staging when on the host
     void* d_out = out;
     cudaStream_t s = ctx->stream;
-    // The context's scratch, kept from call to call: allocations from the stream's default
-    // pool are mapped anew after every wait.
+    // The context's staging, kept from call to call: allocations from the stream's default
+    // pool are mapped anew after every wait.  (Not its scratch, in which a build may still be
+    // sorting on a stream that the context had before.)
     const size_t in_room = in_dev ? 0 : (in_bytes + 255) & ~size_t(255);
-    if (int st = lux::ensure_scratch(ctx, in_room + (out_dev ? 0 : out_bytes))) return st;
-    if (!in_dev) d_in = ctx->scratch;
-    if (!out_dev) d_out = static_cast<char*>(ctx->scratch) + in_room;
+    if (int st = lux::ensure_staging(ctx, in_room + (out_dev ? 0 : out_bytes))) return st;
+    if (!in_dev) d_in = ctx->staging;
+    if (!out_dev) d_out = static_cast<char*>(ctx->staging) + in_room;
     cudaError_t err = cudaSuccess;
     if (!in_dev) err = cudaMemcpyAsync(d_in, film_sum, in_bytes, cudaMemcpyHostToDevice, s);
     if (err != cudaSuccess) return lux::cuda_fail(err, "film staging");

@@ -28,7 +28,8 @@ struct lux_ctx {
     // Growable device scratch, reused across calls on this context.
     void* scratch = nullptr;
     size_t scratch_bytes = 0;
-    // Growable device staging for host inputs / outputs.
+    // Growable device staging for host inputs / outputs (every call that uses it waits for
+    // the stream before it returns).
     void* staging = nullptr;
     size_t staging_bytes = 0;
     // Copy stream and events of the chunked host-ray queries (created on first use).
@@ -116,6 +117,7 @@ inline int occupancy_blocks(lux_ctx* ctx, int slot, Kernel kernel, int threads) 
 int fail(int status, const std::string& message);
 int cuda_fail(cudaError_t err, const char* what);
 int ensure_scratch(lux_ctx* ctx, size_t bytes);
+int ensure_staging(lux_ctx* ctx, size_t bytes);
 // Waits for the stream and reads (and clears) the device error word, in one wait.
 int wait_error_word(lux_ctx* ctx, int* word);
 

@@ -141,7 +141,7 @@ def _encoded(film, spp, fmt):
 
 
 # The film and the output each on the host or on the device: what is on the host goes through
-# the context's scratch, which a build of more than 6,144 triangles shares.
+# the context's staging, which grows and which a build from host triangles shares.
 @pytest.mark.gpu
 @pytest.mark.parametrize("in_dev", [False, True])
 @pytest.mark.parametrize("out_dev", [False, True])

@@ -210,3 +210,16 @@ for spp in (4, 2048):
     out.append(sorted({g // sm for g in grids}))
 """)
     assert out == [[1, 2, 4], [1, 2, 3, 4]], out    # (the stand-in says that four blocks fit)
+
+
+def test_the_film_encoder_leaves_the_builds_scratch_alone(run):
+    """Host films go through the context's staging, which every call that uses it waits for:
+    a build may still be sorting in the scratch on a stream that the context had before."""
+    out = run("""
+film, ppm = np.ones((40, 30, 3), np.float32), np.zeros((40, 30, 3), np.uint8)
+log()
+lib = ctx._lib
+L._check(lib.lux_film_encode(ctx.handle, film.ctypes.data, 30, 40, 1, 0, ppm.ctypes.data))
+out = [ctx.get_option(L.OPT_SCRATCH_BYTES), ctx.get_option(L.OPT_STAGING_BYTES), launched(log())]
+""")
+    assert out[0] == 0 and out[1] >= 40 * 30 * 15 and out[2] == ["k_encode"], out
