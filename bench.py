@@ -319,7 +319,7 @@ def run_lux(args) -> None:
     # L2, so their rate may exceed the DRAM copy rate; the DRAM traffic is about a tenth of
     # that rate.  Traffic per ray of k_trace_wide_persistent: one ncu capture of this
     # generator at 1,048,576 triangles and 1,048,576 rays (0.619 GB read + 0.037 GB written,
-    # 625 B per ray, profiles/walk_build_and_trace_kernels.md), scaled by the ray count.
+    # 625 B per ray), scaled by the ray count.
     box_tests, tri_tests = bvh.trace_stats(d_rays)
     trace_bytes = N_RAYS * (32 + 8) + 32 * box_tests + 36 * tri_tests
     peak, peak_kind = measured_peaks()
@@ -559,7 +559,7 @@ PATH_STATE_BYTES_PER_BOUNCE = 2 * 68
 FILM_BYTES_PER_PATH = 12
 # The Cornell render's kernels run from L1 (a 71-node BLAS): its bound is instruction
 # issue, measured by ncu as the issue-active fraction of the dominant bounce kernel, k_walk
-# (profiles/walk_build_and_trace_kernels.md).
+# on a capture of bounce 1.
 CORNELL_ISSUE_ACTIVE = 0.81
 
 
